@@ -79,6 +79,17 @@ __global__ void __launch_bounds__(AN_TILE)
         } else if (b == BIN_TINY) {
             lb = BIN_TINY;
             cap = (int)ops[row];
+        } else if (b < BIN_WARP0) {
+            // sorted rows need no table: the prediction sizes only the slot,
+            // and only where it at least halves the bound's (which cannot
+            // overflow)
+            lb = b;
+            cap = ub[row];
+            const int c = max(cap_pred[row], 1);
+            if (c < cap / 2) {
+                cap = c;
+                predicted = 1;
+            }
         } else {
             // the prediction is used only where it buys a smaller table than
             // the upper bound would; otherwise the row gets the bound's table
@@ -151,7 +162,7 @@ __global__ void k_need(int32_t rows, const uint8_t* __restrict__ lbin,
         const bool hslot = hmask && hmask[row];
         pr = predicted[row] != 0;
         big = lb == LBIN_EXACT;
-        ovf = hslot ? hovf[row] != 0 : (lb >= BIN_WARP0 && lb < LBIN_EXACT && cnt[row] < 0);
+        ovf = hslot ? hovf[row] != 0 : (lb >= BIN_SORT0 && lb < LBIN_EXACT && cnt[row] < 0);
         nd = (big && !hslot) || ovf;
         under = pr && (ovf || cnt[row] > lcap[row]);
         if (pr && !ovf) {
@@ -576,10 +587,10 @@ int learned_finish(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int
         note_launch(plan, 1);
     }
     int32_t nw = 0;
-    for (int b = BIN_WARP0; b < LBIN_EXACT; ++b) nw += plan->lcount[b];
+    for (int b = BIN_SORT0; b < LBIN_EXACT; ++b) nw += plan->lcount[b];
     if (nw > 0) {
         k_compact_rows<<<(unsigned)(((int64_t)nw * 32 + 255) / 256), 256, 0, plan->stream>>>(
-            lrows + plan->loffs.off[BIN_WARP0], nw, plan->need.as<uint8_t>(),
+            lrows + plan->loffs.off[BIN_SORT0], nw, plan->need.as<uint8_t>(),
             plan->cnt.as<int32_t>(), plan->slot_off.as<int64_t>(), plan->c_rp.as<int32_t>(),
             plan->tmp_ci.as<int32_t>(), plan->tmp_v.as<float>(), c_ci, c_v);
         note_launch(plan, 1);

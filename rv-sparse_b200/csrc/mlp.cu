@@ -155,12 +155,12 @@ __global__ void __launch_bounds__(256)
     // stencil products) leaves before loading the parameters
     bool any = bin == nullptr;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n && !any; r += gridDim.x * blockDim.x)
-        any = bin[r] >= BIN_WARP0;
+        any = bin[r] >= BIN_SORT0;
     if (!__syncthreads_or(any)) return;
     for (int i = threadIdx.x; i < MLP_NPARAM; i += blockDim.x) sP[i] = model.params[i];
     __syncthreads();
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        if (bin && bin[r] < BIN_WARP0) continue;
+        if (bin && bin[r] < BIN_SORT0) continue;
         const float4 f = feat[r];
         const float raw[MLP_IN] = {f.x, f.y, f.z, f.w};
         float x[MLP_IN];

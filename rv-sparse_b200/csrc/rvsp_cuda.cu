@@ -27,6 +27,7 @@
 #include "rvsp_cuda.h"
 #include "rvsp_internal.h"
 #include "spgemm_kernels.cuh"
+#include "sort_rows.cuh"
 
 using namespace rvsp;
 
@@ -310,7 +311,7 @@ static void launch_warp(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             A, B, rows, n, o.c_rp, o.c_v, lo, pm, o.err);
     } else {
         constexpr int W = warps_for<CAP, MODE>();
-        const int fill = g_sms * g_warp_ctas[MODE][b - BIN_WARP0];
+        const int fill = g_sms * g_warp_ctas[MODE][__builtin_ctz(CAP / WARP_CAP_MIN)];
         const int grid = std::min((n + W - 1) / W, fill);
         int32_t* queue = &plan->misc.as<Misc>()->row_queue;
         cudaMemsetAsync(queue, 0, sizeof(int32_t), plan->stream);
@@ -319,6 +320,29 @@ static void launch_warp(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             o.maps ? lo : nullptr, o.maps ? pm : nullptr, o.err, o.ctl, queue);
     }
     note_launch(plan, 1);
+}
+
+// A sort bin of up to 32 E products: k_sort, unless B has too many columns for
+// its packed words (then the hash kernel, with a table twice the bin's size).
+template <int E, int MODE>
+static void launch_sort(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int b,
+                        const RowOut& o) {
+    constexpr int CAP = 32 * E;
+    if constexpr (MODE == REUSE) {
+        launch_warp<CAP, MODE>(plan, A, B, b, o);
+    } else {
+        if (!sort_cols_fit(B.cols, CAP)) return launch_warp<2 * CAP, MODE>(plan, A, B, b, o);
+        const int n = o.learned_bins ? plan->lcount[b] : plan->bin_count[b];
+        const int32_t* rows = o.learned_bins ? plan->lbin_rows.as<int32_t>() + plan->loffs.off[b]
+                                             : plan->bin_rows.as<int32_t>() + plan->offs.off[b];
+        KTime kt(plan->stream, plan->capturing, KF_WARP_COUNT + MODE);
+        k_sort<E, MODE><<<(n + SORT_WARPS - 1) / SORT_WARPS, SORT_WARPS * 32,
+                          SORT_WARPS * sort_warp_bytes<E>(), plan->stream>>>(
+            A, B, rows, n, o.cnt, o.c_rp, o.c_ci, o.c_v,
+            o.maps ? plan->list_off.as<int32_t>() + plan->offs.off[b] : nullptr,
+            o.maps ? plan->pm16.as<uint16_t>() + plan->pm16_base[b] : nullptr, o.err, o.ctl);
+        note_launch(plan, 1);
+    }
 }
 
 template <int MODE>
@@ -345,6 +369,14 @@ static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
                     A, B, r, n, o.cnt, o.c_rp, o.c_ci, o.c_v, o.maps ? lo : nullptr,
                     o.maps ? plan->pm8.as<uint8_t>() : nullptr, o.err, o.ctl);
             note_launch(plan, 1);
+        } else if (b < BIN_WARP0) {
+            switch (SORT_CAP_MIN << (b - BIN_SORT0)) {
+                case 64: launch_sort<2, MODE>(plan, A, B, b, o); break;
+                case 128: launch_sort<4, MODE>(plan, A, B, b, o); break;
+                case 256: launch_sort<8, MODE>(plan, A, B, b, o); break;
+                case 512: launch_sort<16, MODE>(plan, A, B, b, o); break;
+                default: launch_sort<32, MODE>(plan, A, B, b, o); break;
+            }
         } else if (b < BIN_HEAVY) {
             switch (WARP_CAP_MIN << (b - BIN_WARP0)) {
                 case 64: launch_warp<64, MODE>(plan, A, B, b, o); break;
@@ -705,7 +737,7 @@ bool prepare_maps(rvsp_cuda_plan* plan) {
     plan->maps_ready = false;
     if (!plan->map_policy || plan->products <= 0 || plan->products >= INT32_MAX) return false;
     int64_t p8 = plan->host_misc.bin_prod[BIN_TINY], p16 = 0;
-    for (int b = BIN_WARP0; b < BIN_HEAVY; ++b) {
+    for (int b = BIN_SORT0; b < BIN_HEAVY; ++b) {
         plan->pm16_base[b] = p16;
         p16 += plan->host_misc.bin_prod[b];
     }

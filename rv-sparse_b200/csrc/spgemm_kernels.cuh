@@ -10,6 +10,8 @@
 //   k_bin_scatter  rows grouped by bin; heavy rows expanded into
 //                  (row, column-chunk) work items
 //   k_tiny<MODE>   thread per row, rows with <= 32 products
+//   k_sort<E,..>   warp per row, rows of up to 32 E <= 1024 products sorted in
+//                  registers (sort_rows.cuh)
 //   k_warp<CAP,..> warp per row, shared-memory hash table of CAP slots
 //   k_heavy<..>    warp per (row, column chunk), dense shared-memory
 //                  accumulator + occupancy bitmap over CW columns
