@@ -322,22 +322,21 @@ static void launch_warp(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
     note_launch(plan, 1);
 }
 
-// A sort bin of up to 32 E products: k_sort, unless B has too many columns for
-// its packed words (then the hash kernel, with a table twice the bin's size).
-template <int E, int MODE>
+// A sort bin of up to 32 NW E products: k_sort; values alone (REUSE) take the
+// warp kernels, which hold a row of that many entries.
+template <int E, int NW, int MODE>
 static void launch_sort(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int b,
                         const RowOut& o) {
-    constexpr int CAP = 32 * E;
+    using S = SortShape<E, NW>;
     if constexpr (MODE == REUSE) {
-        launch_warp<CAP, MODE>(plan, A, B, b, o);
+        launch_warp<S::CAP, MODE>(plan, A, B, b, o);
     } else {
-        if (!sort_cols_fit(B.cols, CAP)) return launch_warp<2 * CAP, MODE>(plan, A, B, b, o);
         const int n = o.learned_bins ? plan->lcount[b] : plan->bin_count[b];
         const int32_t* rows = o.learned_bins ? plan->lbin_rows.as<int32_t>() + plan->loffs.off[b]
                                              : plan->bin_rows.as<int32_t>() + plan->offs.off[b];
         KTime kt(plan->stream, plan->capturing, KF_WARP_COUNT + MODE);
-        k_sort<E, MODE><<<(n + SORT_WARPS - 1) / SORT_WARPS, SORT_WARPS * 32,
-                          SORT_WARPS * sort_warp_bytes<E>(), plan->stream>>>(
+        k_sort<E, NW, MODE><<<(n + S::ROWS - 1) / S::ROWS, S::ROWS * S::T, S::ROWS * S::BYTES,
+                              plan->stream>>>(
             A, B, rows, n, o.cnt, o.c_rp, o.c_ci, o.c_v,
             o.maps ? plan->list_off.as<int32_t>() + plan->offs.off[b] : nullptr,
             o.maps ? plan->pm16.as<uint16_t>() + plan->pm16_base[b] : nullptr, o.err, o.ctl);
@@ -371,11 +370,12 @@ static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             note_launch(plan, 1);
         } else if (b < BIN_WARP0) {
             switch (SORT_CAP_MIN << (b - BIN_SORT0)) {
-                case 64: launch_sort<2, MODE>(plan, A, B, b, o); break;
-                case 128: launch_sort<4, MODE>(plan, A, B, b, o); break;
-                case 256: launch_sort<8, MODE>(plan, A, B, b, o); break;
-                case 512: launch_sort<16, MODE>(plan, A, B, b, o); break;
-                default: launch_sort<32, MODE>(plan, A, B, b, o); break;
+                case 64: launch_sort<2, 1, MODE>(plan, A, B, b, o); break;
+                case 128: launch_sort<4, 1, MODE>(plan, A, B, b, o); break;
+                case 256: launch_sort<8, 1, MODE>(plan, A, B, b, o); break;
+                case 512: launch_sort<16, 1, MODE>(plan, A, B, b, o); break;
+                case 1024: launch_sort<16, 2, MODE>(plan, A, B, b, o); break;
+                default: launch_sort<16, 4, MODE>(plan, A, B, b, o); break;
             }
         } else if (b < BIN_HEAVY) {
             switch (WARP_CAP_MIN << (b - BIN_WARP0)) {

@@ -1,242 +1,364 @@
-// Medium rows of up to 1024 products: one warp per row, the row's products
-// sorted by column in registers.
+// Medium rows of up to 2048 products: the row's products sorted by column in
+// registers.
 //
-// Expand, sort, compress. Every product becomes one 32-bit word,
-// column << log2(CAP) | index in A-row order; a warp holds CAP = 32 E words,
-// E per lane, and sorts them with a bitonic network (compare-exchanges inside
-// a lane, shuffles between lanes: no shared memory, no serial chain, E
-// independent operations per layer). Equal columns come out together in A-row
-// order, so each run summed left to right from +0.0f is the reference's order
-// of additions (accum_scalar_f32.c:69) and the values are bit-identical.
+// Expand, sort, compress. Every product becomes one word, column <<
+// log2(CAP) | index in A-row order, and its value goes to shared memory at
+// that index. The words are sorted by a bitonic network: E words a thread,
+// compare-exchanges inside a thread, shuffles between a warp's lanes, shared
+// memory only between the warps of a large row. Equal columns come out
+// together in A-row order, so each run summed left to right from +0.0f is the
+// reference's order of additions (accum_scalar_f32.c:69) and the values are
+// bit-identical.
 //
 // Why not the shared-memory table (k_warp): its radix passes and hash probes
 // are serial chains through shared memory, and its 12 bytes a slot leave few
-// warps to hide them. Measured (B200, device time of the launches): 4096^2 x 16
-// a row, FILL 30 -> 12.6 us, COUNT 24 -> 7.4 us; 2M x 100k tall-skinny, rows of
-// 65..1024 products, FILL 5.0 -> 2.7 ms, COUNT 2.4 -> 1.7 ms.
+// warps to hide them. Bound now by instruction issue (ncu: issue active 52-78 %
+// of peak; a 256-word row takes 1,360 instructions). Measured (B200, device
+// time): 4096^2 x 16 a row, FILL 30 -> 11 us, COUNT 24 -> 7.6 us; 2M x 100k
+// tall-skinny, rows of 33..2048 products, FILL 7.1 -> 3.3 ms, COUNT 3.2 -> 2.1
+// ms; 128 batched products, FILL 22.2 -> 9.1 ms. Tried and dropped: the same
+// rows by one counting pass over column buckets (more instructions: the
+// in-bucket loops cost more than the network's layers), 32 words a thread in
+// one warp for 1024 products (1015 us against 902 us with two warps on the
+// tall-skinny product: 114 registers and code past the instruction cache).
 #pragma once
 
 #include "spgemm_kernels.cuh"
 
 namespace rvsp {
 
-constexpr int SORT_WARPS = 4;  // rows (warps) per CTA
+constexpr int SORT_CTA_ROWS = 4;  // one-warp rows per CTA
 
-// Shared memory of one warp: a bit per product (set where an A entry's
-// products start), then the A entries {B position - first index, A value} while
-// the products are gathered, overlaid afterwards by the products' values and
-// the sorted words (padded by one word in 32: a lane stores E consecutive
-// words, and the padding spreads the lanes over the banks).
-template <int E>
-__host__ __device__ constexpr int sort_warp_bytes() {
-    return 4 * E + 8 * 32 * E + 4 * E;
-}
+// Threads of one row: NW warps, CAP = 32 NW E words.
+template <int E, int NW>
+struct SortShape {
+    static constexpr int T = 32 * NW;
+    static constexpr int CAP = T * E;
+    static constexpr int WORDS = CAP / 32;
+    static constexpr int ROWS = NW == 1 ? SORT_CTA_ROWS : 1;  // rows of a CTA
+    static constexpr int PAD = CAP + WORDS;                   // padded array
+    // Shared words of a row: a bit per product (set where an A entry's
+    // products start) and, for rows of several warps, the starts before each
+    // such word, the threads' open runs and counters; the A entries {B
+    // position - first index, A value} while the products are gathered,
+    // overlaid afterwards by the row's columns and values in C's order; the
+    // products' values.
+    static constexpr int EXTRA = NW == 1 ? 0 : WORDS + T + 2 * NW + 2;
+    static constexpr int BYTES = 4 * (WORDS + EXTRA + 2 * PAD + CAP);
+    static_assert((WORDS + EXTRA) % 2 == 0 && BYTES % 8 == 0, "");
+};
 
-template <int E>
-__device__ __forceinline__ void cross_lane(uint32_t (&k)[E], int mask, bool upper, bool flip) {
-    if (flip) {  // partner of word j is word E-1-j of lane ^ mask
+// Padded index: one word in 32 is left out, so lanes a power of two words
+// apart use different banks.
+__device__ __forceinline__ int pad32(int x) { return x + (x >> 5); }
+
+// The row's CAP words ascending, as the floats of the same bits (finite and
+// not negative, so they order like the words): word j of thread t ends as the
+// (t E + j)-th. Bitonic merges in their all-ascending form: a merge starts by
+// comparing each word with its mirror image in the block, so no later step
+// depends on the block's direction.
+//
+// Between lanes, the lane that keeps the larger word holds it negated: its
+// partner's word arrives with the other sign, and min(own, -partner's) is the
+// right choice on both sides. One min a word and step, against min, max and
+// select; the sign changes between steps are multiplications by +-1, which
+// run on the FMA pipe beside the ALU that the mins saturate.
+template <int E, int NW, int SIZE, int STRIDE>
+__device__ __forceinline__ void sort_layer(float (&f)[E], float& sign, int t, float* xbuf) {
+    constexpr bool FLIP = STRIDE == SIZE / 2;
+    if constexpr (STRIDE < E) {
+        if constexpr (STRIDE * 2 == E && SIZE > E) {
 #pragma unroll
-        for (int j = 0; j < (E + 1) / 2; ++j) {
-            const uint32_t a = __shfl_xor_sync(FULL, k[E - 1 - j], mask);
-            if (E - 1 - j != j) {
-                const uint32_t b = __shfl_xor_sync(FULL, k[j], mask);
-                k[E - 1 - j] = upper ? max(k[E - 1 - j], b) : min(k[E - 1 - j], b);
-            }
-            k[j] = upper ? max(k[j], a) : min(k[j], a);
+            for (int j = 0; j < E; ++j) f[j] *= sign;
+            sign = 1.0f;
         }
-    } else {
 #pragma unroll
         for (int j = 0; j < E; ++j) {
-            const uint32_t a = __shfl_xor_sync(FULL, k[j], mask);
-            k[j] = upper ? max(k[j], a) : min(k[j], a);
+            const int p = j ^ (FLIP ? SIZE - 1 : STRIDE);
+            if (p > j) {
+                const float lo = fminf(f[j], f[p]), hi = fmaxf(f[j], f[p]);
+                f[j] = lo;
+                f[p] = hi;
+            }
         }
-    }
-}
-
-// The warp's 32 E words ascending: word j of lane l ends as the (l E + j)-th.
-// Bitonic merges in their all-ascending form: a merge starts by comparing
-// each word with its mirror image in the block, so no later step depends on
-// the block's direction.
-template <int E>
-__device__ __forceinline__ void warp_bitonic_sort(uint32_t (&k)[E]) {
-    const int lane = lane_id();
+    } else if constexpr (STRIDE < 32 * E) {
+        constexpr int MASK = FLIP ? SIZE / E - 1 : STRIDE / E;
+        const float want = (t & (STRIDE / E)) ? -1.0f : 1.0f;
+        const float m = sign * want;
+        sign = want;
 #pragma unroll
-    for (int size = 2; size <= 32 * E; size <<= 1) {
-        if (size <= E) {
+        for (int j = 0; j < E; ++j) f[j] *= m;
+        if constexpr (FLIP) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const int p = (j & ~(size - 1)) + (size - 1 - (j & (size - 1)));
-                if (p > j) {
-                    const uint32_t lo = min(k[j], k[p]), hi = max(k[j], k[p]);
-                    k[j] = lo;
-                    k[p] = hi;
-                }
+            for (int j = 0; j < E / 2; ++j) {
+                const float a = __shfl_xor_sync(FULL, f[E - 1 - j], MASK);
+                const float b = __shfl_xor_sync(FULL, f[j], MASK);
+                f[j] = fminf(f[j], -a);
+                f[E - 1 - j] = fminf(f[E - 1 - j], -b);
             }
         } else {
-            cross_lane<E>(k, size / E - 1, (lane & (size / E / 2)) != 0, true);
-        }
 #pragma unroll
-        for (int stride = size / 4; stride >= 1; stride >>= 1) {
-            if (stride < E) {
-#pragma unroll
-                for (int j = 0; j < E; ++j) {
-                    if ((j & stride) == 0) {
-                        const uint32_t lo = min(k[j], k[j | stride]), hi = max(k[j], k[j | stride]);
-                        k[j] = lo;
-                        k[j | stride] = hi;
-                    }
-                }
-            } else {
-                cross_lane<E>(k, stride / E, (lane & (stride / E)) != 0, false);
-            }
+            for (int j = 0; j < E; ++j) f[j] = fminf(f[j], -__shfl_xor_sync(FULL, f[j], MASK));
         }
+    } else {  // between warps
+        constexpr int MASK = FLIP ? SIZE - 1 : STRIDE;
+        const bool upper = (t & (STRIDE / E)) != 0;
+#pragma unroll
+        for (int j = 0; j < E; ++j) xbuf[pad32(t * E + j)] = f[j];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const float a = xbuf[pad32((t * E + j) ^ MASK)];
+            f[j] = upper ? fmaxf(f[j], a) : fminf(f[j], a);
+        }
+        __syncthreads();
     }
+    if constexpr (STRIDE > 1) sort_layer<E, NW, SIZE, STRIDE / 2>(f, sign, t, xbuf);
 }
 
-// The rows of one sort bin (at most 32 E products each; rows with more, which
+template <int E, int NW, int SIZE = 2>
+__device__ __forceinline__ void sort_words(float (&f)[E], int t, float* xbuf) {
+    static_assert(E >= 2, "");
+    float sign = 1.0f;  // the words' sign in this lane
+    sort_layer<E, NW, SIZE, SIZE / 2>(f, sign, t, xbuf);
+    if constexpr (SIZE < SortShape<E, NW>::CAP) sort_words<E, NW, SIZE * 2>(f, t, xbuf);
+}
+
+// The rows of one sort bin (at most CAP products each; rows with more, which
 // only an operand changed since the analysis can have, flag ERR_STRUCTURE).
 // COUNT writes the row's distinct columns to cnt; FILL writes its sorted
 // columns and values (in the learned sweep, ctl.slot_off, into the row's slot,
 // with the count to cnt, or -1 when it passes the slot) and, with pm, every
-// product's position in the row. Columns must fit 32 - log2(32 E) bits
+// product's position in the row. Words must stay below the bits of infinity
 // (sort_cols_fit).
-template <int E, int MODE>
-__global__ void __launch_bounds__(SORT_WARPS * 32)
+template <int E, int NW, int MODE>
+__global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
     k_sort(CsrView A, CsrView B, const int32_t* __restrict__ rows, int nrows,
            int32_t* __restrict__ cnt, const int32_t* __restrict__ c_rp,
            int32_t* __restrict__ c_ci, float* __restrict__ c_v,
            const int32_t* __restrict__ list_off, uint16_t* __restrict__ pm,
            int32_t* __restrict__ err, RowCtl ctl) {
     static_assert(MODE == COUNT || MODE == FILL, "");
-    constexpr int CAP = 32 * E;
+    using S = SortShape<E, NW>;
+    constexpr int CAP = S::CAP, T = S::T, WORDS = S::WORDS;
     constexpr int IB = __builtin_ctz(CAP);
+    constexpr uint32_t SAME = MODE == FILL ? CAP : 1;  // words of one column differ by less
     extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = lane_id();
-    const int w = blockIdx.x * SORT_WARPS + warp;
+    const int lane = lane_id();
+    const int wi = NW == 1 ? 0 : threadIdx.x >> 5;  // warp of the row
+    const int t = NW == 1 ? lane : threadIdx.x;     // thread of the row
+    const int slot = NW == 1 ? threadIdx.x >> 5 : 0;
+    const int w = blockIdx.x * S::ROWS + slot;
     if (w >= nrows) return;
     const int row = rows[w];
     if (ctl.only && !ctl.only[row]) return;
-    unsigned char* mine = smem + warp * sort_warp_bytes<E>();
-    uint32_t* heads = reinterpret_cast<uint32_t*>(mine);
-    int2* ent = reinterpret_cast<int2*>(mine + 4 * E);
-    float* vals = reinterpret_cast<float*>(mine + 4 * E);
-    uint32_t* sorted = reinterpret_cast<uint32_t*>(vals + CAP);
-    if (lane < E) heads[lane] = 0u;
-    int a0, a1;
-    row_range(A, row, &a0, &a1, err);
-    __syncwarp();
+    uint32_t* heads = reinterpret_cast<uint32_t*>(smem + slot * S::BYTES);
+    int* pre = reinterpret_cast<int*>(heads + WORDS);       // NW > 1: starts before each word
+    float* tails = reinterpret_cast<float*>(pre + WORDS);   // NW > 1: each thread's open run
+    int* red = reinterpret_cast<int*>(tails + T);           // NW > 1: per-warp words, n, total
+    int2* ent = reinterpret_cast<int2*>(heads + WORDS + S::EXTRA);
+    int32_t* scol = reinterpret_cast<int32_t*>(ent);
+    float* sval = reinterpret_cast<float*>(scol + S::PAD);
+    float* vals = sval + S::PAD;
+    const auto sync = [] {
+        if constexpr (NW == 1) __syncwarp();
+        else __syncthreads();
+    };
+    if (t < WORDS) heads[t] = 0u;
+    sync();
     // the row's non-empty entries, in order, and where their products start
-    int n = 0, entries = 0;
-    for (int base = a0; base < a1; base += 32) {
-        const int j = base + lane;
-        int bs = 0, bl = 0;
-        float av = 0.0f;
-        if (j < a1) {
-            int be;
-            row_range(B, A.ci[j], &bs, &be, err);
-            bl = min(be - bs, CAP + 1);
-            if (MODE == FILL) av = A.v[j];
+    int n = 0;
+    if (NW == 1 || wi == 0) {
+        int a0, a1, entries = 0;
+        row_range(A, row, &a0, &a1, err);
+        for (int base = a0; base < a1; base += 32) {
+            const int j = base + lane;
+            int bs = 0, bl = 0;
+            float av = 0.0f;
+            if (j < a1) {
+                int be;
+                row_range(B, A.ci[j], &bs, &be, err);
+                bl = min(be - bs, CAP + 1);
+                if (MODE == FILL) av = A.v[j];
+            }
+            const int incl = warp_incl_scan(bl);
+            const int start = n + incl - bl;
+            const unsigned some = __ballot_sync(FULL, bl > 0);
+            if (bl > 0 && start < CAP) {
+                ent[entries + __popc(some & ((1u << lane) - 1))] =
+                    make_int2(bs - start, __float_as_int(av));
+                atomicOr(&heads[start >> 5], 1u << (start & 31));
+            }
+            entries += __popc(some);
+            n += __shfl_sync(FULL, incl, 31);
+            if (n > CAP) {
+                if (lane == 0) atomicOr(err, ERR_STRUCTURE);
+                n = CAP;
+                break;
+            }
         }
-        const int incl = warp_incl_scan(bl);
-        const int start = n + incl - bl;
-        const unsigned some = __ballot_sync(FULL, bl > 0);
-        if (bl > 0 && start < CAP) {
-            ent[entries + __popc(some & ((1u << lane) - 1))] =
-                make_int2(bs - start, __float_as_int(av));
-            atomicOr(&heads[start >> 5], 1u << (start & 31));
-        }
-        entries += __popc(some);
-        n += __shfl_sync(FULL, incl, 31);
-        if (n > CAP) {
-            if (lane == 0) atomicOr(err, ERR_STRUCTURE);
-            n = CAP;
-            break;
+        if constexpr (NW > 1) {
+            __syncwarp();
+            if (lane == 0) red[2 * NW] = n;
+            int run = 0;
+            for (int x0 = 0; x0 < WORDS; x0 += 32) {
+                const int c = __popc(heads[x0 + lane]);
+                const int incl = warp_incl_scan(c);
+                pre[x0 + lane] = run + incl - c;
+                run += __shfl_sync(FULL, incl, 31);
+            }
         }
     }
-    __syncwarp();
-    // product p = 32 s + lane: its entry is the number of starts up to p
-    uint32_t k[E];
-    float v[MODE == FILL ? E : 1];
+    sync();
+    if constexpr (NW > 1) n = red[2 * NW];
+    // product p = T s + t: its entry is the number of starts up to p
+    float f[E];
     const unsigned upto = 0xffffffffu >> (31 - lane);
-    int before = -1;
-    bool bad = false;
+    {
+        bool bad = false;
+        int before = -1;
 #pragma unroll
-    for (int s = 0; s < E; ++s) {
-        const unsigned h = heads[s];
-        const int p = 32 * s + lane;
-        k[s] = 0xffffffffu;
-        if (MODE == FILL) v[s] = 0.0f;
-        if (p < n) {
-            const int2 e = ent[before + __popc(h & upto)];
-            const int q = e.x + p;
-            const uint32_t col = (uint32_t)__ldg(B.ci + q);
-            if (MODE == FILL) v[s] = __fmul_rn(__int_as_float(e.y), __ldg(B.v + q));
-            bad |= col >= (uint32_t)B.cols;
-            k[s] = MODE == FILL ? (col << IB) | (uint32_t)p : col;
-        }
-        before += __popc(h);
-    }
-    if (bad) atomicOr(err, ERR_STRUCTURE);
-    if (MODE == FILL) {
-        __syncwarp();  // every lane has read the entries
-#pragma unroll
-        for (int s = 0; s < E; ++s) vals[32 * s + lane] = v[s];
-    }
-    warp_bitonic_sort<E>(k);
-    if (MODE == COUNT || ctl.slot_off) {
-        // distinct columns: words that differ from the one before them
-        constexpr int SH = MODE == FILL ? IB : 0;
-        const uint32_t last = __shfl_up_sync(FULL, k[E - 1], 1);
-        int c = 0;
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            const uint32_t prev = j > 0 ? k[j > 0 ? j - 1 : 0] : last;
-            const bool first = j == 0 && lane == 0;
-            c += lane * E + j < n && (first || (prev >> SH) != (k[j] >> SH));
-        }
-        c = __reduce_add_sync(FULL, c);
-        if (MODE == COUNT) {
-            if (lane == 0) cnt[row] = c;
-            return;
-        }
-        const int64_t room = ctl.slot_off[row + 1] - ctl.slot_off[row];
-        if (lane == 0) cnt[row] = c > room ? -1 : c;
-        if (c > room) return;
-    }
-    if constexpr (MODE == FILL) {
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-            const int x = lane * E + j;
-            sorted[x + (x >> 5)] = k[j];
-        }
-        __syncwarp();
-        const int64_t o = ctl.slot_off ? ctl.slot_off[row] : (int64_t)c_rp[row];
-        const int room = ctl.slot_off ? CAP : c_rp[row + 1] - c_rp[row];
-        uint16_t* pp = pm ? pm + (list_off[w] - list_off[0]) : nullptr;
-        int out = 0;
-        for (int b0 = 0; b0 < n; b0 += 32) {
-            const int x = b0 + lane;
-            const uint32_t wd = sorted[x + (x >> 5)];
-            const uint32_t pv = x > 0 ? sorted[(x - 1) + ((x - 1) >> 5)] : ~wd;
-            const bool head = x < n && (pv >> IB) != (wd >> IB);
-            const unsigned hm = __ballot_sync(FULL, head);
-            const int d = out + __popc(hm & upto) - 1;  // the run's place in the row
-            if (pp && x < n) pp[wd & (CAP - 1)] = (uint16_t)d;
-            if (head) {
-                float sum = __fadd_rn(0.0f, vals[wd & (CAP - 1)]);
-                for (int y = x + 1; y < n; ++y) {
-                    const uint32_t wy = sorted[y + (y >> 5)];
-                    if ((wy >> IB) != (wd >> IB)) break;
-                    sum = __fadd_rn(sum, vals[wy & (CAP - 1)]);
+        for (int s = 0; s < E; ++s) {
+            const unsigned h = heads[s * NW + wi];
+            if constexpr (NW > 1) before = pre[s * NW + wi] - 1;
+            const int p = T * s + t;
+            f[s] = __int_as_float(0x7f800000);  // +inf: after every word
+            if (p < n) {
+                const int2 e = ent[before + __popc(h & upto)];
+                const int q = e.x + p;
+                uint32_t col = (uint32_t)__ldg(B.ci + q);
+                if (MODE == FILL) vals[p] = __fmul_rn(__int_as_float(e.y), __ldg(B.v + q));
+                if (col >= (uint32_t)B.cols) {
+                    bad = true;
+                    col = 0;
                 }
-                if (d < room) {
-                    c_ci[o + d] = (int32_t)(wd >> IB);
-                    c_v[o + d] = sum;
+                f[s] = __uint_as_float(MODE == FILL ? col << IB | (uint32_t)p : col);
+            }
+            before += __popc(h);
+        }
+        if (bad) atomicOr(err, ERR_STRUCTURE);
+    }
+    sync();  // every thread has read the entries
+    sort_words<E, NW>(f, t, sval);
+    // heads: words whose column differs from the one before (bit j of mask)
+    const int mine = min(max(n - t * E, 0), E);  // words this thread holds
+    float last = __shfl_up_sync(FULL, f[E - 1], 1);
+    if constexpr (NW > 1) {
+        if (lane == 31) red[wi] = __float_as_int(f[E - 1]);
+        __syncthreads();
+        if (lane == 0 && wi > 0) last = __int_as_float(red[wi - 1]);
+    }
+    unsigned mask = 0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        const uint32_t x = __float_as_uint(f[j]);
+        const uint32_t y = __float_as_uint(j > 0 ? f[j > 0 ? j - 1 : 0] : last);
+        mask |= (unsigned)(j < mine && ((j == 0 && t == 0) || (x ^ y) >= SAME)) << j;
+    }
+    const int own = __popc(mask);
+    int base = warp_incl_scan(own);
+    int total = __shfl_sync(FULL, base, 31);
+    if constexpr (NW > 1) {
+        if (lane == 31) red[NW + wi] = base;
+        __syncthreads();
+        total = 0;
+        for (int x = 0; x < NW; ++x) {
+            const int c = red[NW + x];
+            if (x < wi) base += c;
+            total += c;
+        }
+    }
+    base -= own;  // the place of this thread's first head
+    if constexpr (MODE == COUNT) {
+        if (t == 0) cnt[row] = total;
+    } else {
+        int64_t o;
+        if (ctl.slot_off) {
+            o = ctl.slot_off[row];
+            const bool over = total > ctl.slot_off[row + 1] - o;
+            if (t == 0) cnt[row] = over ? -1 : total;
+            if (over) return;
+        } else {
+            o = c_rp[row];
+            if (total != c_rp[row + 1] - c_rp[row]) {  // an operand changed since the count
+                if (t == 0) atomicOr(err, ERR_STRUCTURE);
+                return;
+            }
+        }
+        // each run summed in order; a thread stores the runs that begin and
+        // end in its words
+        float v[E];
+#pragma unroll
+        for (int j = 0; j < E; ++j) v[j] = vals[__float_as_uint(f[j]) & (CAP - 1)];
+        const bool lead = mine > 0 && !(mask & 1u);  // its first words belong to a run before
+        bool follow = __shfl_down_sync(FULL, (int)lead, 1);  // its last run goes on
+        if (lane == 31) follow = false;
+        if constexpr (NW > 1) {
+            if (lane == 0) red[wi] = lead;
+            __syncthreads();
+            if (lane == 31 && wi + 1 < NW) follow = red[wi + 1] != 0;
+        }
+        float acc = 0.0f;
+        int d = base - 1;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const bool head = mask >> j & 1u;
+            acc = __fadd_rn(head ? 0.0f : acc, v[j]);
+            d += head;
+            const bool end = j == E - 1 ? !follow : (mask >> (j + 1) & 1u) || j + 1 == mine;
+            if (j < mine && end && d >= base) {
+                scol[pad32(d)] = (int32_t)(__float_as_uint(f[j]) >> IB);
+                sval[pad32(d)] = acc;
+            }
+        }
+        if (pm) {
+            uint16_t* pp = pm + (list_off[w] - list_off[0]);
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                if (j < mine)
+                    pp[__float_as_uint(f[j]) & (CAP - 1)] =
+                        (uint16_t)(base - 1 + __popc(mask & ((2u << j) - 1)));
+        }
+        // runs that cross threads, continued from the thread before; once
+        // more for every thread a run passes through from end to end
+        const bool through = lead && mask == 0;
+        bool any;
+        int rounds;
+        if constexpr (NW == 1) {
+            any = __any_sync(FULL, lead);
+            rounds = any ? 1 + __popc(__ballot_sync(FULL, through)) : 0;
+        } else {
+            any = __syncthreads_or(lead);
+            rounds = any ? 1 + __syncthreads_count(through) : 0;
+        }
+        for (int it = 0; it < rounds; ++it) {
+            float in = __shfl_up_sync(FULL, acc, 1);
+            if constexpr (NW > 1) {
+                if (lane == 31) tails[wi] = acc;
+                __syncthreads();
+                if (lane == 0 && wi > 0) in = tails[wi - 1];
+                __syncthreads();
+            }
+            if (lead) {
+                float a = in;
+                const int until = mask ? __ffs(mask) - 1 : mine;
+                int col = 0;
+#pragma unroll
+                for (int j = 0; j < E; ++j)
+                    if (j < until) a = __fadd_rn(a, v[j]);
+                col = (int32_t)(__float_as_uint(f[0]) >> IB);
+                if (through) acc = a;
+                if (!(through && follow)) {
+                    scol[pad32(base - 1)] = col;
+                    sval[pad32(base - 1)] = a;
                 }
             }
-            out += __popc(hm);
         }
-        if (!ctl.slot_off && out != room && lane == 0) atomicOr(err, ERR_STRUCTURE);
+        sync();
+        for (int x = t; x < total; x += T) {
+            c_ci[o + x] = scol[pad32(x)];
+            c_v[o + x] = sval[pad32(x)];
+        }
     }
 }
 

@@ -10,8 +10,8 @@
 //   k_bin_scatter  rows grouped by bin; heavy rows expanded into
 //                  (row, column-chunk) work items
 //   k_tiny<MODE>   thread per row, rows with <= 32 products
-//   k_sort<E,..>   warp per row, rows of up to 32 E <= 1024 products sorted in
-//                  registers (sort_rows.cuh)
+//   k_sort<E,NW,..> 1, 2 or 4 warps per row, rows of up to 2048 products sorted
+//                  in registers (sort_rows.cuh)
 //   k_warp<CAP,..> warp per row, shared-memory hash table of CAP slots
 //   k_heavy<..>    warp per (row, column chunk), dense shared-memory
 //                  accumulator + occupancy bitmap over CW columns
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(AN_TILE)
     const int row = r0 + t;
     const int64_t ops = live ? (int64_t)s_ops[t] : 0;
     const int32_t ub = (int32_t)min(ops, (int64_t)B.cols);
-    const int b = live ? bin_of(ops, ub, P) : -1;
+    const int b = live ? bin_of(ops, ub, B.cols, P) : -1;
     int nch = 0;
     if (live) {
         out.ops[row] = ops;

@@ -39,10 +39,10 @@ constexpr int NUM_WARP_BINS = 7;
 constexpr int WARP_CAP_MAX = WARP_CAP_MIN << (NUM_WARP_BINS - 1);
 constexpr int BIN_EMPTY = 0;
 constexpr int BIN_TINY = 1;
-// rows of at most SORT_CAP_MAX products sorted in registers (k_sort): bins of
-// up to 64, 128, .. 1024 products
+// rows of at most SORT_CAP_MAX products sorted by column (k_sort): bins of
+// up to 64, 128, .. 2048 products
 constexpr int SORT_CAP_MIN = 64;
-constexpr int NUM_SORT_BINS = 5;
+constexpr int NUM_SORT_BINS = 6;
 constexpr int SORT_CAP_MAX = SORT_CAP_MIN << (NUM_SORT_BINS - 1);
 constexpr int BIN_SORT0 = 2;
 constexpr int BIN_WARP0 = BIN_SORT0 + NUM_SORT_BINS;
@@ -151,29 +151,31 @@ __host__ __device__ inline int table_bin(int32_t ub, const BinParams& p) {
     return cap < need ? BIN_HEAVY : b;
 }
 
-// A row goes to a sort bin when its products fit and it could hold at least
-// one distinct column in SORT_UB_RATIO products: sorting costs by the product,
-// a table of few columns by the column.
+// Whether a column index and a product index of a sort bin of cap products
+// share a word below the bits of infinity.
+__host__ __device__ inline bool sort_cols_fit(int32_t b_cols, int cap) {
+    return (int64_t)b_cols * cap <= 0x7f800000;
+}
+
+// A row goes to a sort bin when its products and B's columns fit and it could
+// hold at least one distinct column in SORT_UB_RATIO products: sorting costs
+// by the product, a table of few columns by the column.
 constexpr int SORT_UB_RATIO = 4;
 
-__host__ __device__ inline int bin_of(int64_t ops, int32_t ub, const BinParams& p) {
+__host__ __device__ inline int bin_of(int64_t ops, int32_t ub, int32_t b_cols,
+                                      const BinParams& p) {
     if (ub <= 0) return BIN_EMPTY;
     if (ops <= p.tiny_ops) return BIN_TINY;
-    if (ops <= SORT_CAP_MAX && ops <= p.warp_cap_max && ops <= SORT_UB_RATIO * (int64_t)ub) {
+    const int tb = table_bin(ub, p);
+    if (tb != BIN_HEAVY && ops <= SORT_CAP_MAX && ops <= SORT_UB_RATIO * (int64_t)ub) {
         int cap = SORT_CAP_MIN, b = BIN_SORT0;
         while (cap < ops) {
             cap <<= 1;
             ++b;
         }
-        return b;
+        if (sort_cols_fit(b_cols, cap)) return b;
     }
-    return table_bin(ub, p);
-}
-
-// Whether a column index and a product index of a sort bin of cap products
-// share a 32-bit word.
-__host__ __device__ inline bool sort_cols_fit(int32_t b_cols, int cap) {
-    return (int64_t)b_cols * cap <= int64_t(1) << 32;
+    return tb;
 }
 
 }  // namespace rvsp

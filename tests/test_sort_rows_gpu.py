@@ -1,4 +1,4 @@
-"""Rows sorted in registers (k_sort): row sizes at the bins' edges, short and
+"""Rows sorted by column (k_sort): row sizes at the bins' edges, short and
 long B rows with empty ones between, repeated columns, and column counts at
 the limit of the packed words and past it (where the hash kernel takes the
 rows), bit for bit against the oracle: one-shot exact and learned, and a
@@ -15,11 +15,12 @@ from test_parity_gpu import assert_same, oracle_full
 
 pytestmark = pytest.mark.gpu
 
-EDGES = [33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025]
-LENGTHS = [0, 1, 2, 3, 7, 16, 33, 100]
+EDGES = [33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025,
+         2047, 2048, 2049]
+LENGTHS = [0, 1, 2, 3, 7, 16, 33, 100, 300]
 
 
-def _edge_product(cols, repeats, seed):
+def _edge_product(cols, repeats, seed, clustered=False):
     """A's rows have EDGES products each, made of B rows of LENGTHS entries
     (empty ones among them), every B row used up to `repeats` times."""
     rng = np.random.default_rng(seed)
@@ -27,6 +28,8 @@ def _edge_product(cols, repeats, seed):
     counts = np.minimum(np.repeat(LENGTHS, per), cols)
     parts = [np.sort(rng.choice(cols, n, replace=False)) if cols < 1 << 20
              else np.unique(rng.integers(0, cols, 2 * n))[:n] for n in counts]
+    if clustered:  # runs of columns, few of them: crowded buckets
+        parts = [int(rng.integers(0, 6)) * (cols // 7) + np.arange(n) for n in counts]
     for p in parts:  # the outermost columns occur
         if p.size > 1:
             p[0], p[-1] = 0, cols - 1
@@ -62,14 +65,15 @@ def _edge_product(cols, repeats, seed):
     return A, S
 
 
-CASES = [(5000, 1), (400, 4), (1 << 22, 1), ((1 << 22) + 1, 2), ((1 << 26) + 1, 1)]
+CASES = [(5000, 1, False), (400, 4, False), (1044480, 1, False), (1044481, 2, False),
+         ((1 << 26) + 1, 1, False), (100000, 1, True), (3000, 4, True)]
 
 
-@pytest.mark.parametrize("cols,repeats", CASES)
-def test_row_sizes_at_the_bins_edges(gpu_lib, cols, repeats):
-    A, B = _edge_product(cols, repeats, cols % 97)
+@pytest.mark.parametrize("cols,repeats,clustered", CASES)
+def test_row_sizes_at_the_bins_edges(gpu_lib, cols, repeats, clustered):
+    A, B = _edge_product(cols, repeats, cols % 97, clustered)
     ops = gen.row_products(A, B)
-    assert {64, 65, 128, 256, 512, 1024} & set(ops.tolist())
+    assert {64, 65, 128, 256, 512, 1024, 2048} & set(ops.tolist())
     want = oracle_full(A, B)
     assert_same(oneshot(A, B), want, "exact")
     assert_same(oneshot(A, B, algo=rv.RVSP_CUDA_ALGO_LEARNED), want, "learned")
