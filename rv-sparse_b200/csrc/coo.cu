@@ -6,15 +6,28 @@
 // order (:246-300); each row sorted by column and repeated (row, column)
 // entries summed (:112-131).
 //
-// Here: one stable LSD radix sort of the packed keys (row << cb | column)
-// with the COO index as payload, so entries with equal keys stay in COO
-// order; then each run of equal keys is summed left to right, starting from
-// its first value like the reference (acc = first; acc += next ...), and the
-// row pointer is read off the sorted rows. Every pass is a device kernel;
-// the only host work is the launch sequence and one read of the output size.
+// Here: one stable LSD radix sort of the packed keys (row << cb | column) with
+// the values as payload, so entries with equal keys stay in COO order; then
+// each run of equal keys is summed left to right, starting from its first
+// value like the reference (acc = first; acc += next ...), and the row pointer
+// is written where a run starts a new row. Every pass is a device kernel; the
+// only host work is the launch sequence and one read of the output size.
+//
+// A pass reads and writes every entry once: the digit counts of all passes
+// come from one sweep over the list beforehand, and a tile learns where its
+// digits go from the tiles before it while the pass runs (k_coo_pass), so no
+// pass counts first. Measured (16.8 M entries of 40-bit keys, 5 passes, whole
+// call): 2.72 ms with a histogram, a scan and an uncoalesced scatter per pass
+// and 16-byte entries, 1.22 ms now; 177 us a pass against 62 us of HBM time for
+// its 24 bytes an entry. A tile takes 34,000 cycles, of which the wait for the
+// tiles before it 8,000 (without it a pass takes 122 us, without the output
+// writes 165). Tried and dropped: tiles of 512 threads with 8 entries each (193
+// us with two CTAs an SM, 215 with three), 4 or 16 earlier tiles read at once
+// (no difference).
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <utility>
@@ -27,37 +40,70 @@ using namespace rvsp;
 
 namespace {
 
-constexpr int RS_TPB = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_TPB * RS_ITEMS;  // keys per block and pass
-constexpr int RS_WARPS = RS_TPB / 32;
+constexpr int CS_TPB = 256;
+constexpr int CS_ITEMS = 16;
+constexpr int CS_TILE = CS_TPB * CS_ITEMS;  // entries per tile
+constexpr int CS_WARPS = CS_TPB / 32;
+constexpr int RUN_ITEMS = 8;
+constexpr int RUN_TILE = CS_TPB * RUN_ITEMS;  // sorted entries per tile of the run kernels
+constexpr int CS_PASSES = 8;   // 62-bit keys at most
+constexpr int CS_COPIES = 4;   // shared copies of the digit counters (fewer collisions)
+constexpr unsigned CS_FULL = 0xffffffffu;
+constexpr int COO_BAD = 1;     // error word: an index out of range
+constexpr int COO_STUCK = 2;   // a wait on an earlier tile ran out
 
 __device__ __forceinline__ int c_lane() { return threadIdx.x & 31; }
 
-// Keys and payloads; the mirrored entries of a symmetric matrix go after the
-// stored ones, in the stored order (mpos = exclusive scan of off-diagonal
-// flags). Rows or columns out of range set *bad.
-__global__ void k_coo_keys(int64_t n, int32_t rows, int32_t cols, int cb,
-                           const int32_t* __restrict__ r, const int32_t* __restrict__ c,
-                           int symmetric, const int64_t* __restrict__ mpos,
-                           uint64_t* __restrict__ keys, int64_t* __restrict__ idx,
-                           int32_t* __restrict__ bad) {
+// Digits of the keys: `passes` of db bits.
+struct Digits {
+    int passes, db;
+    __device__ __forceinline__ int of(uint64_t key, int p) const {
+        return (int)(key >> (p * db)) & ((1 << db) - 1);
+    }
+};
+
+// Where a pass reads its keys: the COO list itself or an array of keys.
+struct CooKeys {
+    const int32_t* r;
+    const int32_t* c;
+    int32_t rows, cols;
+    int cb;
+    int32_t* bad;
+    __device__ __forceinline__ uint64_t at(int64_t i) const {
+        const int32_t ri = r[i], ci = c[i];
+        if ((unsigned)ri >= (unsigned)rows || (unsigned)ci >= (unsigned)cols) {
+            atomicOr(bad, COO_BAD);
+            return 0;
+        }
+        return ((uint64_t)ri << cb) | (uint64_t)ci;
+    }
+};
+
+template <class K>
+struct ArrayKeys {
+    const K* k;
+    __device__ __forceinline__ uint64_t at(int64_t i) const { return k[i]; }
+};
+
+// Keys and values of a list: used for symmetric lists, whose mirrored entries
+// go after the stored ones, in the stored order (mpos = exclusive scan of
+// off-diagonal flags), and for keys of no bits, which no pass reads.
+template <class K>
+__global__ void k_coo_keys(int64_t n, CooKeys src, const float* __restrict__ v, int symmetric,
+                           const int64_t* __restrict__ mpos, K* __restrict__ keys,
+                           float* __restrict__ vals) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int32_t ri = r[i], ci = c[i];
-    if ((unsigned)ri >= (unsigned)rows || (unsigned)ci >= (unsigned)cols ||
-        (symmetric && ((unsigned)ci >= (unsigned)rows || (unsigned)ri >= (unsigned)cols))) {
-        atomicOr(bad, 1);
-        keys[i] = 0;
-        idx[i] = i;
-        return;
-    }
-    keys[i] = ((uint64_t)ri << cb) | (uint64_t)ci;
-    idx[i] = i;
+    const uint64_t key = src.at(i);
+    keys[i] = (K)key;
+    if (v) vals[i] = v[i];
+    const int32_t ri = src.r[i], ci = src.c[i];
     if (symmetric && ri != ci) {
         const int64_t j = n + mpos[i];
-        keys[j] = ((uint64_t)ci << cb) | (uint64_t)ri;
-        idx[j] = i;  // the mirror carries the stored entry's value
+        // (rows == cols: an index in range is in range mirrored)
+        const bool ok = (unsigned)ri < (unsigned)src.rows && (unsigned)ci < (unsigned)src.cols;
+        keys[j] = ok ? (K)(((uint64_t)ci << src.cb) | (uint64_t)ri) : (K)0;
+        if (v) vals[j] = v[i];
     }
 }
 
@@ -67,107 +113,300 @@ __global__ void k_offdiag(int64_t n, const int32_t* __restrict__ r, const int32_
     if (i < n) flag[i] = r[i] != c[i];
 }
 
-// Per-block histogram of one 8-bit digit, digit-major: hist[d * blocks + b].
-__global__ void __launch_bounds__(RS_TPB)
-    k_rs_hist(int64_t n, const uint64_t* __restrict__ keys, int shift, int32_t* __restrict__ hist) {
-    __shared__ int32_t h[256];
-    h[threadIdx.x] = 0;
+// Digit counts of every pass in one sweep: counts[p * 256 + digit].
+template <class Src>
+__global__ void __launch_bounds__(CS_TPB)
+    k_coo_digits(int64_t n, Src src, Digits dg, unsigned long long* __restrict__ counts) {
+    __shared__ uint32_t h[CS_COPIES][CS_PASSES * 256];
+    for (int x = threadIdx.x; x < CS_COPIES * CS_PASSES * 256; x += CS_TPB) (&h[0][0])[x] = 0u;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const int64_t i = base + (int64_t)k * RS_TPB + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255], 1);
+    uint32_t* mine = h[threadIdx.x & (CS_COPIES - 1)];
+    const int64_t step = (int64_t)gridDim.x * CS_TPB;
+    for (int64_t i = (int64_t)blockIdx.x * CS_TPB + threadIdx.x; i < n; i += step) {
+        const uint64_t key = src.at(i);
+        for (int p = 0; p < dg.passes; ++p) atomicAdd(&mine[p * 256 + dg.of(key, p)], 1u);
     }
     __syncthreads();
-    hist[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter of one digit: the block walks its tile in order, 256 keys
-// at a time; within a step ranks follow warp then lane order (match_any per
-// warp, per-digit warp counts prefix-summed by one thread per digit).
-__global__ void __launch_bounds__(RS_TPB)
-    k_rs_scatter(int64_t n, const uint64_t* __restrict__ keys, const int64_t* __restrict__ idx,
-                 int shift, const int32_t* __restrict__ off, uint64_t* __restrict__ keys_out,
-                 int64_t* __restrict__ idx_out) {
-    __shared__ int32_t cursor[256];
-    __shared__ int32_t wcnt[RS_WARPS][256];
-    const int t = threadIdx.x, warp = t >> 5, lane = c_lane();
-    cursor[t] = off[(int64_t)t * gridDim.x + blockIdx.x];
-    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const int64_t i = base + (int64_t)k * RS_TPB + t;
-        const bool ok = i < n;
-        uint64_t key = 0;
-        int64_t pl = 0;
-        int d = 256 + lane;  // idle lanes: keys no real digit matches
-        if (ok) {
-            key = keys[i];
-            pl = idx[i];
-            d = (int)((key >> shift) & 255);
-        }
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & ((1u << lane) - 1));
-        if (ok && lane == __ffs(peers) - 1) wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        // thread t: digit t's base for every warp of this step, in warp order
-        int run = cursor[t];
-        int wbase[RS_WARPS];
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) {
-            wbase[w] = run;
-            run += wcnt[w][t];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = wbase[w];
-        cursor[t] = run;
-        __syncthreads();
-        if (ok) {
-            const int pos = wcnt[warp][d] + rank;
-            keys_out[pos] = key;
-            idx_out[pos] = pl;
-        }
-        __syncthreads();
-        for (int w = 0; w < RS_WARPS; ++w) wcnt[w][t] = 0;
-        __syncthreads();
+    for (int x = threadIdx.x; x < dg.passes * 256; x += CS_TPB) {
+        uint32_t s = 0;
+        for (int k = 0; k < CS_COPIES; ++k) s += h[k][x];
+        if (s) atomicAdd(&counts[x], (unsigned long long)s);
     }
 }
 
-__global__ void k_run_heads(int64_t n, const uint64_t* __restrict__ keys,
-                            int32_t* __restrict__ head) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) head[i] = i == 0 || keys[i] != keys[i - 1];
+// Exclusive scan of 256 values, one a thread.
+__device__ __forceinline__ uint32_t scan256(uint32_t x, uint32_t* s_warp) {
+    const int lane = c_lane(), warp = threadIdx.x >> 5;
+    uint32_t incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(CS_FULL, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    __syncthreads();
+    return before + incl - x;
 }
 
-// One output entry per run of equal keys: its column, and the run's values
-// summed in COO order from the first value (no added zero: a lone -0.0 stays).
-__global__ void k_run_sum(int64_t n, const uint64_t* __restrict__ keys,
-                          const int64_t* __restrict__ idx, const int32_t* __restrict__ head,
-                          const int64_t* __restrict__ pos, int cb, const float* __restrict__ v,
-                          int32_t* __restrict__ out_row, int32_t* __restrict__ out_ci,
-                          float* __restrict__ out_v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !head[i]) return;
-    const uint64_t key = keys[i];
-    float acc = v ? v[idx[i]] : 1.0f;
-    for (int64_t j = i + 1; j < n && keys[j] == key; ++j) acc += v ? v[idx[j]] : 1.0f;
-    const int64_t o = pos[i];
-    out_row[o] = (int32_t)(key >> cb);
-    out_ci[o] = (int32_t)(key & ((1ull << cb) - 1));
-    out_v[o] = acc;
+// Where every digit of every pass starts: one CTA a pass.
+__global__ void __launch_bounds__(256)
+    k_coo_starts(const unsigned long long* __restrict__ counts, uint32_t* __restrict__ starts) {
+    __shared__ uint32_t s_warp[8];
+    const int x = blockIdx.x * 256 + threadIdx.x;
+    starts[x] = scan256((uint32_t)counts[x], s_warp);
 }
 
-// Row pointer of the sorted output: entry o starts every row after the
-// previous entry's row up to its own.
-__global__ void k_row_ptr_from_rows(int64_t m, int32_t rows, const int32_t* __restrict__ out_row,
-                                    int32_t* __restrict__ rp) {
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o > m) return;
-    const int32_t cur = o < m ? out_row[o] : rows;
-    const int32_t prev = o > 0 ? out_row[o - 1] : -1;
-    for (int32_t r = prev + 1; r <= cur; ++r) rp[r] = (int32_t)o;
+__device__ __forceinline__ unsigned long long load_word(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void store_word(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" : : "l"(p), "l"(v));
+}
+
+// Lanes whose digit equals the caller's (ok lanes only), a ballot a bit
+// (match_any instead: 195 us a pass against 177).
+__device__ __forceinline__ unsigned same_digit(int d, bool ok) {
+    unsigned peers = __ballot_sync(CS_FULL, ok);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = d >> b & 1;
+        const unsigned bal = __ballot_sync(CS_FULL, bit);
+        peers &= bit ? bal : ~bal;
+    }
+    return peers;
+}
+
+// Polls of one wait before it gives up (a second or more; a tile waits only
+// for tiles that started before it, so an ordinary wait is microseconds).
+constexpr int CS_POLLS = 1 << 20;
+constexpr int CS_BACK = 16;  // earlier tiles read at once
+
+// One stable pass by digit p. Tiles are numbered in the order they start, so
+// every tile a tile waits for is running or done. Per tile: ranks of its
+// entries within their digits (warp by warp, step by step: ballots give
+// the lanes of one digit, counters of half a warp's entries those before), entries to
+// shared memory in digit order, then written out run by run. Where each
+// digit's run goes: the tile publishes its digit counts as soon as it has them
+// (tag 2p + 1), thread d adds up digit d's counts of the tiles before it back
+// to one that has published its running total (tag 2p + 2), and publishes its
+// own. A word holds tag and count, so reading it needs no fence; words of
+// earlier passes carry smaller tags and read as not yet there.
+template <class K, class Src, bool VAL>
+__global__ void __launch_bounds__(CS_TPB, 3)
+    k_coo_pass(int64_t n, Src src, const float* __restrict__ vals, Digits dg, int p,
+               const uint32_t* __restrict__ starts, unsigned long long* __restrict__ status,
+               int32_t* __restrict__ ticket, K* __restrict__ keys_out,
+               float* __restrict__ vals_out, int32_t* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    K* s_key = reinterpret_cast<K*>(smem);
+    float* s_val = reinterpret_cast<float*>(s_key + CS_TILE);
+    uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_val + (VAL ? CS_TILE : 0));  // [half of a warp][256]
+    __shared__ uint32_t s_first[256];  // digit d's first entry in the tile
+    __shared__ int64_t s_to[256];      // its place in the output less s_first
+    __shared__ uint32_t s_warp[8];
+    __shared__ int s_tile, s_dead;
+    const int t = threadIdx.x, lane = c_lane(), warp = t >> 5;
+    if (t == 0) {
+        s_tile = atomicAdd(ticket, 1);
+        s_dead = 0;
+    }
+    for (int x = t; x < CS_WARPS * 256; x += CS_TPB) reinterpret_cast<uint32_t*>(s_cnt)[x] = 0u;
+    __syncthreads();
+    const int tile = s_tile;
+    const int64_t base = (int64_t)tile * CS_TILE + warp * (32 * CS_ITEMS);
+    K key[CS_ITEMS];
+    uint16_t rank[CS_ITEMS];
+    // the warp's entries as two halves with counters of their own, ranked side
+    // by side: two chains through shared memory instead of one twice as long
+    constexpr int HALF = CS_ITEMS / 2;
+    uint16_t* cnt = s_cnt + 2 * warp * 256;
+#pragma unroll
+    for (int s = 0; s < CS_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        key[s] = i < n ? (K)src.at(i) : (K)0;
+    }
+#pragma unroll
+    for (int s = 0; s < HALF; ++s) {
+        int d[2], before[2];
+        unsigned peers[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool ok = base + 32 * (s + h * HALF) + lane < n;
+            d[h] = ok ? dg.of(key[s + h * HALF], p) : 256 + lane;
+            peers[h] = same_digit(d[h], ok);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) before[h] = d[h] < 256 ? cnt[h * 256 + d[h]] : 0;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (d[h] < 256 && lane == 31 - __clz(peers[h]))
+                cnt[h * 256 + d[h]] = (uint16_t)(before[h] + __popc(peers[h]));
+            rank[s + h * HALF] = (uint16_t)(before[h] + __popc(peers[h] & ((1u << lane) - 1)));
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread t: digit t's entries before each half, and in the tile
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < 2 * CS_WARPS; ++w) {
+        const uint32_t c = s_cnt[w * 256 + t];
+        s_cnt[w * 256 + t] = (uint16_t)total;
+        total += c;
+    }
+    unsigned long long* word = status + (int64_t)tile * 256 + t;
+    const unsigned long long tag = (unsigned long long)(2 * p + 1) << 48;
+    const unsigned long long mask48 = (1ull << 48) - 1;
+    store_word(word, (tile == 0 ? tag + (1ull << 48) : tag) | total);
+    const uint32_t first = scan256(total, s_warp);
+    s_first[t] = first;
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < CS_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        if (i < n) {
+            const int d = dg.of(key[s], p);
+            const int at = (int)s_first[d] + cnt[(s < HALF ? 0 : 256) + d] + rank[s];
+            s_key[at] = key[s];
+            if (VAL) s_val[at] = vals[i];
+        }
+    }
+    // digit t's entries in the tiles before
+    unsigned long long excl = 0;
+    int back = tile - 1, polls = 0;
+    while (back >= 0) {
+        unsigned long long wd[CS_BACK];
+#pragma unroll
+        for (int u = 0; u < CS_BACK; ++u)
+            wd[u] = back - u >= 0 ? load_word(status + (int64_t)(back - u) * 256 + t) : 0ull;
+        bool done = false;
+        int u = 0;
+#pragma unroll
+        for (int q = 0; q < CS_BACK; ++q) {
+            if (done || u < q || back - q < 0 || wd[q] < tag) continue;
+            excl += wd[q] & mask48;
+            done = wd[q] >= tag + (1ull << 48);
+            ++u;
+        }
+        if (done) break;
+        back -= u;
+        if (u > 0) polls = 0;
+        else if (++polls > CS_POLLS || ((polls & 1023) == 0 && (load_word(
+                     reinterpret_cast<unsigned long long*>(status) - 1) != 0ull))) {
+            // give up: flag it (for the host, and for the other waits) and
+            // write nothing
+            atomicOr(err, COO_STUCK);
+            store_word(status - 1, 1ull);
+            s_dead = 1;
+            break;
+        }
+    }
+    store_word(word, (tag + (1ull << 48)) | (excl + total));
+    s_to[t] = (int64_t)starts[p * 256 + t] + (int64_t)excl - (int64_t)first;
+    __syncthreads();
+    if (s_dead) return;
+    const int64_t left = n - (int64_t)tile * CS_TILE;
+    const int here = left < CS_TILE ? (int)left : CS_TILE;
+#pragma unroll 4
+    for (int x = t; x < here; x += CS_TPB) {
+        const K k = s_key[x];
+        const int64_t o = s_to[dg.of(k, p)] + x;
+        if (o >= 0 && o < n) {
+            keys_out[o] = k;
+            if (VAL) vals_out[o] = s_val[x];
+        }
+    }
+}
+
+// Runs of equal keys per tile: entries that differ from the one before.
+template <class K>
+__global__ void __launch_bounds__(CS_TPB)
+    k_run_count(int64_t n, const K* __restrict__ keys, int32_t* __restrict__ tile_runs) {
+    __shared__ int s_sum;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    int c = 0;
+#pragma unroll 4
+    for (int s = 0; s < RUN_ITEMS; ++s) {
+        const int64_t i = (int64_t)blockIdx.x * RUN_TILE + s * CS_TPB + threadIdx.x;
+        if (i < n) c += i == 0 || keys[i] != keys[i - 1];
+    }
+    c = __reduce_add_sync(CS_FULL, c);
+    if (c_lane() == 0) atomicAdd(&s_sum, c);
+    __syncthreads();
+    if (threadIdx.x == 0) tile_runs[blockIdx.x] = s_sum;
+}
+
+// One output entry per run: its column, and its values summed in COO order
+// from the first one (no added zero: a lone -0.0 stays). A run that starts a
+// new row writes the row pointer of every row since the last run's; the last
+// entry those after its own.
+template <class K>
+__global__ void __launch_bounds__(CS_TPB)
+    k_run_write(int64_t n, const K* __restrict__ keys, const float* __restrict__ v,
+                const int64_t* __restrict__ tile_off, int cb, int32_t rows, int32_t out_n,
+                int32_t* __restrict__ rp, int32_t* __restrict__ out_ci,
+                float* __restrict__ out_v) {
+    __shared__ int s_warp[CS_WARPS];
+    const int lane = c_lane(), warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * RUN_TILE + warp * (32 * RUN_ITEMS);
+    K key[RUN_ITEMS];
+    unsigned heads = 0;
+    int mine = 0;
+#pragma unroll
+    for (int s = 0; s < RUN_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        key[s] = i < n ? keys[i] : (K)0;
+    }
+    // the key before the warp's first and the one after its last
+    const K edge0 = base > 0 && base <= n ? keys[base - 1] : (K)0;
+    const K edge1 = base + 32 * RUN_ITEMS < n ? keys[base + 32 * RUN_ITEMS] : (K)0;
+#pragma unroll
+    for (int s = 0; s < RUN_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        K prev = __shfl_up_sync(CS_FULL, key[s], 1);
+        const K carry = s > 0 ? __shfl_sync(CS_FULL, key[s > 0 ? s - 1 : 0], 31) : edge0;
+        if (lane == 0) prev = carry;
+        const bool head = i < n && (i == 0 || key[s] != prev);
+        heads |= (unsigned)head << s;
+        mine += __popc(__ballot_sync(CS_FULL, head));
+    }
+    if (lane == 0) s_warp[warp] = mine;
+    __syncthreads();
+    int64_t out = tile_off[blockIdx.x];
+    for (int w = 0; w < warp; ++w) out += s_warp[w];
+#pragma unroll
+    for (int s = 0; s < RUN_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        const bool head = heads >> s & 1u;
+        const unsigned hm = __ballot_sync(CS_FULL, head);
+        K prev = __shfl_up_sync(CS_FULL, key[s], 1), next = __shfl_down_sync(CS_FULL, key[s], 1);
+        const K carry0 = s > 0 ? __shfl_sync(CS_FULL, key[s > 0 ? s - 1 : 0], 31) : edge0;
+        const K carry1 = s + 1 < RUN_ITEMS
+                             ? __shfl_sync(CS_FULL, key[s + 1 < RUN_ITEMS ? s + 1 : 0], 0) : edge1;
+        if (lane == 0) prev = carry0;
+        if (lane == 31) next = carry1;
+        if (head) {
+            const int64_t o = out + __popc(hm & ((1u << lane) - 1));
+            float acc = v ? v[i] : 1.0f;
+            if (next == key[s])
+                for (int64_t j = i + 1; j < n && keys[j] == key[s]; ++j) acc += v ? v[j] : 1.0f;
+            const int32_t row = (int32_t)(key[s] >> cb);
+            out_ci[o] = (int32_t)(key[s] & (((K)1 << cb) - 1));
+            out_v[o] = acc;
+            for (int32_t r = i == 0 ? 0 : (int32_t)(prev >> cb) + 1; r <= row; ++r)
+                rp[r] = (int32_t)o;
+        }
+        if (i == n - 1)
+            for (int32_t r = (int32_t)(key[s] >> cb) + 1; r <= rows; ++r) rp[r] = out_n;
+        out += __popc(hm);
+    }
 }
 
 int bits_for(int64_t x) {  // bits to hold 0 .. x - 1
@@ -193,6 +432,127 @@ struct Bufs {
         n = 0;
     }
 };
+
+// The list sorted by key: keys and values (null: every value 1) on the device,
+// m entries, each tile's first run, and their count in Misc::scan_total.
+struct Sorted {
+    int64_t m = 0;
+    void* keys = nullptr;
+    float* vals = nullptr;
+    int64_t* tile_off = nullptr;
+};
+
+template <class K>
+size_t pass_smem(bool val) {
+    return CS_TILE * (sizeof(K) + (val ? 4 : 0)) + 2 * 2 * CS_WARPS * 256;
+}
+
+template <class K, class Src>
+void launch_pass(cudaStream_t s, int64_t n, const Src& src, const float* vals, const Digits& dg,
+                 int p, const uint32_t* starts, unsigned long long* status, int32_t* ticket,
+                 K* keys_out, float* vals_out, int32_t* err) {
+    const unsigned grid = (unsigned)((n + CS_TILE - 1) / CS_TILE);
+    if (vals)
+        k_coo_pass<K, Src, true><<<grid, CS_TPB, pass_smem<K>(true), s>>>(
+            n, src, vals, dg, p, starts, status, ticket, keys_out, vals_out, err);
+    else
+        k_coo_pass<K, Src, false><<<grid, CS_TPB, pass_smem<K>(false), s>>>(
+            n, src, vals, dg, p, starts, status, ticket, keys_out, vals_out, err);
+    note_launch(nullptr, 1);
+}
+
+template <class K>
+void set_pass_attrs() {
+    // (per device; a few calls, and only the first on a device changes anything)
+    const auto set = [](const void* f, bool val) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)pass_smem<K>(val));
+    };
+    set((const void*)k_coo_pass<K, CooKeys, true>, true);
+    set((const void*)k_coo_pass<K, CooKeys, false>, false);
+    set((const void*)k_coo_pass<K, ArrayKeys<K>, true>, true);
+    set((const void*)k_coo_pass<K, ArrayKeys<K>, false>, false);
+}
+
+template <class K>
+int sort_list(rvsp_cuda_plan* plan, Bufs& b, int32_t rows, int32_t cols, int64_t n, int cb, int rb,
+              const int32_t* d_r, const int32_t* d_c, const float* d_v, int symmetric,
+              Sorted* out) {
+    cudaStream_t s = plan->stream;
+    Misc* misc = plan->misc.as<Misc>();
+    cudaError_t e;
+    int st;
+    const CooKeys list{d_r, d_c, rows, cols, cb, &misc->err};
+    int64_t m = n;
+    int64_t* mpos = nullptr;
+    // expanded count of a symmetric list
+    if (symmetric && n > 0) {
+        int32_t* flag;
+        if ((e = b.get(&mpos, 8 * ((size_t)n + 1))) || (e = b.get(&flag, 4 * (size_t)n)))
+            return fail(e, "COO scratch");
+        k_offdiag<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, d_r, d_c, flag);
+        note_launch(nullptr, 1);
+        if ((st = scan_counts(plan, flag, n, mpos, nullptr, &misc->scan_total2))) return st;
+        if ((e = cudaMemcpyAsync(&m, &misc->scan_total2, 8, cudaMemcpyDeviceToHost, s)) ||
+            (e = cudaStreamSynchronize(s)))
+            return fail(e, "symmetric count");
+        m += n;
+    }
+    out->m = m;
+    if (m == 0) return RVSP_SUCCESS;
+    const int bits = cb + rb;
+    Digits dg{(bits + 7) / 8, 0};
+    dg.db = dg.passes ? (bits + dg.passes - 1) / dg.passes : 0;  // even digits: fewer, longer runs
+    const int64_t tiles = (m + CS_TILE - 1) / CS_TILE, rtiles = (m + RUN_TILE - 1) / RUN_TILE;
+    K *k0, *k1;
+    float *v0 = nullptr, *v1 = nullptr;
+    unsigned long long* work;  // counts, tickets, starts, then the tiles' words after a stop word
+    int32_t* runs;
+    const size_t fixed = 8 * CS_PASSES * 256 + 4 * CS_PASSES * 256 + 8 * CS_PASSES + 8;
+    const size_t work_bytes = fixed + (dg.passes ? 8 * 256 * (size_t)tiles : 0);
+    if ((e = b.get(&k0, sizeof(K) * (size_t)m)) || (e = b.get(&k1, sizeof(K) * (size_t)m)) ||
+        (d_v && ((e = b.get(&v0, 4 * (size_t)m)) || (e = b.get(&v1, 4 * (size_t)m)))) ||
+        (e = b.get(&work, work_bytes)) || (e = b.get(&runs, 4 * (size_t)rtiles)) ||
+        (e = b.get(&out->tile_off, 8 * ((size_t)rtiles + 1))))
+        return fail(e, "COO scratch");
+    unsigned long long* counts = work;
+    uint32_t* starts = reinterpret_cast<uint32_t*>(work + CS_PASSES * 256);
+    int32_t* tickets = reinterpret_cast<int32_t*>(starts + CS_PASSES * 256);
+    unsigned long long* status = reinterpret_cast<unsigned long long*>(tickets + 2 * CS_PASSES) + 1;
+    if ((e = cudaMemsetAsync(work, 0, work_bytes, s)) != cudaSuccess) return fail(e, "memset");
+    const bool direct = !symmetric && dg.passes > 0;  // the first pass reads the list itself
+    if (!direct) {
+        k_coo_keys<K><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, list, d_v, symmetric, mpos, k0,
+                                                                v0);
+        note_launch(nullptr, 1);
+    }
+    if (dg.passes > 0) {
+        set_pass_attrs<K>();
+        const unsigned grid = (unsigned)std::min<int64_t>((m + CS_TPB - 1) / CS_TPB, 148 * 6);
+        if (direct)
+            k_coo_digits<<<grid, CS_TPB, 0, s>>>(m, list, dg, counts);
+        else
+            k_coo_digits<<<grid, CS_TPB, 0, s>>>(m, ArrayKeys<K>{k0}, dg, counts);
+        k_coo_starts<<<dg.passes, 256, 0, s>>>(counts, starts);
+        note_launch(nullptr, 2);
+    }
+    const float* vin = direct ? d_v : v0;
+    for (int p = 0; p < dg.passes; ++p) {
+        if (direct && p == 0)
+            launch_pass<K>(s, m, list, vin, dg, p, starts, status, tickets + p, k1, v1, &misc->err);
+        else
+            launch_pass<K>(s, m, ArrayKeys<K>{k0}, vin, dg, p, starts, status, tickets + p, k1, v1,
+                           &misc->err);
+        std::swap(k0, k1);
+        std::swap(v0, v1);
+        vin = v0;
+    }
+    out->keys = k0;
+    out->vals = v0;
+    k_run_count<K><<<(unsigned)rtiles, CS_TPB, 0, s>>>(m, k0, runs);
+    note_launch(nullptr, 1);
+    return scan_counts(plan, runs, rtiles, out->tile_off, nullptr, &misc->scan_total);
+}
 
 thread_local rvsp_cuda_plan_t t_cplan = nullptr;
 struct CooReaper {
@@ -252,52 +612,25 @@ extern "C" int rvsp_cuda_coo_to_csr(int32_t rows, int32_t cols, int64_t n, const
         d_r = tr, d_c = tc, d_v = tv;
     }
     const int cb = bits_for(cols), rb = bits_for(rows);
-    const int passes = (cb + rb + 7) / 8;
-    uint64_t *k0, *k1;
-    int64_t *i0, *i1, *mpos, *opos;
-    int32_t *flag, *hist, *hoff, *head, *out_row, *rp, *ci;
-    float* v;
-    const int64_t nb = (total + RS_TILE - 1) / RS_TILE;
-    if ((e = b.get(&k0, 8 * (size_t)total)) || (e = b.get(&k1, 8 * (size_t)total)) ||
-        (e = b.get(&i0, 8 * (size_t)total)) || (e = b.get(&i1, 8 * (size_t)total)) ||
-        (e = b.get(&mpos, 8 * ((size_t)n + 1))) || (e = b.get(&flag, 4 * (size_t)n)) ||
-        (e = b.get(&hist, 4 * 256 * (size_t)nb)) || (e = b.get(&hoff, 4 * (256 * (size_t)nb + 1))) ||
-        (e = b.get(&head, 4 * (size_t)total)) || (e = b.get(&opos, 8 * ((size_t)total + 1))) ||
-        (e = b.get(&out_row, 4 * (size_t)total)))
-        return bail(fail(e, "COO scratch"));
-    // expanded count
-    int64_t m = n;
-    if (symmetric && n > 0) {
-        k_offdiag<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, d_r, d_c, flag);
-        if ((st = scan_counts(plan, flag, n, mpos, nullptr, &misc->scan_total2))) return bail(st);
-        if ((e = cudaMemcpyAsync(&m, &misc->scan_total2, 8, cudaMemcpyDeviceToHost, s)) ||
-            (e = cudaStreamSynchronize(s)))
-            return bail(fail(e, "symmetric count"));
-        m += n;
-    }
-    if (n > 0)
-        k_coo_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, rows, cols, cb, d_r, d_c,
-                                                               symmetric, mpos, k0, i0, &misc->err);
-    const int64_t mb = (m + RS_TILE - 1) / RS_TILE;
-    for (int p = 0; p < passes && m > 0; ++p) {
-        k_rs_hist<<<(unsigned)mb, RS_TPB, 0, s>>>(m, k0, 8 * p, hist);
-        if ((st = scan_counts(plan, hist, 256 * mb, nullptr, hoff, &misc->tile_total)))
-            return bail(st);
-        k_rs_scatter<<<(unsigned)mb, RS_TPB, 0, s>>>(m, k0, i0, 8 * p, hoff, k1, i1);
-        std::swap(k0, k1);
-        std::swap(i0, i1);
-    }
+    Sorted so;
+    st = cb + rb <= 32
+             ? sort_list<uint32_t>(plan, b, rows, cols, n, cb, rb, d_r, d_c, d_v, symmetric, &so)
+             : sort_list<uint64_t>(plan, b, rows, cols, n, cb, rb, d_r, d_c, d_v, symmetric, &so);
+    if (st) return bail(st);
+    const int64_t m = so.m;
     int64_t out_n = 0;
-    if (m > 0) {
-        k_run_heads<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, k0, head);
-        if ((st = scan_counts(plan, head, m, opos, nullptr, &misc->scan_total))) return bail(st);
-    }
     int32_t bad = 0;
+    int32_t *rp, *ci;
+    float* v;
     if ((e = cudaMemcpyAsync(&out_n, &misc->scan_total, 8, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaMemcpyAsync(&bad, &misc->err, 4, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
         return bail(fail(e, "COO sort"));
     if (m == 0) out_n = 0;
+    if (bad & COO_STUCK) {
+        g_err = "COO sort: a tile's wait ran out";
+        return bail(RVSP_ERROR_DEVICE_FAILURE);
+    }
     if (bad) {
         g_err = "COO row or column index out of range";
         return bail(RVSP_ERROR_INVALID_ARGUMENT);
@@ -311,10 +644,20 @@ extern "C" int rvsp_cuda_coo_to_csr(int32_t rows, int32_t cols, int64_t n, const
         if (ci) cudaFreeAsync(ci, s);
         return bail(fail(e, "CSR alloc"));
     }
-    if (m > 0)
-        k_run_sum<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, k0, i0, head, opos, cb, d_v,
-                                                              out_row, ci, v);
-    k_row_ptr_from_rows<<<(unsigned)((out_n + 256) / 256), 256, 0, s>>>(out_n, rows, out_row, rp);
+    if (m == 0) {
+        cudaMemsetAsync(rp, 0, 4 * ((size_t)rows + 1), s);
+    } else {
+        const unsigned grid = (unsigned)((m + RUN_TILE - 1) / RUN_TILE);
+        if (cb + rb <= 32)
+            k_run_write<uint32_t><<<grid, CS_TPB, 0, s>>>(m, (const uint32_t*)so.keys, so.vals,
+                                                          so.tile_off, cb, rows, (int32_t)out_n,
+                                                          rp, ci, v);
+        else
+            k_run_write<uint64_t><<<grid, CS_TPB, 0, s>>>(m, (const uint64_t*)so.keys, so.vals,
+                                                          so.tile_off, cb, rows, (int32_t)out_n,
+                                                          rp, ci, v);
+        note_launch(nullptr, 1);
+    }
     b.release();
     if ((e = cudaGetLastError()) != cudaSuccess) {
         cudaFreeAsync(rp, s);
