@@ -480,7 +480,7 @@ int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused) {
             return fail(e, "slots");
     }
     launch_bin_scatter(plan, plan->lbin.as<uint8_t>(), plan->ltile_off.as<int32_t>(),
-                       plan->lbin_rows.as<int32_t>(), false);
+                       plan->lbin_rows.as<int32_t>());
     if (fused && (st = scan_counts(plan, plan->lcap.as<int32_t>(), M, plan->slot_off.as<int64_t>(),
                                    nullptr, &misc->scan_total2)))
         return st;

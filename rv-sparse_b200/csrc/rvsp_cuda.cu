@@ -28,6 +28,7 @@
 #include "rvsp_internal.h"
 #include "spgemm_kernels.cuh"
 #include "sort_rows.cuh"
+#include "heavy_lists.cuh"
 
 using namespace rvsp;
 
@@ -213,19 +214,23 @@ static void set_mode_attrs() {
     set_warp_attr<4096, MODE>();
     cudaFuncSetAttribute(k_heavy<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          HEAVY_SMEM_MAX);
+    cudaFuncSetAttribute(k_heavy_list<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         HEAVY_SMEM_MAX);
 }
 
 // Heavy kernel shape for every mode and chunk width: warps per CTA chosen to
 // keep the most warps resident per SM (each warp holds its own accumulator
 // and bitmap in shared memory), and the resident CTAs per SM; the launches
 // fill the GPU once and the CTAs pull batches of work items from a counter.
-static int g_heavy_w[3][HEAVY_CW_LOG2_MAX + 1];
+// [0..2] k_heavy, [3..5] k_heavy_list, by mode
+static int g_heavy_w[6][HEAVY_CW_LOG2_MAX + 1];
 // dynamic shared memory of a heavy CTA of W warps: their accumulators and
 // bitmaps, then the CTA's work-batch word
 static size_t heavy_launch_smem(int mode, int cl, int W) {
-    return (size_t)W * heavy_smem_bytes(mode, 1 << cl) + 16;
+    return (size_t)W * (mode >= 3 ? list_smem_bytes(mode - 3, 1 << cl)
+                                  : heavy_smem_bytes(mode, 1 << cl)) + 16;
 }
-static int g_heavy_ctas[3][HEAVY_CW_LOG2_MAX + 1];
+static int g_heavy_ctas[6][HEAVY_CW_LOG2_MAX + 1];
 static int g_sms = 148;
 
 static std::once_flag g_attr_once;
@@ -238,11 +243,14 @@ void init_kernel_attributes() {
         if (cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
         for (int cl = HEAVY_CW_LOG2_MIN; cl <= HEAVY_CW_LOG2_MAX; ++cl) {
-            const void* fns[3] = {(const void*)k_heavy<COUNT>, (const void*)k_heavy<FILL>,
-                                  (const void*)k_heavy<REUSE>};
-            for (int m = 0; m < 3; ++m) {
+            const void* fns[6] = {(const void*)k_heavy<COUNT>, (const void*)k_heavy<FILL>,
+                                  (const void*)k_heavy<REUSE>, (const void*)k_heavy_list<COUNT>,
+                                  (const void*)k_heavy_list<FILL>,
+                                  (const void*)k_heavy_list<REUSE>};
+            for (int m = 0; m < 6; ++m) {
                 int best_w = 1, best_n = 1, best = 0;
                 for (int W = 1; W <= HEAVY_MAX_WARPS; ++W) {
+                    if (m >= 3 && W > LIST_MAX_WARPS) break;
                     const size_t bytes = heavy_launch_smem(m, cl, W);
                     if (bytes > (size_t)HEAVY_SMEM_MAX) break;
                     int n = 0;
@@ -393,21 +401,33 @@ static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             // row of the heavy items is kept heavy: no row mask to check)
             RowCtl ctl = o.ctl;
             const int cl = plan->params.heavy_cw_log2;
-            const int W = g_heavy_w[MODE][cl];
-            const int64_t fill = (int64_t)g_sms * g_heavy_ctas[MODE][cl];
+            const int shape = MODE + (plan->lists_ok ? 3 : 0);
+            const int W = g_heavy_w[shape][cl];
+            const int64_t fill = (int64_t)g_sms * g_heavy_ctas[shape][cl];
             const int grid = (int)std::min<int64_t>((plan->n_items + W - 1) / W, fill);
-            const HeavyAux aux{plan->bmeta.as<int4>(), plan->bdoff.as<int64_t>(),
-                               plan->dir_ok ? plan->bdir.as<int32_t>() : nullptr,
-                               plan->ameta_ok ? plan->ameta.as<int4>() : nullptr,
-                               plan->ameta_ok ? plan->adoff.as<int32_t>() : nullptr,
-                               plan->smask_words ? plan->bsmask.as<uint32_t>() : nullptr,
-                               plan->smask_words};
+            const size_t bytes = heavy_launch_smem(shape, cl, W);
             int32_t* queue = &plan->misc.as<Misc>()->heavy_queue;
             cudaMemsetAsync(queue, 0, sizeof(int32_t), plan->stream);
-            k_heavy<MODE><<<grid, W * 32, heavy_launch_smem(MODE, cl, W), plan->stream>>>(
-                A, B, plan->items.as<HeavyItem>(), plan->n_items, plan->item_cnt.as<int32_t>(),
-                o.cnt, plan->item_scan.as<int64_t>(), o.c_rp, o.c_ci, o.c_v, o.err, ctl, cl,
-                aux, queue);
+            if (plan->lists_ok) {
+                const HeavyLists L{plan->item_seg.as<int64_t>(), plan->seg.as<int2>(),
+                                   plan->item_prod.as<int32_t>(), plan->work.as<int2>(),
+                                   &plan->misc.as<Misc>()->nwork};
+                k_heavy_list<MODE><<<grid, W * 32, bytes, plan->stream>>>(
+                    A, B, plan->items.as<HeavyItem>(), plan->n_items, L,
+                    plan->item_cnt.as<int32_t>(), o.cnt, plan->item_scan.as<int64_t>(), o.c_rp,
+                    o.c_ci, o.c_v, o.err, ctl, cl, queue);
+            } else {
+                const HeavyAux aux{plan->bmeta.as<int4>(), plan->bdoff.as<int64_t>(),
+                                   plan->dir_ok ? plan->bdir.as<int32_t>() : nullptr,
+                                   plan->ameta_ok ? plan->ameta.as<int4>() : nullptr,
+                                   plan->ameta_ok ? plan->adoff.as<int32_t>() : nullptr,
+                                   plan->smask_words ? plan->bsmask.as<uint32_t>() : nullptr,
+                                   plan->smask_words};
+                k_heavy<MODE><<<grid, W * 32, bytes, plan->stream>>>(
+                    A, B, plan->items.as<HeavyItem>(), plan->n_items, plan->item_cnt.as<int32_t>(),
+                    o.cnt, plan->item_scan.as<int64_t>(), o.c_rp, o.c_ci, o.c_v, o.err, ctl, cl,
+                    aux, queue);
+            }
             note_launch(plan, 1);
         }
     }
@@ -575,9 +595,159 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     ENS(plan->item_scan, ((size_t)plan->n_items + 1) * 8);
 #undef ENS
     launch_bin_scatter(plan, plan->bin.as<uint8_t>(), plan->tile_off.as<int32_t>(),
-                       plan->bin_rows.as<int32_t>(), true);
+                       plan->bin_rows.as<int32_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "analysis launch");
-    if (plan->n_items > 0 && (st = build_heavy_aux(plan, A, B))) return st;
+    if (plan->n_items > 0) {
+        if ((st = build_heavy_lists(plan, A, B))) return st;
+        if (!plan->lists_ok && (st = build_heavy_aux(plan, A, B))) return st;
+    }
+    return RVSP_SUCCESS;
+}
+
+// The heavy rows' work items, and their segment lists (heavy_lists.cuh) unless
+// B has too many chunks for a unit's counters, an A row has too many entries
+// for a segment's word, or the lists would pass LIST_MAX_SEGS segments (8
+// bytes each) or not fit: lists_ok says whether they exist. One device->host
+// read of their size.
+constexpr int64_t LIST_MAX_SEGS = int64_t(1) << 30;
+constexpr int64_t LIST_MAX_CELLS = int64_t(1) << 28;
+int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
+    const int nh = plan->bin_count[BIN_HEAVY];
+    const int cl = plan->params.heavy_cw_log2;
+    const int64_t K = plan->b_rows, Z = plan->b_nnz;
+    const int64_t chunks = ((int64_t)plan->b_cols + (1 << cl) - 1) >> cl;
+    const int64_t units = plan->host_misc.totals[2], cells = plan->host_misc.totals[3];
+    const int64_t tiles = (Z + 1 + RUNS_TILE - 1) / RUNS_TILE;  // (Z itself has a word too)
+    const int32_t* rows = plan->bin_rows.as<int32_t>() + plan->offs.off[BIN_HEAVY];
+    Misc* misc = plan->misc.as<Misc>();
+    cudaError_t e;
+    int st;
+#define ENS(buf, bytes) \
+    if ((e = (buf).ensure(bytes)) != cudaSuccess) return fail(e, "heavy rows " #buf)
+    ENS(plan->hchunks, (size_t)nh * 4);
+    ENS(plan->hunits, (size_t)nh * 4);
+    ENS(plan->hcells, (size_t)nh * 4);
+    ENS(plan->hitem0, ((size_t)nh + 1) * 4);
+    ENS(plan->hunit0, ((size_t)nh + 1) * 4);
+    ENS(plan->hcell0, ((size_t)nh + 1) * 8);
+#undef ENS
+    const size_t bits_bytes = ((size_t)Z / 32 + 1) * 4;
+    bool lists = chunks <= LIST_MAX_CHUNKS && units <= INT32_MAX && cells <= LIST_MAX_CELLS &&
+                 plan->brow_bits.ensure(bits_bytes) == cudaSuccess &&
+                 plan->brun_cnt.ensure((size_t)tiles * 4) == cudaSuccess &&
+                 plan->brun_off.ensure(((size_t)tiles + 1) * 8) == cudaSuccess &&
+                 plan->brun_words.ensure((size_t)tiles * (RUNS_TILE / 32) * 8) == cudaSuccess &&
+                 plan->bruns.ensure((size_t)Z * 8) == cudaSuccess &&
+                 plan->brows.ensure((size_t)K * 16) == cudaSuccess &&
+                 plan->cell_cnt.ensure((size_t)cells * 4) == cudaSuccess &&
+                 plan->cell_prod.ensure((size_t)cells * 4) == cudaSuccess &&
+                 plan->work.ensure((size_t)plan->n_items * 8) == cudaSuccess &&
+                 plan->item_prod.ensure((size_t)plan->n_items * 4) == cudaSuccess &&
+                 plan->cell_off.ensure(((size_t)cells + 1) * 8) == cudaSuccess &&
+                 plan->item_seg.ensure(((size_t)plan->n_items + 1) * 8) == cudaSuccess;
+    cudaGetLastError();  // a refused allocation leaves the lookups
+    {
+        KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+        k_heavy_rows<<<(nh + 255) / 256, 256, 0, plan->stream>>>(
+            A, rows, nh, plan->nchunks.as<int32_t>(), plan->hchunks.as<int32_t>(),
+            plan->hunits.as<int32_t>(), plan->hcells.as<int32_t>(), &misc->longest, &misc->err);
+        note_launch(plan, 1);
+    }
+    if ((st = scan_counts(plan, plan->hchunks.as<int32_t>(), nh, nullptr,
+                          plan->hitem0.as<int32_t>(), &misc->tile_total)))
+        return st;
+    const unsigned hgrid = (unsigned)(((int64_t)nh * 32 + 255) / 256);
+    const unsigned lgrid = (unsigned)((units + ALIST_WARPS - 1) / ALIST_WARPS);
+    int64_t total = 0;
+    if (lists) {
+        if ((st = scan_counts(plan, plan->hunits.as<int32_t>(), nh, nullptr,
+                              plan->hunit0.as<int32_t>(), &misc->tile_total)) ||
+            (st = scan_counts(plan, plan->hcells.as<int32_t>(), nh, plan->hcell0.as<int64_t>(),
+                              nullptr, &misc->tile_total)))
+            return st;
+        const unsigned kgrid = (unsigned)((K + 255) / 256);
+        if ((e = cudaMemsetAsync(plan->brow_bits.p, 0, bits_bytes, plan->stream)) != cudaSuccess)
+            return fail(e, "memset");
+        {
+            KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+            k_row_starts<<<kgrid, 256, 0, plan->stream>>>(B, plan->brow_bits.as<uint32_t>(),
+                                                          &misc->err);
+            k_chunk_runs<COUNT><<<(unsigned)tiles, RUNS_TPB, 0, plan->stream>>>(
+                B, cl, plan->brow_bits.as<uint32_t>(), plan->brun_cnt.as<int32_t>(), nullptr,
+                nullptr, nullptr, &misc->err);
+            note_launch(plan, 2);
+        }
+        if ((st = scan_counts(plan, plan->brun_cnt.as<int32_t>(), tiles,
+                              plan->brun_off.as<int64_t>(), nullptr, &misc->tile_total)))
+            return st;
+        {
+            KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+            k_chunk_runs<FILL><<<(unsigned)tiles, RUNS_TPB, 0, plan->stream>>>(
+                B, cl, plan->brow_bits.as<uint32_t>(), nullptr, plan->brun_off.as<int64_t>(),
+                plan->bruns.as<int2>(), plan->brun_words.as<int2>(), &misc->err);
+            k_row_runs<<<kgrid, 256, 0, plan->stream>>>(B, plan->brun_words.as<int2>(),
+                                                        plan->brows.as<int4>(), &misc->err);
+            note_launch(plan, 2);
+        }
+        {
+            KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+            k_alist_count<<<lgrid, ALIST_WARPS * 32, (size_t)ALIST_WARPS * 4 * (size_t)chunks,
+                            plan->stream>>>(
+                A, B, rows, nh, (int)units, plan->hunit0.as<int32_t>(), plan->hunits.as<int32_t>(),
+                plan->hcell0.as<int64_t>(), cells, plan->chunk_lo.as<int32_t>(),
+                plan->nchunks.as<int32_t>(), plan->brows.as<int4>(), plan->bruns.as<int2>(), cl,
+                plan->cell_cnt.as<int32_t>(), plan->cell_prod.as<int32_t>(), &misc->err,
+                (int)chunks);
+            note_launch(plan, 1);
+        }
+        if ((st = scan_counts(plan, plan->cell_cnt.as<int32_t>(), cells,
+                              plan->cell_off.as<int64_t>(), nullptr, &misc->dir_total)))
+            return st;
+        struct {
+            int64_t total;
+            int32_t longest;
+        } got = {0, 0};
+        if ((e = cudaMemcpyAsync(&got, &misc->dir_total, 12, cudaMemcpyDeviceToHost,
+                                 plan->stream)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(plan->stream)) != cudaSuccess)
+            return fail(e, "segment lists");
+        total = got.total;
+        lists = total <= LIST_MAX_SEGS && got.longest <= INT32_MAX >> cl &&
+                plan->seg.ensure((size_t)total * 8) == cudaSuccess;
+        cudaGetLastError();
+    }
+    {
+        KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+        if (lists) {
+            k_alist_fill<<<lgrid, ALIST_WARPS * 32, 0, plan->stream>>>(
+                A, B, rows, nh, (int)units, plan->hunit0.as<int32_t>(), plan->hunits.as<int32_t>(),
+                plan->hcell0.as<int64_t>(), cells, plan->chunk_lo.as<int32_t>(),
+                plan->nchunks.as<int32_t>(), plan->brows.as<int4>(), plan->bruns.as<int2>(),
+                plan->cell_off.as<int64_t>(), plan->seg.as<int2>(), total, cl, &misc->err,
+                (int)chunks);
+            note_launch(plan, 1);
+        }
+        k_heavy_items<<<hgrid, 256, 0, plan->stream>>>(
+            A.rp, rows, nh, plan->hitem0.as<int32_t>(), plan->chunk_lo.as<int32_t>(),
+            plan->nchunks.as<int32_t>(), plan->hcell0.as<int64_t>(), plan->hunits.as<int32_t>(),
+            plan->cell_off.as<int64_t>(), plan->cell_prod.as<int32_t>(), cells, plan->n_items, cl,
+            plan->items.as<HeavyItem>(), lists ? plan->item_seg.as<int64_t>() : nullptr,
+            plan->item_prod.as<int32_t>(), plan->hchunks.as<int32_t>());
+        note_launch(plan, 1);
+    }
+    if (lists) {
+        if ((st = scan_counts(plan, plan->hchunks.as<int32_t>(), nh, nullptr,
+                              plan->hunit0.as<int32_t>(), &misc->nwork)))
+            return st;
+        KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+        k_heavy_work<<<hgrid, 256, 0, plan->stream>>>(
+            rows, nh, plan->hitem0.as<int32_t>(), plan->nchunks.as<int32_t>(),
+            plan->item_prod.as<int32_t>(), plan->hunit0.as<int32_t>(), plan->n_items, cl,
+            plan->work.as<int2>());
+        note_launch(plan, 1);
+    }
+    plan->lists_ok = lists;
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "heavy rows launch");
     return RVSP_SUCCESS;
 }
 
@@ -665,16 +835,13 @@ int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     return RVSP_SUCCESS;
 }
 
-// Stable partition of the plan's rows by bin (k_bin_scatter); with
-// heavy_items the heavy rows also get their column-chunk work items.
+// Stable partition of the plan's rows by bin (k_bin_scatter).
 void launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* tile_off,
-                        int32_t* bin_rows, bool heavy_items) {
+                        int32_t* bin_rows) {
     const int64_t M = plan->a_rows;
-    Misc* misc = plan->misc.as<Misc>();
     KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
     k_bin_scatter<<<(unsigned)((M + AN_TILE - 1) / AN_TILE), AN_TILE, 0, plan->stream>>>(
-        (int32_t)M, bin, tile_off, plan->chunk_lo.as<int32_t>(), plan->nchunks.as<int32_t>(),
-        bin_rows, &misc->item_cursor, heavy_items ? plan->items.as<HeavyItem>() : nullptr);
+        (int32_t)M, bin, tile_off, bin_rows);
     note_launch(plan, 1);
 }
 
@@ -903,7 +1070,10 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t p) {
                       &p->list_off, &p->lbin, &p->lcap, &p->ltile_hist, &p->ltile_off,
                       &p->lbin_rows, &p->need, &p->pflag, &p->hmask, &p->hovf,
                       &p->item_off, &p->bmeta, &p->bdcount, &p->bdscan, &p->bdoff, &p->bdir,
-                      &p->ameta, &p->adoff, &p->bsmask};
+                      &p->ameta, &p->adoff, &p->bsmask, &p->hchunks, &p->hunits, &p->hcells,
+                      &p->hitem0, &p->hunit0, &p->hcell0, &p->brow_bits, &p->brun_cnt,
+                      &p->brun_off, &p->brun_words, &p->bruns, &p->brows, &p->cell_cnt,
+                      &p->cell_off, &p->item_seg, &p->seg, &p->cell_prod, &p->item_prod, &p->work};
     for (DevBuf* b : bufs) b->release();
     if (p->side) {
         cudaStreamSynchronize(p->side);

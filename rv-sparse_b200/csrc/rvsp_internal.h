@@ -29,8 +29,8 @@ struct DevBuf {
 struct Misc {
     int32_t hist[NUM_BINS];    // rows per bin
     int32_t cursor[NUM_BINS];  // bin scatter cursors
-    int64_t totals[2];         // heavy items, products
-    int32_t item_cursor;
+    int64_t totals[4];         // heavy items, products, heavy units, heavy cells
+    int32_t pad0;
     int32_t overflow;          // a 32-bit row pointer would overflow
     int64_t scan_total;        // nnz(C)
     int64_t scan_total2;       // heavy item total / learned capacity total
@@ -48,7 +48,10 @@ struct Misc {
     int64_t slot_total;        // learned path: sum of predicted capacities
     int64_t lstats[8];         // learned path statistics (see rvsp_cuda_plan_learned_stats)
     int64_t ltile_total;
-    int64_t dir_total;         // heavy-row B directory entries
+    int64_t dir_total;         // heavy-row B directory entries, or listed segments
+    int32_t longest;           // entries of the longest heavy row of A
+    int32_t pad3;
+    int64_t nwork;             // heavy rows: entries of the work list
     int32_t heavy_queue;       // next heavy work item of the running launch
     int32_t row_queue;         // next row of the running warp-bin launch
     unsigned long long pool_fill;  // learned path: entries placed in the overflow pool
@@ -164,6 +167,12 @@ struct rvsp_cuda_plan {
     rvsp::DevBuf bmeta, bdcount, bdscan, bdoff, bdir;
     rvsp::DevBuf ameta, adoff;  // per A entry of heavy rows (HeavyAux)
     rvsp::DevBuf bsmask;        // chunk presence of B rows without a directory
+    // heavy rows' segment lists (heavy_lists.cuh), lists_ok when they exist
+    // (the kernels look segments up through the fields above otherwise)
+    rvsp::DevBuf hchunks, hunits, hcells, hitem0, hunit0, hcell0;
+    rvsp::DevBuf brow_bits, brun_cnt, brun_off, brun_words, bruns, brows;
+    rvsp::DevBuf cell_cnt, cell_prod, cell_off, item_seg, item_prod, work, seg;
+    bool lists_ok = false;
     bool ameta_ok = false;
     bool dir_ok = false;
     int32_t smask_words = 0;    // words per B row of bsmask, 0: no masks
@@ -237,8 +246,9 @@ int scan_counts(rvsp_cuda_plan* plan, const int32_t* in, int64_t n, int64_t* out
 void note_launch(rvsp_cuda_plan* plan, int n);
 void reset_graph(rvsp_cuda_plan* plan);
 int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
+int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 void launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* tile_off,
-                        int32_t* bin_rows, bool heavy_items);
+                        int32_t* bin_rows);
 int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused);
 int learned_finish(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* c_ci,
                    float* c_v);

@@ -7,14 +7,15 @@
 //
 //   k_analyze      per-row op count (rvsp_symbolic.c:41), upper bound on the
 //                  row's distinct columns, learned-model features, bin id
-//   k_bin_scatter  rows grouped by bin; heavy rows expanded into
-//                  (row, column-chunk) work items
+//   k_bin_scatter  rows grouped by bin
 //   k_tiny<MODE>   thread per row, rows with <= 32 products
 //   k_sort<E,NW,..> 1, 2 or 4 warps per row, rows of up to 2048 products sorted
 //                  in registers (sort_rows.cuh)
 //   k_warp<CAP,..> warp per row, shared-memory hash table of CAP slots
 //   k_heavy<..>    warp per (row, column chunk), dense shared-memory
-//                  accumulator + occupancy bitmap over CW columns
+//                  accumulator + occupancy bitmap over CW columns; k_heavy_list
+//                  (heavy_lists.cuh) walks listed segments instead of looking
+//                  them up
 //   k_scan_*       exclusive scan of row counts into C's row pointer
 //
 // Each row kernel runs in one of three modes:
@@ -144,7 +145,7 @@ struct AnalyzeOut {
     float4* feat;        // [rows] learned-model features (optional)
     int32_t* hist;       // [NUM_BINS] rows per bin
     int32_t* tile_hist;  // [NUM_BINS][tiles] rows per bin per tile (stable binning)
-    int64_t* totals;     // [0] heavy items, [1] products
+    int64_t* totals;     // [0] heavy items, [1] products, [2] heavy units, [3] heavy cells
     int64_t* bin_prod;   // [NUM_BINS] products per bin
     int32_t* err;        // ERR_* bits
     int32_t* nnz_ab;     // [2] nnz of A and B as the kernel used them (read back with the bins)
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(AN_TILE)
     __shared__ int32_t s_maxc[AN_TILE];
     __shared__ int32_t s_hist[NUM_BINS];
     __shared__ unsigned long long s_bprod[NUM_BINS];
-    __shared__ unsigned long long s_items, s_prod;
+    __shared__ unsigned long long s_items, s_prod, s_units, s_cells;
     __shared__ int s_long;
 
     // An operand's nnz passed as -1 is not known on the host (a device-
@@ -212,6 +213,8 @@ __global__ void __launch_bounds__(AN_TILE)
     if (t == 0) {
         s_items = 0;
         s_prod = 0;
+        s_units = 0;
+        s_cells = 0;
         s_long = 0;
     }
     __syncthreads();
@@ -274,56 +277,80 @@ __global__ void __launch_bounds__(AN_TILE)
         // instead of 32 lanes contending for the same shared counters
         const int p0 = max(s_rp[0], 0), p1 = min(s_rp[nr], A.nnz);
         const int lane = t & 31;
-        for (int base = p0 + (t & ~31); base < p1; base += blockDim.x) {
-            const int p = base + lane;
-            int lo = -1, len = 0, first = INT_MAX, last = -1;
-            if (p < p1) {
-                int l = 0, h = nr;  // largest i with s_rp[i] <= p
-                while (h - l > 1) {
-                    const int mid = (l + h) >> 1;
-                    if (s_rp[mid] <= p) l = mid; else h = mid;
-                }
-                if (s_rp[l + 1] - s_rp[l] > AN_SHORT) {
-                    int bs, be;
-                    row_range(B, A.ci[p], &bs, &be, out.err);
-                    if (be > bs) {
-                        const int f = B.ci[bs], g = B.ci[be - 1];
-                        if (f < 0 || g >= B.cols || g < f) {
-                            atomicOr(out.err, ERR_STRUCTURE);
-                        } else {
-                            lo = l;
-                            len = be - bs;
-                            first = f;
-                            last = g;
-                        }
+        // four entries a thread, their three dependent loads in flight
+        // together: a tile of hub rows is one CTA's (R-MAT 2^17: 0.78 ms of
+        // the analysis with one entry a thread)
+        for (int base0 = p0 + (t & ~31); base0 < p1; base0 += 4 * blockDim.x) {
+            int lo[4], len[4], first[4], last[4], k[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int64_t p = (int64_t)base0 + u * (int)blockDim.x + lane;
+                lo[u] = -1;
+                len[u] = 0;
+                first[u] = INT_MAX;
+                last[u] = -1;
+                k[u] = -1;
+                if (p < p1) {
+                    int l = 0, h = nr;  // largest i with s_rp[i] <= p
+                    while (h - l > 1) {
+                        const int mid = (l + h) >> 1;
+                        if (s_rp[mid] <= p) l = mid; else h = mid;
+                    }
+                    if (s_rp[l + 1] - s_rp[l] > AN_SHORT) {
+                        lo[u] = l;
+                        k[u] = A.ci[p];
                     }
                 }
             }
-            const unsigned has = __ballot_sync(FULL, lo >= 0);
-            if (!has) continue;
-            const int lead = __ffs(has) - 1;
-            const int lrow = __shfl_sync(FULL, lo, lead);
-            if (__all_sync(FULL, lo < 0 || lo == lrow)) {
-                unsigned long long sum = (unsigned long long)len;
-                int mxl = len, mnc = first, mxc = last;
+            int bs[4], be[4];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    sum += __shfl_xor_sync(FULL, sum, o);
-                    mxl = max(mxl, __shfl_xor_sync(FULL, mxl, o));
-                    mnc = min(mnc, __shfl_xor_sync(FULL, mnc, o));
-                    mxc = max(mxc, __shfl_xor_sync(FULL, mxc, o));
+            for (int u = 0; u < 4; ++u) {
+                bs[u] = be[u] = 0;
+                if (lo[u] >= 0) row_range(B, k[u], &bs[u], &be[u], out.err);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                int f = 0, g = -1;
+                if (be[u] > bs[u]) {
+                    f = B.ci[bs[u]];
+                    g = B.ci[be[u] - 1];
                 }
-                if (lane == lead) {
-                    atomicAdd(&s_ops[lrow], sum);
-                    atomicMax(&s_maxlen[lrow], mxl);
-                    atomicMin(&s_minc[lrow], mnc);
-                    atomicMax(&s_maxc[lrow], mxc);
+                if (be[u] <= bs[u]) {
+                    lo[u] = -1;
+                } else if (f < 0 || g >= B.cols || g < f) {
+                    atomicOr(out.err, ERR_STRUCTURE);
+                    lo[u] = -1;
+                } else {
+                    len[u] = be[u] - bs[u];
+                    first[u] = f;
+                    last[u] = g;
                 }
-            } else if (lo >= 0) {
-                atomicAdd(&s_ops[lo], (unsigned long long)len);
-                atomicMax(&s_maxlen[lo], len);
-                atomicMin(&s_minc[lo], first);
-                atomicMax(&s_maxc[lo], last);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned has = __ballot_sync(FULL, lo[u] >= 0);
+                if (!has) continue;
+                const int lead = __ffs(has) - 1;
+                const int lrow = __shfl_sync(FULL, lo[u], lead);
+                if (__all_sync(FULL, lo[u] < 0 || lo[u] == lrow)) {
+                    unsigned long long sum = (unsigned long long)len[u];
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+                    const int mxl = __reduce_max_sync(FULL, len[u]);
+                    const int mnc = __reduce_min_sync(FULL, first[u]);
+                    const int mxc = __reduce_max_sync(FULL, last[u]);
+                    if (lane == lead) {
+                        atomicAdd(&s_ops[lrow], sum);
+                        atomicMax(&s_maxlen[lrow], mxl);
+                        atomicMin(&s_minc[lrow], mnc);
+                        atomicMax(&s_maxc[lrow], mxc);
+                    }
+                } else if (lo[u] >= 0) {
+                    atomicAdd(&s_ops[lo[u]], (unsigned long long)len[u]);
+                    atomicMax(&s_maxlen[lo[u]], len[u]);
+                    atomicMin(&s_minc[lo[u]], first[u]);
+                    atomicMax(&s_maxc[lo[u]], last[u]);
+                }
             }
         }
         __syncthreads();
@@ -355,6 +382,15 @@ __global__ void __launch_bounds__(AN_TILE)
     warp_bin_add(b, NUM_BINS, (unsigned long long)ops, s_hist, s_bprod);
     const unsigned long long wprod = warp_sum64((unsigned long long)ops);
     const unsigned long long witems = warp_sum64((unsigned long long)nch);
+    if (__any_sync(FULL, nch > 0)) {  // heavy rows: their units and (chunk, unit) cells
+        const unsigned long long u =
+            nch > 0 ? (unsigned long long)(s_rp[t + 1] - s_rp[t] + HEAVY_UNIT - 1) / HEAVY_UNIT : 0ull;
+        const unsigned long long wu = warp_sum64(u), wc = warp_sum64(u * (unsigned long long)nch);
+        if (lane_id() == 0) {
+            atomicAdd(&s_units, wu);
+            atomicAdd(&s_cells, wc);
+        }
+    }
     if (lane_id() == 0) {
         if (wprod) atomicAdd(&s_prod, wprod);
         if (witems) atomicAdd(&s_items, witems);
@@ -366,20 +402,21 @@ __global__ void __launch_bounds__(AN_TILE)
         if (s_bprod[t]) atomicAdd((unsigned long long*)&out.bin_prod[t], s_bprod[t]);
     }
     if (t == 0) {
-        if (s_items) atomicAdd((unsigned long long*)&out.totals[0], s_items);
+        if (s_items) {
+            atomicAdd((unsigned long long*)&out.totals[0], s_items);
+            atomicAdd((unsigned long long*)&out.totals[2], s_units);
+            atomicAdd((unsigned long long*)&out.totals[3], s_cells);
+        }
         atomicAdd((unsigned long long*)&out.totals[1], s_prod);
     }
 }
 
 // Stable partition of rows by bin: tile_off[b * tiles + tile] is where the
 // tile's rows of bin b start in bin_rows (an exclusive scan of tile_hist), so
-// every bin lists its rows in ascending order. Heavy rows reserve a block of
-// consecutive work items.
+// every bin lists its rows in ascending order.
 __global__ void __launch_bounds__(AN_TILE)
     k_bin_scatter(int32_t rows, const uint8_t* __restrict__ bin,
-                  const int32_t* __restrict__ tile_off, const int32_t* __restrict__ chunk_lo,
-                  const int32_t* __restrict__ nchunks, int32_t* __restrict__ bin_rows,
-                  int32_t* __restrict__ item_cursor, HeavyItem* __restrict__ items) {
+                  const int32_t* __restrict__ tile_off, int32_t* __restrict__ bin_rows) {
     __shared__ int32_t s_wc[AN_TILE / 32][NUM_BINS];
     const int t = threadIdx.x, lane = lane_id(), warp = t >> 5;
     const int row = blockIdx.x * AN_TILE + t;
@@ -395,12 +432,6 @@ __global__ void __launch_bounds__(AN_TILE)
     const int pos = tile_off[b * gridDim.x + blockIdx.x] + before +
                     __popc(peers & ((1u << lane) - 1));
     bin_rows[pos] = row;
-    if (b == BIN_HEAVY && items) {
-        const int n = nchunks[row];
-        const int first = atomicAdd(item_cursor, n);
-        const int lo = chunk_lo[row];
-        for (int c = 0; c < n; ++c) items[first + c] = HeavyItem{row, lo + c, first, 0};
-    }
 }
 
 // Per-row product counts in bin-list order (int32; rows beyond INT32_MAX

@@ -50,6 +50,7 @@ constexpr int BIN_HEAVY = BIN_WARP0 + NUM_WARP_BINS;
 constexpr int NUM_BINS = BIN_HEAVY + 1;
 constexpr int HEAVY_CW_LOG2_MIN = 9;    // heavy column chunks: 512 ..
 constexpr int HEAVY_CW_LOG2_MAX = 13;   // .. 8192 columns per work item
+constexpr int HEAVY_UNIT = 64;          // A entries of a heavy row listed by one warp
 constexpr int AN_TILE = 256;    // rows per analysis / binning tile
 
 // Runtime bin parameters of a plan.
@@ -81,7 +82,7 @@ struct HeavyItem {
     int32_t row;
     int32_t chunk;
     int32_t first;  // index of the row's first item
-    int32_t pad;
+    int32_t a0;     // where the row starts in A
 };
 
 // Per-B-row lookups for the heavy kernel, built by the analysis when the
