@@ -11,7 +11,12 @@
 // entries whose sum is exactly zero are not stored (the FP32 path keeps
 // them, as the reference's FP32 path does).
 //
-// Pipeline: the structure comes from the FP32 machinery (exact analysis,
+// Pipeline: where every row has at most 2048 products (the sort bins), the
+// analysis is followed by one pass of the sorting kernel on the typed values
+// (k_sort, sort_rows.cuh), which leaves each row's columns and nonzero sums in
+// a slot of its upper bound; the slots are then copied into C. 100k x 100k, 12
+// a row, FP64: 0.95 ms by the general way below, 0.37 ms so.
+// Otherwise the structure comes from the FP32 machinery (exact analysis,
 // count, fill with zero-valued operands, which only the column indices of
 // are used); a warp per output row then recomputes the values in the typed
 // arithmetic, positions found by binary search in the row's sorted columns
@@ -229,6 +234,43 @@ __global__ void k_nonzero_compact(int32_t rows, const int32_t* __restrict__ c_rp
     }
 }
 
+// Rows from their slots into C, 16 lanes a row.
+template <class T>
+__global__ void __launch_bounds__(256)
+    k_slots_to_rows(int32_t rows, const int64_t* __restrict__ slot_off,
+                    const int32_t* __restrict__ slot_ci, const T* __restrict__ slot_v,
+                    const int32_t* __restrict__ rp, int32_t* __restrict__ ci,
+                    T* __restrict__ v) {
+    const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4);
+    const int lane = threadIdx.x & 15;
+    if (row >= rows) return;
+    const int64_t src = slot_off[row];
+    const int dst = rp[row], n = rp[row + 1] - dst;
+    for (int x0 = lane; x0 < n; x0 += 64) {
+        int32_t c[4];
+        T y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int x = x0 + 16 * u;
+            if (x < n) {
+                c[u] = slot_ci[src + x];
+                y[u] = slot_v[src + x];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int x = x0 + 16 * u;
+            if (x < n) {
+                ci[dst + x] = c[u];
+                v[dst + x] = y[u];
+            }
+        }
+    }
+}
+
+// Products whose slots (12 bytes a product at most) the sorting pass may take.
+constexpr int64_t TYPED_SLOT_PRODUCTS = int64_t(1) << 29;
+
 thread_local rvsp_cuda_plan_t t_tplan = nullptr;
 
 struct TypedReaper {
@@ -288,16 +330,13 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
     cudaStream_t s = plan->stream;
     const bool dev = is_dev(a_rp);
     cudaError_t e;
-    int32_t a_nnz = 0, b_nnz = 0;
-    if (dev) {
-        if ((e = cudaMemcpy(&a_nnz, a_rp + a_rows, 4, cudaMemcpyDeviceToHost)) != cudaSuccess ||
-            (e = cudaMemcpy(&b_nnz, b_rp + a_cols, 4, cudaMemcpyDeviceToHost)) != cudaSuccess)
-            return fail(e, "row_ptr read");
-    } else {
+    // (device operands' nnz are read by the analysis)
+    int32_t a_nnz = -1, b_nnz = -1;
+    if (!dev) {
         a_nnz = a_rp[a_rows];
         b_nnz = b_rp[a_cols];
+        if (a_nnz < 0 || b_nnz < 0) return RVSP_ERROR_INVALID_CSR;
     }
-    if (a_nnz < 0 || b_nnz < 0) return RVSP_ERROR_INVALID_CSR;
     Scratch sc(s);
     auto bail = [&](int code) {
         sc.release();
@@ -323,37 +362,61 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
         cudaMemcpyAsync(t5, b_v, sizeof(In) * (size_t)b_nnz, cudaMemcpyHostToDevice, s);
         d_arp = t0, d_aci = t1, d_brp = t2, d_bci = t3, d_av = t4, d_bv = t5;
     }
-    // structure: exact analysis and count, then a fill on zero-valued operands
-    int64_t nnz = 0;
-    size_t ws = 0;
-    if ((st = rvsp_cuda_symbolic(plan, a_rows, a_cols, a_nnz, d_arp, d_aci, a_cols, b_cols, b_nnz,
-                                 d_brp, d_bci, &nnz, &ws)))
-        return bail(st);
-    float* zeros;
-    int32_t *s_rp, *s_ci, *cnt, *o_rp;
-    float* s_fv;
-    Out* s_v;
-    const size_t zn = (size_t)std::max(a_nnz, b_nnz) + 1, cn = (size_t)(nnz > 0 ? nnz : 1);
-    if ((e = sc.get(&zeros, 4 * zn)) || (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) ||
-        (e = sc.get(&s_ci, 4 * cn)) || (e = sc.get(&s_fv, 4 * cn)) ||
-        (e = sc.get(&s_v, sizeof(Out) * cn)) || (e = sc.get(&cnt, 4 * (size_t)a_rows)) ||
-        (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
-        return bail(fail(e, "typed scratch"));
-    cudaMemsetAsync(zeros, 0, 4 * zn, s);
-    if ((st = rvsp_cuda_numeric(plan, d_arp, d_aci, zeros, d_brp, d_bci, zeros, s_rp, s_ci, s_fv, 1,
-                                nullptr)))
-        return bail(st);
-    // typed values on that structure
+    plan->analysed = false;
+    plan->maps_ready = false;
+    plan->filled = nullptr;
+    plan->filled_host = nullptr;
+    reset_graph(plan);
+    plan->a_rows = a_rows;
+    plan->a_cols = a_cols;
+    plan->a_nnz = a_nnz;
+    plan->b_rows = a_cols;
+    plan->b_cols = b_cols;
+    plan->b_nnz = b_nnz;
+    memset(plan->key, 0, sizeof(plan->key));
+    CsrView A{d_arp, d_aci, nullptr, a_rows, a_cols, a_nnz};
+    CsrView B{d_brp, d_bci, nullptr, a_cols, b_cols, b_nnz};
+    if ((st = analyze(plan, A, B, false))) return bail(st);
+    a_nnz = plan->a_nnz;
+    b_nnz = plan->b_nnz;
     Misc* misc = plan->misc.as<Misc>();
-    const CsrView A{d_arp, d_aci, nullptr, a_rows, a_cols, a_nnz};
-    const CsrView B{d_brp, d_bci, nullptr, a_cols, b_cols, b_nnz};
-    const int grid = (int)std::min<int64_t>(((int64_t)a_rows + TYPED_WARPS - 1) / TYPED_WARPS,
-                                            148 * 16);
-    k_typed_numeric<Ops><<<grid, TYPED_WARPS * 32, 0, s>>>(A, B, d_av, d_bv, s_rp, s_ci, s_v,
-                                                          &misc->err);
+    int32_t *s_rp = nullptr, *s_ci = nullptr, *cnt, *o_rp;
+    Out* s_v = nullptr;
     const unsigned wgrid = (unsigned)(((int64_t)a_rows * 32 + 255) / 256);
-    k_nonzero_count<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_v, cnt);
-    note_launch(plan, 2);
+    const bool slots = typed_rows_sort(plan) && plan->products <= TYPED_SLOT_PRODUCTS;
+    if (slots) {
+        const size_t pn = (size_t)(plan->products > 0 ? plan->products : 1);
+        if ((e = sc.get(&s_ci, 4 * pn)) || (e = sc.get(&s_v, sizeof(Out) * pn)) ||
+            (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
+            return bail(fail(e, "typed scratch"));
+        if ((st = run_rows_typed(plan, sizeof(In) == 8, A, B, d_av, d_bv, s_ci, s_v)))
+            return bail(st);
+        cnt = plan->cnt.as<int32_t>();
+    } else {
+        // structure: exact analysis and count, then a fill on zero-valued operands
+        if ((st = count_exact(plan, A, B))) return bail(st);
+        plan->analysed = true;
+        const int64_t nnz = plan->c_nnz;
+        float* zeros;
+        float* s_fv;
+        const size_t zn = (size_t)std::max(a_nnz, b_nnz) + 1, cn = (size_t)(nnz > 0 ? nnz : 1);
+        if ((e = sc.get(&zeros, 4 * zn)) || (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) ||
+            (e = sc.get(&s_ci, 4 * cn)) || (e = sc.get(&s_fv, 4 * cn)) ||
+            (e = sc.get(&s_v, sizeof(Out) * cn)) || (e = sc.get(&cnt, 4 * (size_t)a_rows)) ||
+            (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
+            return bail(fail(e, "typed scratch"));
+        cudaMemsetAsync(zeros, 0, 4 * zn, s);
+        if ((st = rvsp_cuda_numeric(plan, d_arp, d_aci, zeros, d_brp, d_bci, zeros, s_rp, s_ci,
+                                    s_fv, 1, nullptr)))
+            return bail(st);
+        // typed values on that structure
+        const int grid = (int)std::min<int64_t>(((int64_t)a_rows + TYPED_WARPS - 1) / TYPED_WARPS,
+                                                148 * 16);
+        k_typed_numeric<Ops><<<grid, TYPED_WARPS * 32, 0, s>>>(A, B, d_av, d_bv, s_rp, s_ci, s_v,
+                                                              &misc->err);
+        k_nonzero_count<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_v, cnt);
+        note_launch(plan, 2);
+    }
     if ((st = scan_counts(plan, cnt, a_rows, nullptr, o_rp, &misc->scan_total))) return bail(st);
     int64_t total = 0;
     int32_t err = 0;
@@ -377,7 +440,11 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
         return bail(fail(e, "C alloc"));
     }
     cudaMemcpyAsync(rp, o_rp, 4 * ((size_t)a_rows + 1), cudaMemcpyDeviceToDevice, s);
-    k_nonzero_compact<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_ci, s_v, o_rp, ci, v);
+    if (slots)
+        k_slots_to_rows<Out><<<(unsigned)(((int64_t)a_rows * 16 + 255) / 256), 256, 0, s>>>(
+            a_rows, plan->slot_off.as<int64_t>(), s_ci, s_v, o_rp, ci, v);
+    else
+        k_nonzero_compact<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_ci, s_v, o_rp, ci, v);
     note_launch(plan, 1);
     sc.release();
     if ((e = cudaGetLastError()) != cudaSuccess) {

@@ -343,9 +343,9 @@ static void launch_sort(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
         const int32_t* rows = o.learned_bins ? plan->lbin_rows.as<int32_t>() + plan->loffs.off[b]
                                              : plan->bin_rows.as<int32_t>() + plan->offs.off[b];
         KTime kt(plan->stream, plan->capturing, KF_WARP_COUNT + MODE);
-        k_sort<E, NW, MODE><<<(n + S::ROWS - 1) / S::ROWS, S::ROWS * S::T, S::ROWS * S::BYTES,
-                              plan->stream>>>(
-            A, B, rows, n, o.cnt, o.c_rp, o.c_ci, o.c_v,
+        k_sort<E, NW, MODE, F32Values><<<(n + S::ROWS - 1) / S::ROWS, S::ROWS * S::T,
+                                         S::ROWS * S::BYTES, plan->stream>>>(
+            A, B, A.v, B.v, rows, n, o.cnt, o.c_rp, o.c_ci, o.c_v,
             o.maps ? plan->list_off.as<int32_t>() + plan->offs.off[b] : nullptr,
             o.maps ? plan->pm16.as<uint16_t>() + plan->pm16_base[b] : nullptr, o.err, o.ctl);
         note_launch(plan, 1);
@@ -431,6 +431,64 @@ static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             note_launch(plan, 1);
         }
     }
+}
+
+// One bin of a typed product, into the rows' slots (the rows of the tiny bin
+// are sorted too).
+template <int E, int NW, class V>
+static void launch_sort_typed(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B,
+                              const void* a_v, const void* b_v, int b, int32_t* slot_ci,
+                              void* slot_v) {
+    using S = SortShape<E, NW, V>;
+    const int n = plan->bin_count[b];
+    if (n == 0) return;
+    constexpr size_t smem = (size_t)S::ROWS * S::BYTES;
+    const auto kernel = k_sort<E, NW, FILL, V>;
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    RowCtl ctl = {};
+    ctl.slot_off = plan->slot_off.as<int64_t>();
+    kernel<<<(n + S::ROWS - 1) / S::ROWS, S::ROWS * S::T, smem, plan->stream>>>(
+        A, B, static_cast<const typename V::In*>(a_v), static_cast<const typename V::In*>(b_v),
+        plan->bin_rows.as<int32_t>() + plan->offs.off[b], n, plan->cnt.as<int32_t>(), nullptr,
+        slot_ci, static_cast<typename V::Out*>(slot_v), nullptr, nullptr,
+        &plan->misc.as<Misc>()->err, ctl);
+    note_launch(plan, 1);
+}
+
+template <class V>
+static void run_typed(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, const void* a_v,
+                      const void* b_v, int32_t* slot_ci, void* slot_v) {
+    launch_sort_typed<2, 1, V>(plan, A, B, a_v, b_v, BIN_TINY, slot_ci, slot_v);
+    launch_sort_typed<2, 1, V>(plan, A, B, a_v, b_v, BIN_SORT0, slot_ci, slot_v);
+    launch_sort_typed<4, 1, V>(plan, A, B, a_v, b_v, BIN_SORT0 + 1, slot_ci, slot_v);
+    launch_sort_typed<8, 1, V>(plan, A, B, a_v, b_v, BIN_SORT0 + 2, slot_ci, slot_v);
+    launch_sort_typed<16, 1, V>(plan, A, B, a_v, b_v, BIN_SORT0 + 3, slot_ci, slot_v);
+    launch_sort_typed<16, 2, V>(plan, A, B, a_v, b_v, BIN_SORT0 + 4, slot_ci, slot_v);
+    launch_sort_typed<16, 4, V>(plan, A, B, a_v, b_v, BIN_SORT0 + 5, slot_ci, slot_v);
+}
+
+bool typed_rows_sort(const rvsp_cuda_plan* plan) {
+    for (int b = BIN_WARP0; b < NUM_BINS; ++b)
+        if (plan->bin_count[b]) return false;
+    // (the tiny rows' words must fit too)
+    return sort_cols_fit(plan->b_cols, SORT_CAP_MIN);
+}
+
+int run_rows_typed(rvsp_cuda_plan* plan, bool f64, const CsrView& A, const CsrView& B,
+                   const void* a_v, const void* b_v, int32_t* slot_ci, void* slot_v) {
+    const int64_t M = plan->a_rows;
+    Misc* misc = plan->misc.as<Misc>();
+    cudaError_t e = plan->slot_off.ensure(((size_t)M + 1) * 8);
+    if (e == cudaSuccess) e = cudaMemsetAsync(plan->cnt.p, 0, (size_t)M * 4, plan->stream);
+    if (e != cudaSuccess) return fail(e, "typed slots");
+    int st = scan_counts(plan, plan->ub.as<int32_t>(), M, plan->slot_off.as<int64_t>(), nullptr,
+                         &misc->scan_total2);
+    if (st) return st;
+    KTime kt(plan->stream, plan->capturing, KF_WARP_FILL);
+    if (f64) run_typed<F64Values>(plan, A, B, a_v, b_v, slot_ci, slot_v);
+    else run_typed<I8Values>(plan, A, B, a_v, b_v, slot_ci, slot_v);
+    return RVSP_SUCCESS;
 }
 
 void run_rows(rvsp_cuda_plan* plan, int mode, const CsrView& A, const CsrView& B,

@@ -241,6 +241,12 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
                          int64_t* c_nnz_out);
 void run_rows(rvsp_cuda_plan* plan, int mode, const CsrView& A, const CsrView& B,
               const RowOut& o);
+// FP64 / INT8 products whose rows are all tiny or sorted rows (typed_rows_sort,
+// after the analysis): columns and nonzero sums of row r into slots of ub[r]
+// entries (plan->slot_off), their number to plan->cnt.
+bool typed_rows_sort(const rvsp_cuda_plan* plan);
+int run_rows_typed(rvsp_cuda_plan* plan, bool f64, const CsrView& A, const CsrView& B,
+                   const void* a_v, const void* b_v, int32_t* slot_ci, void* slot_v);
 int scan_counts(rvsp_cuda_plan* plan, const int32_t* in, int64_t n, int64_t* out64,
                 int32_t* out32, int64_t* total_dev);
 void note_launch(rvsp_cuda_plan* plan, int n);

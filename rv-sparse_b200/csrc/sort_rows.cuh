@@ -29,8 +29,48 @@ namespace rvsp {
 
 constexpr int SORT_CTA_ROWS = 4;  // one-warp rows per CTA
 
+// The value types of k_sort. arg() is what an A entry's products need of it,
+// one word beside the entry's position; entries whose sum is zero are kept
+// (KEEP_ZERO, the FP32 path) or dropped (the reference's FP64 and INT8
+// kernels, csr_scalar_f64.c:49-272 and csr_scalar_i8.c:24-196).
+struct F32Values {
+    using In = float;
+    using Out = float;
+    static constexpr bool KEEP_ZERO = true;
+    static __device__ __forceinline__ int arg(const float* a, int j) { return __float_as_int(a[j]); }
+    static __device__ __forceinline__ float mul(const float*, int arg, float b) {
+        return __fmul_rn(__int_as_float(arg), b);
+    }
+    static __device__ __forceinline__ float add(float x, float y) { return __fadd_rn(x, y); }
+    static __device__ __forceinline__ float read(const float* p) { return __ldg(p); }
+};
+struct F64Values {
+    using In = double;
+    using Out = double;
+    static constexpr bool KEEP_ZERO = false;
+    static __device__ __forceinline__ int arg(const double*, int j) { return j; }
+    static __device__ __forceinline__ double mul(const double* a, int j, double b) {
+        return __dmul_rn(__ldg(a + j), b);
+    }
+    static __device__ __forceinline__ double add(double x, double y) { return __dadd_rn(x, y); }
+    static __device__ __forceinline__ double read(const double* p) { return __ldg(p); }
+};
+struct I8Values {
+    using In = int8_t;
+    using Out = int32_t;
+    static constexpr bool KEEP_ZERO = false;
+    static __device__ __forceinline__ int arg(const int8_t* a, int j) { return a[j]; }
+    static __device__ __forceinline__ int32_t mul(const int8_t*, int a, int8_t b) {
+        return (int32_t)((uint32_t)a * (uint32_t)(int32_t)b);
+    }
+    static __device__ __forceinline__ int32_t add(int32_t x, int32_t y) {
+        return (int32_t)((uint32_t)x + (uint32_t)y);
+    }
+    static __device__ __forceinline__ int8_t read(const int8_t* p) { return *p; }
+};
+
 // Threads of one row: NW warps, CAP = 32 NW E words.
-template <int E, int NW>
+template <int E, int NW, class V = F32Values>
 struct SortShape {
     static constexpr int T = 32 * NW;
     static constexpr int CAP = T * E;
@@ -43,9 +83,10 @@ struct SortShape {
     // position - first index, A value} while the products are gathered,
     // overlaid afterwards by the row's columns and values in C's order; the
     // products' values.
-    static constexpr int EXTRA = NW == 1 ? 0 : WORDS + T + 2 * NW + 2;
-    static constexpr int BYTES = 4 * (WORDS + EXTRA + 2 * PAD + CAP);
-    static_assert((WORDS + EXTRA) % 2 == 0 && BYTES % 8 == 0, "");
+    static constexpr int OW = sizeof(typename V::Out) / 4;  // words of a value
+    static constexpr int EXTRA = NW == 1 ? 0 : WORDS + OW * T + 2 * NW + 2;
+    static constexpr int BYTES = 4 * (WORDS + EXTRA + (1 + OW) * PAD + OW * CAP);
+    static_assert((WORDS + EXTRA) % 2 == 0 && PAD % 2 == 0 && BYTES % 8 == 0, "");
 };
 
 // Padded index: one word in 32 is left out, so lanes a power of two words
@@ -131,15 +172,17 @@ __device__ __forceinline__ void sort_words(float (&f)[E], int t, float* xbuf) {
 // with the count to cnt, or -1 when it passes the slot) and, with pm, every
 // product's position in the row. Words must stay below the bits of infinity
 // (sort_cols_fit).
-template <int E, int NW, int MODE>
-__global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
-    k_sort(CsrView A, CsrView B, const int32_t* __restrict__ rows, int nrows,
+template <int E, int NW, int MODE, class V>
+__global__ void __launch_bounds__(SortShape<E, NW, V>::T * SortShape<E, NW, V>::ROWS)
+    k_sort(CsrView A, CsrView B, const typename V::In* __restrict__ a_v,
+           const typename V::In* __restrict__ b_v, const int32_t* __restrict__ rows, int nrows,
            int32_t* __restrict__ cnt, const int32_t* __restrict__ c_rp,
-           int32_t* __restrict__ c_ci, float* __restrict__ c_v,
+           int32_t* __restrict__ c_ci, typename V::Out* __restrict__ c_v,
            const int32_t* __restrict__ list_off, uint16_t* __restrict__ pm,
            int32_t* __restrict__ err, RowCtl ctl) {
     static_assert(MODE == COUNT || MODE == FILL, "");
-    using S = SortShape<E, NW>;
+    using S = SortShape<E, NW, V>;
+    using Out = typename V::Out;
     constexpr int CAP = S::CAP, T = S::T, WORDS = S::WORDS;
     constexpr int IB = __builtin_ctz(CAP);
     constexpr uint32_t SAME = MODE == FILL ? CAP : 1;  // words of one column differ by less
@@ -154,12 +197,12 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
     if (ctl.only && !ctl.only[row]) return;
     uint32_t* heads = reinterpret_cast<uint32_t*>(smem + slot * S::BYTES);
     int* pre = reinterpret_cast<int*>(heads + WORDS);       // NW > 1: starts before each word
-    float* tails = reinterpret_cast<float*>(pre + WORDS);   // NW > 1: each thread's open run
+    Out* tails = reinterpret_cast<Out*>(pre + WORDS);       // NW > 1: each thread's open run
     int* red = reinterpret_cast<int*>(tails + T);           // NW > 1: per-warp words, n, total
     int2* ent = reinterpret_cast<int2*>(heads + WORDS + S::EXTRA);
     int32_t* scol = reinterpret_cast<int32_t*>(ent);
-    float* sval = reinterpret_cast<float*>(scol + S::PAD);
-    float* vals = sval + S::PAD;
+    Out* sval = reinterpret_cast<Out*>(scol + S::PAD);
+    Out* vals = sval + S::PAD;
     const auto sync = [] {
         if constexpr (NW == 1) __syncwarp();
         else __syncthreads();
@@ -173,20 +216,18 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
         row_range(A, row, &a0, &a1, err);
         for (int base = a0; base < a1; base += 32) {
             const int j = base + lane;
-            int bs = 0, bl = 0;
-            float av = 0.0f;
+            int bs = 0, bl = 0, arg = 0;
             if (j < a1) {
                 int be;
                 row_range(B, A.ci[j], &bs, &be, err);
                 bl = min(be - bs, CAP + 1);
-                if (MODE == FILL) av = A.v[j];
+                if (MODE == FILL) arg = V::arg(a_v, j);
             }
             const int incl = warp_incl_scan(bl);
             const int start = n + incl - bl;
             const unsigned some = __ballot_sync(FULL, bl > 0);
             if (bl > 0 && start < CAP) {
-                ent[entries + __popc(some & ((1u << lane) - 1))] =
-                    make_int2(bs - start, __float_as_int(av));
+                ent[entries + __popc(some & ((1u << lane) - 1))] = make_int2(bs - start, arg);
                 atomicOr(&heads[start >> 5], 1u << (start & 31));
             }
             entries += __popc(some);
@@ -227,7 +268,7 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
                 const int2 e = ent[before + __popc(h & upto)];
                 const int q = e.x + p;
                 uint32_t col = (uint32_t)__ldg(B.ci + q);
-                if (MODE == FILL) vals[p] = __fmul_rn(__int_as_float(e.y), __ldg(B.v + q));
+                if (MODE == FILL) vals[p] = V::mul(a_v, e.y, V::read(b_v + q));
                 if (col >= (uint32_t)B.cols) {
                     bad = true;
                     col = 0;
@@ -239,7 +280,7 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
         if (bad) atomicOr(err, ERR_STRUCTURE);
     }
     sync();  // every thread has read the entries
-    sort_words<E, NW>(f, t, sval);
+    sort_words<E, NW>(f, t, reinterpret_cast<float*>(scol));
     // heads: words whose column differs from the one before (bit j of mask)
     const int mine = min(max(n - t * E, 0), E);  // words this thread holds
     float last = __shfl_up_sync(FULL, f[E - 1], 1);
@@ -276,7 +317,7 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
         if (ctl.slot_off) {
             o = ctl.slot_off[row];
             const bool over = total > ctl.slot_off[row + 1] - o;
-            if (t == 0) cnt[row] = over ? -1 : total;
+            if (V::KEEP_ZERO && t == 0) cnt[row] = over ? -1 : total;
             if (over) return;
         } else {
             o = c_rp[row];
@@ -287,7 +328,7 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
         }
         // each run summed in order; a thread stores the runs that begin and
         // end in its words
-        float v[E];
+        Out v[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) v[j] = vals[__float_as_uint(f[j]) & (CAP - 1)];
         const bool lead = mine > 0 && !(mask & 1u);  // its first words belong to a run before
@@ -298,12 +339,12 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
             __syncthreads();
             if (lane == 31 && wi + 1 < NW) follow = red[wi + 1] != 0;
         }
-        float acc = 0.0f;
+        Out acc = Out(0);
         int d = base - 1;
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             const bool head = mask >> j & 1u;
-            acc = __fadd_rn(head ? 0.0f : acc, v[j]);
+            acc = V::add(head ? Out(0) : acc, v[j]);
             d += head;
             const bool end = j == E - 1 ? !follow : (mask >> (j + 1) & 1u) || j + 1 == mine;
             if (j < mine && end && d >= base) {
@@ -332,7 +373,7 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
             rounds = any ? 1 + __syncthreads_count(through) : 0;
         }
         for (int it = 0; it < rounds; ++it) {
-            float in = __shfl_up_sync(FULL, acc, 1);
+            Out in = __shfl_up_sync(FULL, acc, 1);
             if constexpr (NW > 1) {
                 if (lane == 31) tails[wi] = acc;
                 __syncthreads();
@@ -340,12 +381,12 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
                 __syncthreads();
             }
             if (lead) {
-                float a = in;
+                Out a = in;
                 const int until = mask ? __ffs(mask) - 1 : mine;
                 int col = 0;
 #pragma unroll
                 for (int j = 0; j < E; ++j)
-                    if (j < until) a = __fadd_rn(a, v[j]);
+                    if (j < until) a = V::add(a, v[j]);
                 col = (int32_t)(__float_as_uint(f[0]) >> IB);
                 if (through) acc = a;
                 if (!(through && follow)) {
@@ -355,9 +396,26 @@ __global__ void __launch_bounds__(SortShape<E, NW>::T * SortShape<E, NW>::ROWS)
             }
         }
         sync();
-        for (int x = t; x < total; x += T) {
-            c_ci[o + x] = scol[pad32(x)];
-            c_v[o + x] = sval[pad32(x)];
+        if constexpr (V::KEEP_ZERO) {
+            for (int x = t; x < total; x += T) {
+                c_ci[o + x] = scol[pad32(x)];
+                c_v[o + x] = sval[pad32(x)];
+            }
+        } else if (NW == 1 || wi == 0) {
+            // without the zero sums, by one warp; the count is what is left
+            int kept = 0;
+            for (int x0 = 0; x0 < total; x0 += 32) {
+                const int x = x0 + lane;
+                const Out s = x < total ? sval[pad32(x)] : Out(0);
+                const unsigned m = __ballot_sync(FULL, s != Out(0));
+                if (s != Out(0)) {
+                    const int64_t to = o + kept + __popc(m & ((1u << lane) - 1));
+                    c_ci[to] = scol[pad32(x)];
+                    c_v[to] = s;
+                }
+                kept += __popc(m);
+            }
+            if (lane == 0) cnt[row] = kept;
         }
     }
 }

@@ -11,6 +11,7 @@ import oracle
 import rvsp_b200 as rv
 from gpu_util import DevCSR, bits, dev, oneshot
 from rvsp_b200 import gen
+from test_legacy_dtypes_gpu import assert_typed_same, cuda_typed, typed_pair
 from test_parity_gpu import assert_same, oracle_full
 
 pytestmark = pytest.mark.gpu
@@ -108,3 +109,22 @@ def test_signed_zeros_and_non_finite_values(gpu_lib):
     nan = np.isnan(want[2])
     assert np.array_equal(np.isnan(got[2]), nan)
     assert np.array_equal(bits(got[2])[~nan], bits(want[2])[~nan])
+
+
+@pytest.mark.parametrize("dtype", ["f64", "i8"])
+@pytest.mark.parametrize("cols,repeats,clustered", [(5000, 1, False), (400, 4, False),
+                                                    (1044480, 1, False), (3000, 4, True)])
+def test_typed_rows_at_the_bins_edges(gpu_lib, dtype, cols, repeats, clustered):
+    """FP64 and INT8 through the sorting pass (rows of up to 2048 products; the
+    2049-product rows dropped), zero sums left out."""
+    A, B = _edge_product(cols, repeats, cols % 97, clustered)
+    keep = np.flatnonzero(gen.row_products(A, B) <= 2048)
+    rp = A.row_ptr
+    A = gen.CSR(keep.size, A.cols,
+                np.concatenate([[0], np.cumsum(np.diff(rp)[keep])]).astype(np.int32),
+                np.concatenate([A.col_idx[rp[r]:rp[r + 1]] for r in keep]),
+                np.concatenate([A.values[rp[r]:rp[r + 1]] for r in keep]))
+    A, B = typed_pair(A, B, dtype, seed=3)
+    want = oracle.spgemm_typed(A, B, dtype)
+    for device in (True, False):
+        assert_typed_same(cuda_typed(A, B, dtype, device), want, dtype, f"{cols} {device}")
