@@ -356,7 +356,7 @@ template <int MODE>
 static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B,
                         const RowOut& o) {
     const int32_t* rows = o.learned_bins ? plan->lbin_rows.as<int32_t>() : plan->bin_rows.as<int32_t>();
-    for (int b = BIN_TINY; b < NUM_BINS; ++b) {
+    for (int b = o.bin_first; b < o.bin_end; ++b) {
         const int n = o.learned_bins ? plan->lcount[b] : plan->bin_count[b];
         if (n == 0) continue;
         // heavy rows in the learned sweep: into their predicted slots when
@@ -587,7 +587,7 @@ int stage_operands(rvsp_cuda_plan* plan, const int32_t* a_rp, const int32_t* a_c
 // Analysis + binning. Leaves per-row op counts, bins and heavy items in the
 // plan; one device->host read of the bin histogram.
 int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
-            int (*pre_sync)(rvsp_cuda_plan*)) {
+            int (*pre_sync)(rvsp_cuda_plan*), bool slots) {
     const int64_t M = plan->a_rows;
     cudaError_t e;
 #define ENS(buf, bytes)                                        \
@@ -605,10 +605,12 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     ENS(plan->tile_hist, NUM_BINS * tiles * 4);
     ENS(plan->tile_off, (NUM_BINS * tiles + 1) * 4);
     if (features) ENS(plan->feat, M * 16);
+    if (slots) ENS(plan->slot_len, M * 4);
     Misc* misc = plan->misc.as<Misc>();
     if ((e = cudaMemsetAsync(misc, 0, sizeof(Misc), plan->stream)) != cudaSuccess)
         return fail(e, "memset");
-    AnalyzeOut out{plan->ops.as<int64_t>(), plan->ub.as<int32_t>(), plan->bin.as<uint8_t>(),
+    AnalyzeOut out{plan->ops.as<int64_t>(), plan->ub.as<int32_t>(),
+                   slots ? plan->slot_len.as<int32_t>() : nullptr, plan->bin.as<uint8_t>(),
                    plan->chunk_lo.as<int32_t>(), plan->nchunks.as<int32_t>(),
                    features ? plan->feat.as<float4>() : nullptr, misc->hist,
                    plan->tile_hist.as<int32_t>(), misc->totals, misc->bin_prod, &misc->err,
@@ -909,16 +911,25 @@ int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     return st ? st : count_read(plan);
 }
 
-// The count kernels and scans, enqueued only: C's row pointer lands in
-// plan->c_rp, the heavy chunks' offsets in plan->item_scan, nnz(C) in
+// The count kernels and scans, enqueued only (with slot_ci, tiny and sorted
+// rows are filled into their slots instead, plan->slot_off, which counts
+// them): C's row pointer lands in plan->c_rp, the heavy chunks' offsets in plan->item_scan, nnz(C) in
 // Misc::scan_total.
-int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
+int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* slot_ci,
+                 float* slot_v) {
     cudaError_t e;
     const int64_t M = plan->a_rows;
     if ((e = cudaMemsetAsync(plan->cnt.p, 0, M * 4, plan->stream)) != cudaSuccess)
         return fail(e, "memset");
     Misc* misc = plan->misc.as<Misc>();
     RowOut o{plan->cnt.as<int32_t>(), nullptr, nullptr, nullptr, &misc->err, false};
+    if (slot_ci) {
+        RowOut f{plan->cnt.as<int32_t>(), nullptr, slot_ci, slot_v, &misc->err, false};
+        f.ctl.slot_off = plan->slot_off.as<int64_t>();
+        f.bin_end = BIN_WARP0;
+        run_rows(plan, FILL, A, B, f);
+        o.bin_first = BIN_WARP0;
+    }
     run_rows(plan, COUNT, A, B, o);
     int st = scan_counts(plan, plan->cnt.as<int32_t>(), M, nullptr, plan->c_rp.as<int32_t>(),
                          &misc->scan_total);
@@ -1123,7 +1134,7 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t p) {
                       &p->ops, &p->ub, &p->bin, &p->chunk_lo, &p->nchunks, &p->feat,
                       &p->cnt, &p->c_rp, &p->bin_rows, &p->items, &p->item_cnt,
                       &p->item_scan, &p->scan_tmp, &p->misc, &p->s_cci, &p->s_cv,
-                      &p->pred_cap, &p->slot_off, &p->tmp_ci, &p->tmp_v, &p->row_flag,
+                      &p->pred_cap, &p->slot_off, &p->slot_len, &p->tmp_ci, &p->tmp_v, &p->row_flag,
                       &p->tile_hist, &p->tile_off, &p->pm8, &p->pm16, &p->list_ops,
                       &p->list_off, &p->lbin, &p->lcap, &p->ltile_hist, &p->ltile_off,
                       &p->lbin_rows, &p->need, &p->pflag, &p->hmask, &p->hovf,
@@ -1394,6 +1405,50 @@ namespace rvsp {
 // count and the fill.
 constexpr int64_t ONESHOT_FUSED_PRODUCTS = int64_t(1) << 25;
 
+// Tiny and sorted rows of a one-shot product are filled before they are
+// counted, into slots of their upper bound (8 bytes a product), and copied
+// into C once the row pointer is known: the copy moves 16 bytes an entry,
+// where counting first means sorting every product twice (tall-skinny 2M x
+// 100k: counts 2.1 ms, copy 1.1 ms, call 8.0 -> 7.0 ms). Below
+// SLOT_MIN_PRODUCTS the scan of the slots and the copy cost what the counts do
+// (4096^2 x 16, 2^20 products: 113 us against 105); above SLOT_MAX_PRODUCTS (4
+// GiB of slots) the rows are counted.
+constexpr int64_t SLOT_MIN_PRODUCTS = int64_t(1) << 22;
+constexpr int64_t SLOT_MAX_PRODUCTS = int64_t(1) << 29;
+
+// Rows from their slots into C, 16 lanes a row; rows without a slot are left.
+static __global__ void __launch_bounds__(256)
+    k_slots_to_c(int32_t rows, const int64_t* __restrict__ slot_off,
+                 const int32_t* __restrict__ slot_ci, const float* __restrict__ slot_v,
+                 const int32_t* __restrict__ rp, int32_t* __restrict__ ci, float* __restrict__ v) {
+    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    const int lane = threadIdx.x & 15;
+    if (row >= rows) return;
+    const int64_t src = slot_off[row];
+    if (slot_off[row + 1] == src) return;
+    const int dst = rp[row], n = rp[row + 1] - dst;
+    for (int x0 = lane; x0 < n; x0 += 64) {
+        int32_t c[4];
+        float y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int x = x0 + 16 * u;
+            if (x < n) {
+                c[u] = slot_ci[src + x];
+                y[u] = slot_v[src + x];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int x = x0 + 16 * u;
+            if (x < n) {
+                ci[dst + x] = c[u];
+                v[dst + x] = y[u];
+            }
+        }
+    }
+}
+
 int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, int32_t b_cols,
                          const int32_t* a_rp, const int32_t* a_ci, const float* a_v,
                          const int32_t* b_rp, const int32_t* b_ci, const float* b_v,
@@ -1414,19 +1469,50 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     CsrView A, B;
     int st = stage_operands(plan, a_rp, a_ci, a_v, b_rp, b_ci, b_v, false, &A, &B);
     if (st) return st;
-    if ((st = analyze(plan, A, B, plan->features))) return st;
+    if ((st = analyze(plan, A, B, plan->features, nullptr, true))) return st;
     const int64_t M = a_rows;
-    const bool fused = plan->products <= ONESHOT_FUSED_PRODUCTS;
-    int64_t cap;
-    if (fused) {
-        if ((st = count_launch(plan, A, B))) return st;
-        cap = plan->products;
-    } else {
-        if ((st = count_exact(plan, A, B))) return st;
-        cap = plan->c_nnz;
+    Misc* misc = plan->misc.as<Misc>();
+    int64_t slot_products = 0;
+    for (int b = BIN_TINY; b < BIN_WARP0; ++b) slot_products += plan->host_misc.bin_prod[b];
+    int32_t *rp = nullptr, *ci = nullptr, *slot_ci = nullptr;
+    float *v = nullptr, *slot_v = nullptr;
+    const auto release_slots = [&] {
+        if (slot_ci) cudaFreeAsync(slot_ci, plan->stream);
+        if (slot_v) cudaFreeAsync(slot_v, plan->stream);
+        slot_ci = nullptr;
+        slot_v = nullptr;
+    };
+    const auto release = [&] {
+        release_slots();
+        if (rp) cudaFreeAsync(rp, plan->stream);
+        if (ci) cudaFreeAsync(ci, plan->stream);
+        if (v) cudaFreeAsync(v, plan->stream);
+    };
+    bool slots = slot_products >= SLOT_MIN_PRODUCTS && slot_products <= SLOT_MAX_PRODUCTS;
+    if (slots && (plan->slot_off.ensure(((size_t)M + 1) * 8) != cudaSuccess ||
+                  cudaMallocAsync((void**)&slot_ci, 4 * (size_t)slot_products, plan->stream) !=
+                      cudaSuccess ||
+                  cudaMallocAsync((void**)&slot_v, 4 * (size_t)slot_products, plan->stream) !=
+                      cudaSuccess)) {
+        cudaGetLastError();
+        release_slots();  // without the memory the rows are counted
+        slots = false;
     }
-    int32_t *rp = nullptr, *ci = nullptr;
-    float* v = nullptr;
+    if (slots) {
+        if ((st = scan_counts(plan, plan->slot_len.as<int32_t>(), M, plan->slot_off.as<int64_t>(),
+                              nullptr, &misc->scan_total2))) {
+            release();
+            return st;
+        }
+    }
+    const bool fused = plan->products <= ONESHOT_FUSED_PRODUCTS;
+    int64_t cap = plan->products;
+    if ((st = count_launch(plan, A, B, slots ? slot_ci : nullptr, slot_v)) ||
+        (!fused && (st = count_read(plan)))) {
+        release();
+        return st;
+    }
+    if (!fused) cap = plan->c_nnz;
     const size_t alloc = cap > 0 ? (size_t)cap : 1;
     cudaError_t e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&ci, alloc * 4, plan->stream);
@@ -1434,22 +1520,25 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(rp, plan->c_rp.p, ((size_t)M + 1) * 4, cudaMemcpyDeviceToDevice,
                             plan->stream);
-    Misc* misc = plan->misc.as<Misc>();
     if (e == cudaSuccess) {
         RowOut o{nullptr, plan->c_rp.as<int32_t>(), ci, v, &misc->err, false};
+        if (slots) {
+            o.bin_first = BIN_WARP0;
+            KTime kt(plan->stream, plan->capturing, KF_COMPACT);
+            k_slots_to_c<<<(unsigned)((M * 16 + 255) / 256), 256, 0, plan->stream>>>(
+                a_rows, plan->slot_off.as<int64_t>(), slot_ci, slot_v, plan->c_rp.as<int32_t>(), ci,
+                v);
+            note_launch(plan, 1);
+        }
         run_rows(plan, FILL, A, B, o);
         e = cudaGetLastError();
     }
+    release_slots();
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&plan->host_misc, misc, sizeof(Misc), cudaMemcpyDeviceToHost,
                             plan->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
     trace_point("one-shot exact (synced)");
-    const auto release = [&] {
-        if (rp) cudaFreeAsync(rp, plan->stream);
-        if (ci) cudaFreeAsync(ci, plan->stream);
-        if (v) cudaFreeAsync(v, plan->stream);
-    };
     if (e != cudaSuccess) {
         release();
         return fail(e, "one-shot product");

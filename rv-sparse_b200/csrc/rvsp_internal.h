@@ -69,6 +69,7 @@ struct RowOut {
     bool maps;           // FILL: record position maps; REUSE: replay them
     RowCtl ctl = {nullptr, nullptr, 0, nullptr, nullptr, nullptr, 0, 0};
     bool learned_bins = false;  // iterate the predicted-capacity bins instead
+    int bin_first = BIN_TINY, bin_end = NUM_BINS;  // the bins to run
     // REUSE, every row a tiny row: the map-replay kernel also writes the
     // caller's row pointer (the copy of the analysed one is skipped)
     int32_t* rp_out = nullptr;
@@ -207,7 +208,7 @@ struct rvsp_cuda_plan {
     rvsp::BinOffsets loffs = {};
     int64_t slot_total = 0;
     int64_t lstats[10] = {};  // see rvsp_cuda_plan_learned_stats
-    rvsp::DevBuf pred_cap, slot_off, tmp_ci, tmp_v, row_flag;
+    rvsp::DevBuf pred_cap, slot_off, slot_len, tmp_ci, tmp_v, row_flag;
     // heavy rows of the learned sweep: rows kept heavy (hmask), rows whose
     // chunks found no room (hovf), where each chunk went in the slot buffer
     // (item_off), the size of the shared overflow pool after the slots
@@ -227,9 +228,10 @@ int stage_operands(rvsp_cuda_plan* plan, const int32_t* a_rp, const int32_t* a_c
                    const float* a_v, const int32_t* b_rp, const int32_t* b_ci, const float* b_v,
                    bool cache_index, CsrView* A, CsrView* B);
 int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
-            int (*pre_sync)(rvsp_cuda_plan*) = nullptr);
+            int (*pre_sync)(rvsp_cuda_plan*) = nullptr, bool slots = false);
 int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
-int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
+int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B,
+                 int32_t* slot_ci = nullptr, float* slot_v = nullptr);
 int count_read(rvsp_cuda_plan* plan);
 // One-shot exact product of device-resident operands into new device arrays
 // (rvsp_cuda_spgemm_f32's exact path when every operand array is on the

@@ -139,6 +139,7 @@ __device__ __forceinline__ void ordered_add(float* vals, int slot, bool active, 
 struct AnalyzeOut {
     int64_t* ops;        // [rows] intermediate products per row
     int32_t* ub;         // [rows] min(ops, b_cols)
+    int32_t* slot_len;   // [rows] ub of tiny and sorted rows, 0 for the others (optional)
     uint8_t* bin;        // [rows]
     int32_t* chunk_lo;   // [rows] first heavy column chunk
     int32_t* nchunks;    // [rows] heavy column chunks (0 for other bins)
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(AN_TILE)
     if (live) {
         out.ops[row] = ops;
         out.ub[row] = ub;
+        if (out.slot_len) out.slot_len[row] = b < BIN_WARP0 ? ub : 0;
         out.bin[row] = (uint8_t)b;
         int clo = 0;
         if (b == BIN_HEAVY) {
