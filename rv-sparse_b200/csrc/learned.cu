@@ -429,8 +429,7 @@ static int learned_pre_sync(rvsp_cuda_plan* plan) {
             plan->pred_cap.as<int32_t>(), lo, plan->params);
     }
     note_launch(plan, 2);
-    return scan_counts(plan, plan->ltile_hist.as<int32_t>(), NUM_BINS * tiles, nullptr,
-                       plan->ltile_off.as<int32_t>(), &misc->ltile_total);
+    return RVSP_SUCCESS;
 }
 
 // Learned analysis, one sweep over the predicted-capacity bins, exact counts
@@ -479,8 +478,10 @@ int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused) {
         if ((e = plan->tmp_v.ensure((size_t)tmp_total * 4)) != cudaSuccess)
             return fail(e, "slots");
     }
-    launch_bin_scatter(plan, plan->lbin.as<uint8_t>(), plan->ltile_off.as<int32_t>(),
-                       plan->lbin_rows.as<int32_t>());
+    if ((st = launch_bin_scatter(plan, plan->lbin.as<uint8_t>(), misc->lhist,
+                                 plan->ltile_hist.as<int32_t>(), plan->ltile_off.as<int32_t>(),
+                                 plan->lbin_rows.as<int32_t>())))
+        return st;
     if (fused && (st = scan_counts(plan, plan->lcap.as<int32_t>(), M, plan->slot_off.as<int64_t>(),
                                    nullptr, &misc->scan_total2)))
         return st;
@@ -536,10 +537,7 @@ int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused) {
                           plan->item_scan.as<int64_t>(), nullptr, &misc->tile_total)))
         return st;
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "learned launch");
-    if ((e = cudaMemcpyAsync(&plan->host_misc, misc, sizeof(Misc), cudaMemcpyDeviceToHost,
-                             plan->stream)) != cudaSuccess)
-        return fail(e, "learned read");
-    if ((e = cudaStreamSynchronize(plan->stream)) != cudaSuccess) return fail(e, "learned sweep");
+    if ((e = read_misc(plan)) != cudaSuccess) return fail(e, "learned sweep");
     trace_point("learned: sweep (synced)");
     if (plan->host_misc.err) {
         g_err = "operand structure out of range (row_ptr or col_idx)";

@@ -479,8 +479,7 @@ int run_rows_typed(rvsp_cuda_plan* plan, bool f64, const CsrView& A, const CsrVi
                    const void* a_v, const void* b_v, int32_t* slot_ci, void* slot_v) {
     const int64_t M = plan->a_rows;
     Misc* misc = plan->misc.as<Misc>();
-    cudaError_t e = plan->slot_off.ensure(((size_t)M + 1) * 8);
-    if (e == cudaSuccess) e = cudaMemsetAsync(plan->cnt.p, 0, (size_t)M * 4, plan->stream);
+    const cudaError_t e = plan->slot_off.ensure(((size_t)M + 1) * 8);
     if (e != cudaSuccess) return fail(e, "typed slots");
     int st = scan_counts(plan, plan->ub.as<int32_t>(), M, plan->slot_off.as<int64_t>(), nullptr,
                          &misc->scan_total2);
@@ -610,7 +609,8 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     if ((e = cudaMemsetAsync(misc, 0, sizeof(Misc), plan->stream)) != cudaSuccess)
         return fail(e, "memset");
     AnalyzeOut out{plan->ops.as<int64_t>(), plan->ub.as<int32_t>(),
-                   slots ? plan->slot_len.as<int32_t>() : nullptr, plan->bin.as<uint8_t>(),
+                   slots ? plan->slot_len.as<int32_t>() : nullptr, plan->cnt.as<int32_t>(),
+                   plan->bin.as<uint8_t>(),
                    plan->chunk_lo.as<int32_t>(), plan->nchunks.as<int32_t>(),
                    features ? plan->feat.as<float4>() : nullptr, misc->hist,
                    plan->tile_hist.as<int32_t>(), misc->totals, misc->bin_prod, &misc->err,
@@ -620,14 +620,9 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
         k_analyze<<<(unsigned)tiles, AN_TILE, 0, plan->stream>>>(A, B, out, plan->params);
     }
     note_launch(plan, 1);
-    int st = scan_counts(plan, plan->tile_hist.as<int32_t>(), NUM_BINS * tiles, nullptr,
-                         plan->tile_off.as<int32_t>(), &misc->tile_total);
-    if (st) return st;
+    int st = RVSP_SUCCESS;
     if (pre_sync && (st = pre_sync(plan))) return st;
-    if ((e = cudaMemcpyAsync(&plan->host_misc, misc, sizeof(Misc), cudaMemcpyDeviceToHost,
-                             plan->stream)) != cudaSuccess)
-        return fail(e, "histogram read");
-    if ((e = cudaStreamSynchronize(plan->stream)) != cudaSuccess) return fail(e, "analysis");
+    if ((e = read_misc(plan)) != cudaSuccess) return fail(e, "analysis");
     trace_point("analysis (synced)");
     if (plan->host_misc.err) {
         g_err = "operand structure out of range (row_ptr or col_idx)";
@@ -654,8 +649,10 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     ENS(plan->item_cnt, (size_t)plan->n_items * 4);
     ENS(plan->item_scan, ((size_t)plan->n_items + 1) * 8);
 #undef ENS
-    launch_bin_scatter(plan, plan->bin.as<uint8_t>(), plan->tile_off.as<int32_t>(),
-                       plan->bin_rows.as<int32_t>());
+    if ((st = launch_bin_scatter(plan, plan->bin.as<uint8_t>(), misc->hist,
+                                 plan->tile_hist.as<int32_t>(), plan->tile_off.as<int32_t>(),
+                                 plan->bin_rows.as<int32_t>())))
+        return st;
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "analysis launch");
     if (plan->n_items > 0) {
         if ((st = build_heavy_lists(plan, A, B))) return st;
@@ -895,14 +892,34 @@ int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     return RVSP_SUCCESS;
 }
 
-// Stable partition of the plan's rows by bin (k_bin_scatter).
-void launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* tile_off,
-                        int32_t* bin_rows) {
-    const int64_t M = plan->a_rows;
+int launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* hist,
+                       const int32_t* tile_hist, int32_t* tile_off, int32_t* bin_rows) {
+    const int64_t M = plan->a_rows, tiles = (M + AN_TILE - 1) / AN_TILE;
+    const bool scan = tiles > SCATTER_SUM_TILES;
+    int st;
+    if (scan && (st = scan_counts(plan, tile_hist, NUM_BINS * tiles, nullptr, tile_off,
+                                  &plan->misc.as<Misc>()->tile_total)))
+        return st;
     KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
-    k_bin_scatter<<<(unsigned)((M + AN_TILE - 1) / AN_TILE), AN_TILE, 0, plan->stream>>>(
-        (int32_t)M, bin, tile_off, bin_rows);
+    k_bin_scatter<<<(unsigned)tiles, AN_TILE, 0, plan->stream>>>(
+        (int32_t)M, bin, scan ? tile_off : nullptr, hist, tile_hist, bin_rows);
     note_launch(plan, 1);
+    return RVSP_SUCCESS;
+}
+
+// (into pinned memory: a copy into pageable memory goes through the driver's
+// bounce buffer on this thread)
+cudaError_t read_misc(rvsp_cuda_plan* plan) {
+    if (!plan->misc_pin && cudaMallocHost((void**)&plan->misc_pin, sizeof(Misc)) != cudaSuccess) {
+        cudaGetLastError();
+        plan->misc_pin = nullptr;
+    }
+    Misc* to = plan->misc_pin ? plan->misc_pin : &plan->host_misc;
+    cudaError_t e = cudaMemcpyAsync(to, plan->misc.p, sizeof(Misc), cudaMemcpyDeviceToHost,
+                                    plan->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+    if (e == cudaSuccess && to != &plan->host_misc) plan->host_misc = *to;
+    return e;
 }
 
 // Exact count + scan: C's row pointer in plan->c_rp, nnz in plan->c_nnz.
@@ -913,15 +930,13 @@ int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
 
 // The count kernels and scans, enqueued only (with slot_ci, tiny and sorted
 // rows are filled into their slots instead, plan->slot_off, which counts
-// them): C's row pointer lands in plan->c_rp, the heavy chunks' offsets in plan->item_scan, nnz(C) in
+// them): C's row pointer lands in c_rp, or plan->c_rp when it is null, the heavy chunks' offsets in plan->item_scan, nnz(C) in
 // Misc::scan_total.
-int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* slot_ci,
-                 float* slot_v) {
+int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* c_rp,
+                 int32_t* slot_ci, float* slot_v) {
     cudaError_t e;
     const int64_t M = plan->a_rows;
-    if ((e = cudaMemsetAsync(plan->cnt.p, 0, M * 4, plan->stream)) != cudaSuccess)
-        return fail(e, "memset");
-    Misc* misc = plan->misc.as<Misc>();
+    Misc* misc = plan->misc.as<Misc>();  // (the analysis zeroed cnt)
     RowOut o{plan->cnt.as<int32_t>(), nullptr, nullptr, nullptr, &misc->err, false};
     if (slot_ci) {
         RowOut f{plan->cnt.as<int32_t>(), nullptr, slot_ci, slot_v, &misc->err, false};
@@ -931,8 +946,8 @@ int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32
         o.bin_first = BIN_WARP0;
     }
     run_rows(plan, COUNT, A, B, o);
-    int st = scan_counts(plan, plan->cnt.as<int32_t>(), M, nullptr, plan->c_rp.as<int32_t>(),
-                         &misc->scan_total);
+    int st = scan_counts(plan, plan->cnt.as<int32_t>(), M, nullptr,
+                         c_rp ? c_rp : plan->c_rp.as<int32_t>(), &misc->scan_total);
     if (st) return st;
     if (plan->n_items > 0) {
         st = scan_counts(plan, plan->item_cnt.as<int32_t>(), plan->n_items,
@@ -946,12 +961,8 @@ int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32
 
 // Waits for count_launch's work and takes nnz(C) into plan->c_nnz.
 int count_read(rvsp_cuda_plan* plan) {
-    cudaError_t e;
-    Misc* misc = plan->misc.as<Misc>();
-    if ((e = cudaMemcpyAsync(&plan->host_misc, misc, sizeof(Misc), cudaMemcpyDeviceToHost,
-                             plan->stream)) != cudaSuccess)
-        return fail(e, "count read");
-    if ((e = cudaStreamSynchronize(plan->stream)) != cudaSuccess) return fail(e, "count");
+    const cudaError_t e = read_misc(plan);
+    if (e != cudaSuccess) return fail(e, "count");
     trace_point("exact count (synced)");
     if (plan->host_misc.err) {
         g_err = "operand structure out of range (row_ptr or col_idx)";
@@ -1150,6 +1161,7 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t p) {
     }
     if (p->side_fork) cudaEventDestroy(p->side_fork);
     if (p->host_pin) cudaFreeHost(p->host_pin);
+    if (p->misc_pin) cudaFreeHost(p->misc_pin);
     if (p->stream) cudaStreamDestroy(p->stream);
     delete p;
 }
@@ -1380,14 +1392,9 @@ int rvsp_cuda_numeric(rvsp_cuda_plan_t plan, const int32_t* a_rp, const int32_t*
     }
     const bool all_dev = dev_rp && dev_ci && dev_v;
     if (!(plan->async && all_dev)) {
-        int32_t err = 0;
-        if ((e = cudaMemcpyAsync(&plan->host_misc.err, &plan->misc.as<Misc>()->err, 4,
-                                 cudaMemcpyDeviceToHost, plan->stream)) != cudaSuccess)
-            return fail(e, "error word read");
-        if ((e = cudaStreamSynchronize(plan->stream)) != cudaSuccess) return fail(e, "numeric");
+        if ((e = read_misc(plan)) != cudaSuccess) return fail(e, "numeric");
         trace_point("numeric (synced)");
-        err = plan->host_misc.err;
-        if (err) {
+        if (plan->host_misc.err) {
             g_err = "operand structure out of range (row_ptr or col_idx)";
             return RVSP_ERROR_INVALID_CSR;
         }
@@ -1466,10 +1473,9 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     plan->b_cols = b_cols;
     plan->b_nnz = -1;
     memset(plan->key, 0, sizeof(plan->key));
-    CsrView A, B;
-    int st = stage_operands(plan, a_rp, a_ci, a_v, b_rp, b_ci, b_v, false, &A, &B);
+    CsrView A{a_rp, a_ci, a_v, a_rows, a_cols, -1}, B{b_rp, b_ci, b_v, a_cols, b_cols, -1};
+    int st = analyze(plan, A, B, plan->features, nullptr, true);
     if (st) return st;
-    if ((st = analyze(plan, A, B, plan->features, nullptr, true))) return st;
     const int64_t M = a_rows;
     Misc* misc = plan->misc.as<Misc>();
     int64_t slot_products = 0;
@@ -1507,37 +1513,35 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     }
     const bool fused = plan->products <= ONESHOT_FUSED_PRODUCTS;
     int64_t cap = plan->products;
-    if ((st = count_launch(plan, A, B, slots ? slot_ci : nullptr, slot_v)) ||
+    // (the scan writes C's own row pointer, which the fill then reads)
+    cudaError_t e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
+    if (e != cudaSuccess) {
+        release();
+        return fail(e, "one-shot product");
+    }
+    if ((st = count_launch(plan, A, B, rp, slots ? slot_ci : nullptr, slot_v)) ||
         (!fused && (st = count_read(plan)))) {
         release();
         return st;
     }
     if (!fused) cap = plan->c_nnz;
     const size_t alloc = cap > 0 ? (size_t)cap : 1;
-    cudaError_t e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&ci, alloc * 4, plan->stream);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, alloc * 4, plan->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(rp, plan->c_rp.p, ((size_t)M + 1) * 4, cudaMemcpyDeviceToDevice,
-                            plan->stream);
     if (e == cudaSuccess) {
-        RowOut o{nullptr, plan->c_rp.as<int32_t>(), ci, v, &misc->err, false};
+        RowOut o{nullptr, rp, ci, v, &misc->err, false};
         if (slots) {
             o.bin_first = BIN_WARP0;
             KTime kt(plan->stream, plan->capturing, KF_COMPACT);
             k_slots_to_c<<<(unsigned)((M * 16 + 255) / 256), 256, 0, plan->stream>>>(
-                a_rows, plan->slot_off.as<int64_t>(), slot_ci, slot_v, plan->c_rp.as<int32_t>(), ci,
-                v);
+                a_rows, plan->slot_off.as<int64_t>(), slot_ci, slot_v, rp, ci, v);
             note_launch(plan, 1);
         }
         run_rows(plan, FILL, A, B, o);
         e = cudaGetLastError();
     }
     release_slots();
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&plan->host_misc, misc, sizeof(Misc), cudaMemcpyDeviceToHost,
-                            plan->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);
+    if (e == cudaSuccess) e = read_misc(plan);
     trace_point("one-shot exact (synced)");
     if (e != cudaSuccess) {
         release();

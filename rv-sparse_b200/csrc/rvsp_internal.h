@@ -148,6 +148,7 @@ struct rvsp_cuda_plan {
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr;
     int32_t* host_pin = nullptr;  // pinned words for small device->host reads
+    rvsp::Misc* misc_pin = nullptr;  // pinned landing place of Misc (read_misc)
     bool analysed = false;
     bool capturing = false;
     int32_t a_rows = 0, a_cols = 0, a_nnz = 0, b_rows = 0, b_cols = 0, b_nnz = 0;
@@ -231,7 +232,7 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
             int (*pre_sync)(rvsp_cuda_plan*) = nullptr, bool slots = false);
 int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B,
-                 int32_t* slot_ci = nullptr, float* slot_v = nullptr);
+                 int32_t* c_rp = nullptr, int32_t* slot_ci = nullptr, float* slot_v = nullptr);
 int count_read(rvsp_cuda_plan* plan);
 // One-shot exact product of device-resident operands into new device arrays
 // (rvsp_cuda_spgemm_f32's exact path when every operand array is on the
@@ -255,8 +256,13 @@ void note_launch(rvsp_cuda_plan* plan, int n);
 void reset_graph(rvsp_cuda_plan* plan);
 int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
-void launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* tile_off,
-                        int32_t* bin_rows);
+// Stable partition of the plan's rows by bin from the tiles' histograms and
+// their totals (hist); tile_off is scratch for their scan.
+int launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* hist,
+                       const int32_t* tile_hist, int32_t* tile_off, int32_t* bin_rows);
+// Waits for the plan's stream and brings its counters and flags to
+// plan->host_misc.
+cudaError_t read_misc(rvsp_cuda_plan* plan);
 int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused);
 int learned_finish(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* c_ci,
                    float* c_v);

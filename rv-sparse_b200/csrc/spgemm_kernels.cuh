@@ -140,6 +140,7 @@ struct AnalyzeOut {
     int64_t* ops;        // [rows] intermediate products per row
     int32_t* ub;         // [rows] min(ops, b_cols)
     int32_t* slot_len;   // [rows] ub of tiny and sorted rows, 0 for the others (optional)
+    int32_t* cnt;        // [rows] zeroed for the count
     uint8_t* bin;        // [rows]
     int32_t* chunk_lo;   // [rows] first heavy column chunk
     int32_t* nchunks;    // [rows] heavy column chunks (0 for other bins)
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(AN_TILE)
     if (live) {
         out.ops[row] = ops;
         out.ub[row] = ub;
+        out.cnt[row] = 0;
         if (out.slot_len) out.slot_len[row] = b < BIN_WARP0 ? ub : 0;
         out.bin[row] = (uint8_t)b;
         int clo = 0;
@@ -415,15 +417,33 @@ __global__ void __launch_bounds__(AN_TILE)
 
 // Stable partition of rows by bin: tile_off[b * tiles + tile] is where the
 // tile's rows of bin b start in bin_rows (an exclusive scan of tile_hist), so
-// every bin lists its rows in ascending order.
+// every bin lists its rows in ascending order. Without tile_off (at most
+// SCATTER_SUM_TILES tiles, where the scan's launch costs more) each CTA sums
+// what lies before its tile's rows itself: the bins before (hist) and the
+// tiles before (tile_hist).
+constexpr int SCATTER_SUM_TILES = 64;
+
 __global__ void __launch_bounds__(AN_TILE)
     k_bin_scatter(int32_t rows, const uint8_t* __restrict__ bin,
-                  const int32_t* __restrict__ tile_off, int32_t* __restrict__ bin_rows) {
+                  const int32_t* __restrict__ tile_off, const int32_t* __restrict__ hist,
+                  const int32_t* __restrict__ tile_hist, int32_t* __restrict__ bin_rows) {
     __shared__ int32_t s_wc[AN_TILE / 32][NUM_BINS];
+    __shared__ int32_t s_off[NUM_BINS];
     const int t = threadIdx.x, lane = lane_id(), warp = t >> 5;
     const int row = blockIdx.x * AN_TILE + t;
     const int b = row < rows ? (int)bin[row] : NUM_BINS;
     for (int i = t; i < (AN_TILE / 32) * NUM_BINS; i += blockDim.x) (&s_wc[0][0])[i] = 0;
+    for (int c = warp; c < NUM_BINS; c += AN_TILE / 32) {
+        int o = 0;
+        if (tile_off) {
+            o = tile_off[c * gridDim.x + blockIdx.x];
+        } else {
+            if (lane < c) o = hist[lane];
+            for (int x = lane; x < blockIdx.x; x += 32) o += tile_hist[c * gridDim.x + x];
+            o = __reduce_add_sync(FULL, o);
+        }
+        if (lane == 0) s_off[c] = o;
+    }
     __syncthreads();
     const unsigned peers = __match_any_sync(FULL, b);
     if (b < NUM_BINS && lane == __ffs(peers) - 1) s_wc[warp][b] = __popc(peers);
@@ -431,10 +451,9 @@ __global__ void __launch_bounds__(AN_TILE)
     if (b >= NUM_BINS) return;
     int before = 0;
     for (int w = 0; w < warp; ++w) before += s_wc[w][b];
-    const int pos = tile_off[b * gridDim.x + blockIdx.x] + before +
-                    __popc(peers & ((1u << lane) - 1));
-    bin_rows[pos] = row;
+    bin_rows[s_off[b] + before + __popc(peers & ((1u << lane) - 1))] = row;
 }
+static_assert(NUM_BINS <= 32, "");
 
 // Per-row product counts in bin-list order (int32; rows beyond INT32_MAX
 // products flag *overflow), the input of the position-map offsets.
