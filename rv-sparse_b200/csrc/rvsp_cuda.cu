@@ -8,7 +8,7 @@
 //
 // Pipeline of one product (all on the plan's stream):
 //   analysis   k_analyze -> (bin histogram to host) -> k_bin_scatter
-//   count      k_tiny / k_warp / k_heavy in COUNT mode -> k_scan_* -> nnz
+//   count      k_tiny_sort / k_sort / k_warp / k_heavy in COUNT mode -> k_scan_* -> nnz
 //   fill       the same kernels in FILL mode write sorted columns + values
 //   reuse      REUSE mode writes values on the known pattern (graph replay)
 
@@ -29,6 +29,7 @@
 #include "spgemm_kernels.cuh"
 #include "sort_rows.cuh"
 #include "heavy_lists.cuh"
+#include "tiny_rows.cuh"
 
 using namespace rvsp;
 
@@ -367,6 +368,21 @@ static void launch_bins(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B
             KTime kt(plan->stream, plan->capturing, KF_TINY_COUNT + MODE);
             const int32_t* lo = plan->list_off.as<int32_t>() + plan->offs.off[b];
             const int grid = (n + TINY_TPB - 1) / TINY_TPB;
+            if constexpr (MODE != REUSE) {
+                if (B.cols <= TS_MAX_COLS) {
+                    const int g = (n + 32 * TS_WARPS - 1) / (32 * TS_WARPS);
+                    if (MODE == FILL && o.maps)
+                        k_tiny_sort<MODE, MODE == FILL><<<g, TS_WARPS * 32, 0, plan->stream>>>(
+                            A, B, r, n, o.cnt, o.c_rp, o.c_ci, o.c_v, lo, plan->pm8.as<uint8_t>(),
+                            o.err, o.ctl);
+                    else
+                        k_tiny_sort<MODE, false><<<g, TS_WARPS * 32, 0, plan->stream>>>(
+                            A, B, r, n, o.cnt, o.c_rp, o.c_ci, o.c_v, nullptr, nullptr, o.err,
+                            o.ctl);
+                    note_launch(plan, 1);
+                    continue;
+                }
+            }
             if (MODE == REUSE && o.maps)
                 k_tiny_reuse_map<<<(n + 32 * TRM_WARPS - 1) / (32 * TRM_WARPS), 32 * TRM_WARPS, 0,
                                    plan->stream>>>(A, B, r, n, o.c_rp, o.c_v, lo,
@@ -976,6 +992,8 @@ int count_read(rvsp_cuda_plan* plan) {
     return RVSP_SUCCESS;
 }
 
+constexpr size_t MAPS_ASK_BYTES = (size_t)256 << 20;
+
 // Allocates the position maps and their offsets (an exclusive scan of the
 // per-row product counts in bin-list order) when the plan records them and
 // they fit: total products below 2^31 and map bytes within a quarter of the
@@ -988,14 +1006,18 @@ bool prepare_maps(rvsp_cuda_plan* plan) {
         plan->pm16_base[b] = p16;
         p16 += plan->host_misc.bin_prod[b];
     }
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
     const int64_t M = plan->a_rows;
     const size_t need = (size_t)p8 + 2 * (size_t)p16 + 8 * (size_t)(M + 1);
-    if (need > free_b / 4) return false;
+    // (the query is a driver call of some 100 us: only maps that could matter
+    // to the device's memory ask)
+    if (need > MAPS_ASK_BYTES) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (need > free_b / 4) return false;
+    }
     if (plan->pm8.ensure((size_t)p8) != cudaSuccess || plan->pm16.ensure(2 * (size_t)p16) != cudaSuccess ||
         plan->list_ops.ensure(4 * (size_t)M) != cudaSuccess ||
         plan->list_off.ensure(4 * (size_t)(M + 1)) != cudaSuccess) {

@@ -8,7 +8,8 @@
 //   k_analyze      per-row op count (rvsp_symbolic.c:41), upper bound on the
 //                  row's distinct columns, learned-model features, bin id
 //   k_bin_scatter  rows grouped by bin
-//   k_tiny<MODE>   thread per row, rows with <= 32 products
+//   k_tiny<MODE>   thread per row, rows with <= 32 products (COUNT and FILL:
+//                  k_tiny_sort in tiny_rows.cuh for all but the widest B)
 //   k_sort<E,NW,..> 1, 2 or 4 warps per row, rows of up to 2048 products sorted
 //                  in registers (sort_rows.cuh)
 //   k_warp<CAP,..> warp per row, shared-memory hash table of CAP slots
