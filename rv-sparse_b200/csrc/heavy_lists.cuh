@@ -20,13 +20,13 @@
 //   k_heavy_list  the products: a warp per item or group of items
 //
 // Measured (B200; device time, the lookup kernel k_heavy first): R-MAT 2^17,
-// COUNT 5.4 -> 3.0 ms, FILL 11.3 -> 7.3 ms; one 2^31-product row panel of R-MAT
-// 2^20, learned FILL 42.9 -> 19.8 ms (30.1 with lists alone, 19.8 with
-// sparse_stretch); reuse of R-MAT 2^16, 4.5 -> 2.6 ms; the lists themselves and
-// the items take 0.8 ms of the first and 4.0 ms of the second (the lookups'
-// tables took 0.3 and 1.5). FILL is bound by shared memory and by the latency
-// of short work on 27 resident warps an SM (issue active 54 %); COUNT by issue
-// (83 %).
+// COUNT 5.4 -> 3.0 ms, FILL 11.3 -> 5.8 ms; one 2^31-product row panel of R-MAT
+// 2^20, learned FILL 42.9 -> 17.5 ms; reuse of R-MAT 2^16, 4.5 -> 2.2 ms; the
+// lists themselves and the items take 0.8 ms of the first and 4.0 ms of the
+// second (the lookups' tables took 0.3 and 1.5). FILL is bound by the latency
+// of short work on 28 resident warps an SM and by the size of its code: every
+// path that is added costs all others (a third step in flight 12 %, a second
+// way to combine equal columns 3 %). COUNT is bound by issue (83 %).
 #pragma once
 
 #include "spgemm_kernels.cuh"
@@ -414,23 +414,53 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Marked sums: negated, so that zero bits mean no product yet (FILL needs no
+// bitmap of the columns that occur). A sum that starts from +0.0f is never
+// -0.0f (rounding to nearest gives -0.0f only for -0.0f + -0.0f), so its
+// negation never is +0.0f, and the negation of zero bits plus +0.0f is the
+// +0.0f that a sum starts from.
+__device__ __forceinline__ float marked_sum(float t) { return __fadd_rn(-t, 0.0f); }
+__device__ __forceinline__ float marked(float v) {
+    return __uint_as_float(__float_as_uint(v) ^ 0x80000000u);
+}
+
+// *sum += pr.
+template <bool MARKED>
+__device__ __forceinline__ void add_one(float* sum, float pr) {
+    *sum = MARKED ? marked(__fadd_rn(marked_sum(*sum), pr)) : __fadd_rn(*sum, pr);
+}
+
+// Adds one step's products (lane's pr into acc[at], where in) in lane order;
+// starts: the lanes after the first at which a segment starts. A segment's
+// columns are distinct, so the segments add one after the other. (Finding and
+// combining equal columns, ordered_add, takes longer however many segments
+// there are, not least by its size: code here is executed from an instruction
+// cache that it fills. R-MAT 2^17 whole, fill: 6.72 ms with ordered_add for two
+// segments and more, 6.10 for more than 8, 5.87 without.)
+template <bool MARKED>
+__device__ __forceinline__ void add_step(float* acc, int at, bool in, float pr, unsigned starts) {
+    const int turn = in ? __popc(starts & (0xffffffffu >> (31 - lane_id()))) : -1;
+    const int last = __popc(starts);
+#pragma unroll 1
+    for (int r = 0; r <= last; ++r) {
+        if (turn == r) add_one<MARKED>(acc + at, pr);
+        __syncwarp();
+    }
+}
+
 // One step of up to 32 products per half h: lane's column c[h] (relative to
-// the chunk), B value b[h] and A value a[h], in[h] where it has one; distinct
-// where no two lanes share a column.
+// the chunk), B value b[h] and A value a[h], in[h] where it has one; starts:
+// as in add_step.
 template <int MODE>
-__device__ __forceinline__ void list_add(int c, float a, float b, bool in, bool distinct, int cw,
+__device__ __forceinline__ void list_add(int c, float a, float b, bool in, unsigned starts, int cw,
                                          float* acc, unsigned* bits, int32_t* err) {
     const bool ok = in && (unsigned)c < (unsigned)cw;
     if (in && !ok) atomicOr(err, ERR_STRUCTURE);  // B row not sorted
-    if (MODE != REUSE && ok) atomicOr(&bits[c >> 5], 1u << (c & 31));
-    if (MODE != COUNT) {
+    if constexpr (MODE == COUNT) {
+        if (ok) atomicOr(&bits[c >> 5], 1u << (c & 31));
+    } else {
         const float pr = __fmul_rn(a, b);
-        if (distinct) {
-            if (ok) acc[c] = __fadd_rn(acc[c], pr);
-        } else {
-            ordered_add(acc, ok ? c : 0, ok, pr);
-        }
-        __syncwarp();
+        add_step<MODE == FILL>(acc, ok ? c : 0, ok, pr, starts);
     }
 }
 
@@ -439,9 +469,8 @@ __device__ __forceinline__ void list_add(int c, float a, float b, bool in, bool 
 // shorter than LIST_LONG are walked 32 products at a time over consecutive
 // segments: each lane finds its segment from the bits of the segments that
 // start within its 32 products; two steps are located and loaded before
-// either is accumulated; a step within one segment has distinct columns, the
-// others combine equal columns in lane order (ordered_add). Longer segments
-// are walked on their own, which needs neither.
+// either is accumulated (add_step). Longer segments are walked on their own,
+// which needs no finding.
 template <int MODE>
 __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len, float av, int lo,
                                               int cw, float* acc, unsigned* bits, int32_t* err) {
@@ -461,7 +490,7 @@ __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len
             for (int f0 = p0; f0 < p1; f0 += 64) {
                 int c[2], q[2];
                 float a[2], b[2];
-                bool one[2];
+                unsigned starts[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int rel = start - (f0 + 32 * h);
@@ -469,7 +498,7 @@ __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len
                         __reduce_or_sync(FULL, mine && (unsigned)rel < 32u ? 1u << rel : 0u);
                     const int e = max(e0 + __popc(__ballot_sync(FULL, mine && rel < 0)) +
                                           __popc(m & upto) - 1, 0);
-                    one[h] = (m >> 1) == 0;
+                    starts[h] = m & ~1u;
                     q[h] = __shfl_sync(FULL, off, e) + f0 + 32 * h + lane;
                     a[h] = MODE != COUNT ? __shfl_sync(FULL, av, e) : 0.0f;
                 }
@@ -482,9 +511,9 @@ __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len
                         if (MODE != COUNT) b[h] = __ldg(B.v + q[h]);
                     }
                 }
-                list_add<MODE>(c[0], a[0], b[0], f0 + lane < p1, one[0], cw, acc, bits, err);
+                list_add<MODE>(c[0], a[0], b[0], f0 + lane < p1, starts[0], cw, acc, bits, err);
                 if (f0 + 32 < p1)
-                    list_add<MODE>(c[1], a[1], b[1], f0 + 32 + lane < p1, one[1], cw, acc, bits,
+                    list_add<MODE>(c[1], a[1], b[1], f0 + 32 + lane < p1, starts[1], cw, acc, bits,
                                    err);
             }
             e0 = e1;
@@ -510,9 +539,10 @@ __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len
                         if ((unsigned)c[h] >= (unsigned)cw) {
                             atomicOr(err, ERR_STRUCTURE);
                         } else {
-                            if (MODE != REUSE) atomicOr(&bits[c[h] >> 5], 1u << (c[h] & 31));
-                            if (MODE != COUNT)
-                                acc[c[h]] = __fadd_rn(acc[c[h]], __fmul_rn(ae, b[h]));
+                            if (MODE == COUNT)
+                                atomicOr(&bits[c[h] >> 5], 1u << (c[h] & 31));
+                            else
+                                add_one<MODE == FILL>(acc + c[h], __fmul_rn(ae, b[h]));
                         }
                     }
                 }
@@ -565,9 +595,89 @@ constexpr int SPARSE_BYTES =
 // over it, and the sparse path's bits of segment starts.
 __host__ __device__ constexpr int list_smem_bytes(int mode, int cw) {
     return mode == COUNT ? heavy_smem_bytes(mode, cw)
-                         : (heavy_smem_bytes(mode, cw) > SPARSE_BYTES ? heavy_smem_bytes(mode, cw)
-                                                                      : SPARSE_BYTES) +
-                               64;
+                         : (4 * cw > SPARSE_BYTES ? 4 * cw : SPARSE_BYTES) + 64;
+}
+
+// Lane 0 of the learned sweep's FILL: where `total` entries of item w go, the
+// next place in the row's slot, else in the shared overflow pool, -1 if
+// neither has room (the row is then filled again).
+__device__ __forceinline__ long long learned_place(int w, int row, int total,
+                                                   int32_t* __restrict__ item_cnt,
+                                                   int32_t* __restrict__ row_cnt,
+                                                   const RowCtl& ctl) {
+    item_cnt[w] = total;
+    const int off = atomicAdd(&row_cnt[row], total);
+    const int64_t t0 = ctl.slot_off[row], cap = ctl.slot_off[row + 1] - t0;
+    long long dst = -1;
+    if ((int64_t)off + total <= cap) {
+        dst = t0 + off;
+    } else if (total > 0) {
+        const unsigned long long p = atomicAdd(ctl.pool_fill, (unsigned long long)total);
+        if ((int64_t)p + total <= ctl.pool_cap) dst = ctl.pool_base + (int64_t)p;
+    } else {
+        dst = t0;  // an empty stretch needs no room
+    }
+    ctl.item_off[w] = dst;
+    if (dst < 0) ctl.ovf[row] = 1;
+    return dst;
+}
+
+// FILL, a dense chunk's end: its marked sums leave for C in column order, 32
+// columns a step (lanes' places from the ballot of those that are there), and
+// the accumulator is left zero. R-MAT 2^17 whole, fill: 7.26 ms with a bitmap
+// and a lane writing each of its words' columns, 6.72 so.
+__device__ __forceinline__ void list_finish(int w, const HeavyItem& it, int lo, int cw, float* acc,
+                                            int32_t* __restrict__ item_cnt,
+                                            int32_t* __restrict__ row_cnt,
+                                            const int64_t* __restrict__ item_scan,
+                                            const int32_t* __restrict__ c_rp,
+                                            int32_t* __restrict__ c_ci, float* __restrict__ c_v,
+                                            int32_t* __restrict__ err, const RowCtl& ctl) {
+    const int lane = lane_id();
+    __syncwarp();
+    int64_t dst, room;
+    if (ctl.item_off) {
+        int c = 0;
+        for (int x = lane; x < cw >> 2; x += 32) {
+            const uint4 t = reinterpret_cast<const uint4*>(acc)[x];
+            c += (t.x != 0u) + (t.y != 0u) + (t.z != 0u) + (t.w != 0u);
+        }
+        c = __reduce_add_sync(FULL, c);
+        long long d = 0;
+        if (lane == 0) d = learned_place(w, it.row, c, item_cnt, row_cnt, ctl);
+        dst = __shfl_sync(FULL, d, 0);
+        room = dst >= 0 ? INT64_MAX : 0;
+    } else {
+        // (counts that disagree with this fill would only come from an
+        // operand changed in between: stay inside the row)
+        dst = (int64_t)c_rp[it.row] + (item_scan[w] - item_scan[it.first]);
+        room = (int64_t)c_rp[it.row + 1] - dst;
+    }
+    const int m = (int)max(min(room, (int64_t)cw), (int64_t)0);
+    int32_t* oc = c_ci + dst;
+    float* ov = c_v + dst;
+    const unsigned below = (1u << lane) - 1;
+    int at = 0;
+    constexpr int STEP = 4;  // (cw is a multiple of 512)
+    for (int x0 = lane; x0 < cw; x0 += 32 * STEP) {
+        float t[STEP];
+#pragma unroll
+        for (int h = 0; h < STEP; ++h) t[h] = acc[x0 + 32 * h];
+#pragma unroll
+        for (int h = 0; h < STEP; ++h) {
+            acc[x0 + 32 * h] = 0.0f;
+            const bool there = __float_as_uint(t[h]) != 0u;
+            const unsigned b = __ballot_sync(FULL, there);
+            const int pos = at + __popc(b & below);
+            if (there && pos < m) {
+                oc[pos] = lo + x0 + 32 * h;
+                ov[pos] = marked(t[h]);
+            }
+            at += __popc(b);
+        }
+    }
+    if (!ctl.item_off && at > m && lane == 0) atomicOr(err, ERR_STRUCTURE);
+    __syncwarp();
 }
 
 // Sparse stretch [lo, lo + width) of `row`, segments [s0, s1): work items w ..
@@ -617,7 +727,6 @@ __device__ __forceinline__ void sparse_stretch(
     __syncwarp();
     // (loops kept small: unrolled over the steps, the code outgrows the
     // instruction cache and the warps wait for it)
-    unsigned many = 0;  // steps that hold more than one segment
     int before = -1;
 #pragma unroll 2
     for (int s = 0; 32 * s < n; ++s) {
@@ -633,7 +742,6 @@ __device__ __forceinline__ void sparse_stretch(
             if (ok) atomicOr(&bm[c >> 5], 1u << (c & 31));
         }
         before += __popc(h);
-        many |= ((h & ~1u) != 0u ? 1u : 0u) << s;
     }
     __syncwarp();
     // rank of every 64 columns: each lane counts SPARSE_COLS / 32 columns
@@ -658,22 +766,7 @@ __device__ __forceinline__ void sparse_stretch(
     // where the entries go
     long long dst = 0;
     if (MODE == FILL && ctl.item_off) {
-        if (lane == 0) {
-            item_cnt[w] = total;
-            const int off = atomicAdd(&row_cnt[it.row], total);
-            const int64_t t0 = ctl.slot_off[it.row], cap = ctl.slot_off[it.row + 1] - t0;
-            dst = -1;
-            if ((int64_t)off + total <= cap) {
-                dst = t0 + off;
-            } else if (total > 0) {
-                const unsigned long long p = atomicAdd(ctl.pool_fill, (unsigned long long)total);
-                if ((int64_t)p + total <= ctl.pool_cap) dst = ctl.pool_base + (int64_t)p;
-            } else {
-                dst = t0;
-            }
-            ctl.item_off[w] = dst;
-            if (dst < 0) ctl.ovf[it.row] = 1;
-        }
+        if (lane == 0) dst = learned_place(w, it.row, total, item_cnt, row_cnt, ctl);
         if (lane > 0 && lane < n_items) {
             item_cnt[w + lane] = 0;
             ctl.item_off[w + lane] = ctl.slot_off[it.row];
@@ -700,12 +793,7 @@ __device__ __forceinline__ void sparse_stretch(
                 (upper ? __popc(b2.y & below) : 0);
             cols[r] = (uint16_t)c;
         }
-        if (many >> s & 1u) {
-            ordered_add(acc, r, in, pr);
-        } else if (in) {
-            acc[r] = __fadd_rn(acc[r], pr);
-        }
-        __syncwarp();
+        add_step<false>(acc, r, in, pr, heads[s] & ~1u);
     }
     dst = __shfl_sync(FULL, dst, 0);
     // (counts that disagree with this fill would only come from an operand
@@ -744,7 +832,7 @@ __global__ void __launch_bounds__(LIST_MAX_WARPS * 32)
     const int bytes = list_smem_bytes(MODE, cw);
     unsigned char* mine = smem + warp * bytes;
     float* acc = reinterpret_cast<float*>(mine);
-    unsigned* bits = reinterpret_cast<unsigned*>(mine + (MODE == COUNT ? 0 : 4 * cw));
+    unsigned* bits = reinterpret_cast<unsigned*>(mine);  // (COUNT)
     for (int x = lane; x < bytes / 16; x += 32)
         reinterpret_cast<float4*>(mine)[x] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
@@ -833,8 +921,8 @@ __global__ void __launch_bounds__(LIST_MAX_WARPS * 32)
                     }
                     if (MODE == FILL) {
                         const HeavyItem mineit{it.row, it.chunk + k, it.first, it.a0};
-                        heavy_finish<MODE>(B, item, mineit, row, lo, cw, acc, bits, item_cnt,
-                                           row_cnt, item_scan, c_rp, c_ci, c_v, err, ctl);
+                        list_finish(item, mineit, lo, cw, acc, item_cnt, row_cnt, item_scan, c_rp,
+                                    c_ci, c_v, err, ctl);
                     } else {
                         // REUSE: the chunk's entries of C, in order, and back to zero
                         __syncwarp();

@@ -8,7 +8,7 @@ import pytest
 
 import oracle
 import rvsp_b200 as rv
-from gpu_util import DevCSR, dev, oneshot
+from gpu_util import DevCSR, bits, dev, oneshot
 from rvsp_b200 import gen
 from test_parity_gpu import assert_same, oracle_full
 
@@ -66,3 +66,26 @@ def test_heavy_rows_match_oracle(gpu_lib, cols, cw):
         d.close()
     finally:
         rv.set_default_params(None)
+
+
+def test_zero_sums_and_non_finite_values(gpu_lib):
+    """Sums that cancel, that are zero of either sign and that are not finite
+    in dense chunks and sparse stretches: every occurring column is there, bit
+    for bit (a NaN as a NaN: its payload is not specified)."""
+    A, B = _product(40000, 7)
+    rng = np.random.default_rng(11)
+    A.values[:] = rng.choice(np.float32([1, -1, 0.0, -0.0]), A.nnz)
+    B.values[:] = rng.choice(np.float32([1, -1, 0.0, -0.0, 2]), B.nnz)
+    B.values[5::997] = np.inf
+    want = oracle_full(A, B)
+    assert (want[2] == 0).sum() > 1000 and np.isnan(want[2]).any()
+    nan = np.isnan(want[2])
+    try:
+        rv.check(rv.set_default_params((32, 2, 64, 11)))
+        for algo in (rv.RVSP_CUDA_ALGO_EXACT, rv.RVSP_CUDA_ALGO_LEARNED):
+            got = oneshot(A, B, algo=algo)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+            assert np.array_equal(np.isnan(got[2]), nan)
+            assert np.array_equal(bits(got[2])[~nan], bits(want[2])[~nan])
+    finally:
+        rv.check(rv.set_default_params(None))
