@@ -7,7 +7,7 @@
 // numeric-only pass used when the descriptor is reused.
 //
 // Pipeline of one product (all on the plan's stream):
-//   analysis   k_analyze -> (bin histogram to host) -> k_bin_scatter
+//   analysis   k_analyze (k_analyze_big) -> (bin histogram to host) -> k_bin_scatter
 //   count      k_tiny_sort / k_sort / k_warp / k_heavy in COUNT mode -> k_scan_* -> nnz
 //   fill       the same kernels in FILL mode write sorted columns + values
 //   reuse      REUSE mode writes values on the known pattern (graph replay)
@@ -633,9 +633,21 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
                    misc->nnz_ab};
     {
         KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
-        k_analyze<<<(unsigned)tiles, AN_TILE, 0, plan->stream>>>(A, B, out, plan->params);
+        // (the list lies in tile_off, which the scan of the bins fills later)
+        AnBig big{&misc->big_tiles, nullptr, nullptr, nullptr};
+        if (tiles >= AN_BIG_MIN_TILES && tiles <= AN_BIG_MAX_TILES) {
+            big.first = plan->tile_off.as<int64_t>();
+            big.tile = reinterpret_cast<int32_t*>(big.first + tiles);
+            big.done = big.tile + tiles;
+        }
+        k_analyze<<<(unsigned)tiles, AN_TILE, 0, plan->stream>>>(A, B, out, plan->params, big);
+        note_launch(plan, 1);
+        if (big.done) {
+            k_analyze_big<<<4 * g_sms, AN_TILE, 0, plan->stream>>>(A, B, out, plan->params, big,
+                                                                  (int)tiles);
+            note_launch(plan, 1);
+        }
     }
-    note_launch(plan, 1);
     int st = RVSP_SUCCESS;
     if (pre_sync && (st = pre_sync(plan))) return st;
     if ((e = read_misc(plan)) != cudaSuccess) return fail(e, "analysis");

@@ -55,6 +55,7 @@ struct Misc {
     int32_t heavy_queue;       // next heavy work item of the running launch
     int32_t row_queue;         // next row of the running warp-bin launch
     unsigned long long pool_fill;  // learned path: entries placed in the overflow pool
+    unsigned long long big_tiles;  // analysis: tiles left to k_analyze_big (AnBig::total)
     int32_t nnz_ab[2];         // nnz of A and B as the analysis read them (operands
                                // whose nnz the host did not know)
 };

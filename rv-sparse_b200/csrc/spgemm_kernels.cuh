@@ -180,19 +180,200 @@ __device__ __forceinline__ void warp_bin_add(int key, int nkeys, unsigned long l
 }
 
 // Rows of at most AN_SHORT entries are summarised by their own thread;
-// longer rows by the whole CTA striding over their entries.
+// longer rows by the whole CTA striding over their entries, or, in a tile of
+// more than AN_BIG entries and AN_BIG_MEANS times the mean, by k_analyze_big:
+// one CTA held 9 % of the entries of a whole R-MAT graph of 2^17 rows, and the
+// analysis, 0.05 ms of work, took the 0.74 ms that this CTA did; 0.10 with
+// both kernels (8192 entries and 8 means: 0.15). Elsewhere the second launch
+// costs 2 us; a tile can only hold that much more than the mean among many,
+// and short calls (under AN_BIG_MIN_TILES) go without.
 constexpr int AN_SHORT = 32;
+constexpr int AN_BIG = 4096;
+constexpr int AN_BIG_MEANS = 2;
+constexpr int AN_BIG_CHUNK = 1024;  // entries a CTA of k_analyze_big takes at a time
+
+// What a tile's CTA keeps of its rows.
+struct AnTile {
+    int32_t rp[AN_TILE + 1];
+    unsigned long long ops[AN_TILE];
+    int32_t maxlen[AN_TILE], minc[AN_TILE], maxc[AN_TILE];
+    int32_t hist[NUM_BINS];
+    unsigned long long bprod[NUM_BINS];
+    unsigned long long items, prod, units, cells;
+};
+
+// Tiles left to k_analyze_big: their number << 44 | their chunks, and for each
+// the first chunk, the tile and the chunks that are done. Their rows' sums so
+// far wait in out.ops, ub (longest B row), chunk_lo and nchunks (first and last
+// column). At most 2^18 tiles of 2^21 chunks: neither half can overflow, even
+// by a broken row pointer.
+struct AnBig {
+    unsigned long long* total;
+    int64_t* first;
+    int32_t *tile, *done;  // (null: no tile is left)
+};
+constexpr int64_t AN_BIG_MIN_TILES = 32, AN_BIG_MAX_TILES = int64_t(1) << 18;
+
+__device__ __forceinline__ void an_clear(AnTile& s, int t) {
+    if (t < NUM_BINS) {
+        s.hist[t] = 0;
+        s.bprod[t] = 0;
+    }
+    if (t == 0) {
+        s.items = 0;
+        s.prod = 0;
+        s.units = 0;
+        s.cells = 0;
+    }
+}
+
+// The tile's entries [p0, p1) that are of long rows, the CTA striding over
+// them; a warp whose entries all fall in one row (a long row's stretch)
+// combines them in registers and updates the row once, instead of 32 lanes
+// contending for the same shared counters. Four entries a thread, their three
+// dependent loads in flight together.
+__device__ __forceinline__ void an_long(const CsrView& A, const CsrView& B, AnTile& s, int nr,
+                                        int p0, int p1, int32_t* err) {
+    const int t = threadIdx.x, lane = t & 31;
+    for (int64_t base0 = p0 + (t & ~31); base0 < p1; base0 += 4 * blockDim.x) {
+        int lo[4], len[4], first[4], last[4], k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t p = base0 + u * (int)blockDim.x + lane;
+            lo[u] = -1;
+            len[u] = 0;
+            first[u] = INT_MAX;
+            last[u] = -1;
+            k[u] = -1;
+            if (p < p1) {
+                int l = 0, h = nr;  // largest i with s.rp[i] <= p
+                while (h - l > 1) {
+                    const int mid = (l + h) >> 1;
+                    if (s.rp[mid] <= p) l = mid; else h = mid;
+                }
+                if (s.rp[l + 1] - s.rp[l] > AN_SHORT) {
+                    lo[u] = l;
+                    k[u] = A.ci[p];
+                }
+            }
+        }
+        int bs[4], be[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            bs[u] = be[u] = 0;
+            if (lo[u] >= 0) row_range(B, k[u], &bs[u], &be[u], err);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            int f = 0, g = -1;
+            if (be[u] > bs[u]) {
+                f = B.ci[bs[u]];
+                g = B.ci[be[u] - 1];
+            }
+            if (be[u] <= bs[u]) {
+                lo[u] = -1;
+            } else if (f < 0 || g >= B.cols || g < f) {
+                atomicOr(err, ERR_STRUCTURE);
+                lo[u] = -1;
+            } else {
+                len[u] = be[u] - bs[u];
+                first[u] = f;
+                last[u] = g;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned has = __ballot_sync(FULL, lo[u] >= 0);
+            if (!has) continue;
+            const int lead = __ffs(has) - 1;
+            const int lrow = __shfl_sync(FULL, lo[u], lead);
+            if (__all_sync(FULL, lo[u] < 0 || lo[u] == lrow)) {
+                unsigned long long sum = (unsigned long long)len[u];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+                const int mxl = __reduce_max_sync(FULL, len[u]);
+                const int mnc = __reduce_min_sync(FULL, first[u]);
+                const int mxc = __reduce_max_sync(FULL, last[u]);
+                if (lane == lead) {
+                    atomicAdd(&s.ops[lrow], sum);
+                    atomicMax(&s.maxlen[lrow], mxl);
+                    atomicMin(&s.minc[lrow], mnc);
+                    atomicMax(&s.maxc[lrow], mxc);
+                }
+            } else if (lo[u] >= 0) {
+                atomicAdd(&s.ops[lo[u]], (unsigned long long)len[u]);
+                atomicMax(&s.maxlen[lo[u]], len[u]);
+                atomicMin(&s.minc[lo[u]], first[u]);
+                atomicMax(&s.maxc[lo[u]], last[u]);
+            }
+        }
+    }
+}
+
+// Per row: bound, bin, heavy chunks, features; warp-aggregated counters.
+__device__ __forceinline__ void an_finish(const AnalyzeOut& out, const BinParams& P, int b_cols,
+                                          AnTile& s, int tile, int tiles, int nr) {
+    const int t = threadIdx.x, r0 = tile * AN_TILE;
+    const bool live = t < nr;
+    const int row = r0 + t;
+    const int64_t ops = live ? (int64_t)s.ops[t] : 0;
+    const int32_t ub = (int32_t)min(ops, (int64_t)b_cols);
+    const int b = live ? bin_of(ops, ub, b_cols, P) : -1;
+    int nch = 0;
+    if (live) {
+        out.ops[row] = ops;
+        out.ub[row] = ub;
+        out.cnt[row] = 0;
+        if (out.slot_len) out.slot_len[row] = b < BIN_WARP0 ? ub : 0;
+        out.bin[row] = (uint8_t)b;
+        int clo = 0;
+        if (b == BIN_HEAVY) {
+            clo = s.minc[t] >> P.heavy_cw_log2;
+            nch = (s.maxc[t] >> P.heavy_cw_log2) - clo + 1;
+        }
+        out.chunk_lo[row] = clo;
+        out.nchunks[row] = nch;
+        if (out.feat) {
+            const int anz = s.rp[t + 1] - s.rp[t];
+            const int span = ops > 0 ? s.maxc[t] - s.minc[t] + 1 : 0;
+            out.feat[row] = make_float4((float)anz, (float)ops, (float)s.maxlen[t], (float)span);
+        }
+    }
+    warp_bin_add(b, NUM_BINS, (unsigned long long)ops, s.hist, s.bprod);
+    const unsigned long long wprod = warp_sum64((unsigned long long)ops);
+    const unsigned long long witems = warp_sum64((unsigned long long)nch);
+    if (__any_sync(FULL, nch > 0)) {  // heavy rows: their units and (chunk, unit) cells
+        const unsigned long long u =
+            nch > 0 ? (unsigned long long)(s.rp[t + 1] - s.rp[t] + HEAVY_UNIT - 1) / HEAVY_UNIT : 0ull;
+        const unsigned long long wu = warp_sum64(u), wc = warp_sum64(u * (unsigned long long)nch);
+        if (lane_id() == 0) {
+            atomicAdd(&s.units, wu);
+            atomicAdd(&s.cells, wc);
+        }
+    }
+    if (lane_id() == 0) {
+        if (wprod) atomicAdd(&s.prod, wprod);
+        if (witems) atomicAdd(&s.items, witems);
+    }
+    __syncthreads();
+    if (t < NUM_BINS) {
+        out.tile_hist[t * tiles + tile] = s.hist[t];
+        if (s.hist[t]) atomicAdd(&out.hist[t], s.hist[t]);
+        if (s.bprod[t]) atomicAdd((unsigned long long*)&out.bin_prod[t], s.bprod[t]);
+    }
+    if (t == 0) {
+        if (s.items) {
+            atomicAdd((unsigned long long*)&out.totals[0], s.items);
+            atomicAdd((unsigned long long*)&out.totals[2], s.units);
+            atomicAdd((unsigned long long*)&out.totals[3], s.cells);
+        }
+        atomicAdd((unsigned long long*)&out.totals[1], s.prod);
+    }
+}
 
 __global__ void __launch_bounds__(AN_TILE)
-    k_analyze(CsrView A, CsrView B, AnalyzeOut out, BinParams P) {
-    __shared__ int32_t s_rp[AN_TILE + 1];
-    __shared__ unsigned long long s_ops[AN_TILE];
-    __shared__ int32_t s_maxlen[AN_TILE];
-    __shared__ int32_t s_minc[AN_TILE];
-    __shared__ int32_t s_maxc[AN_TILE];
-    __shared__ int32_t s_hist[NUM_BINS];
-    __shared__ unsigned long long s_bprod[NUM_BINS];
-    __shared__ unsigned long long s_items, s_prod, s_units, s_cells;
+    k_analyze(CsrView A, CsrView B, AnalyzeOut out, BinParams P, AnBig big) {
+    __shared__ AnTile s;
     __shared__ int s_long;
 
     // An operand's nnz passed as -1 is not known on the host (a device-
@@ -208,22 +389,13 @@ __global__ void __launch_bounds__(AN_TILE)
     const int r0 = blockIdx.x * AN_TILE;
     const int nr = min(AN_TILE, A.rows - r0);
     const int t = threadIdx.x;
-    for (int i = t; i <= nr; i += blockDim.x) s_rp[i] = A.rp[r0 + i];
-    if (t < NUM_BINS) {
-        s_hist[t] = 0;
-        s_bprod[t] = 0;
-    }
-    if (t == 0) {
-        s_items = 0;
-        s_prod = 0;
-        s_units = 0;
-        s_cells = 0;
-        s_long = 0;
-    }
+    for (int i = t; i <= nr; i += blockDim.x) s.rp[i] = A.rp[r0 + i];
+    an_clear(s, t);
+    if (t == 0) s_long = 0;
     __syncthreads();
     // short rows: one thread each, no atomics
     if (t < nr) {
-        const int s0 = s_rp[t], s1 = s_rp[t + 1];
+        const int s0 = s.rp[t], s1 = s.rp[t + 1];
         unsigned long long ops = 0;
         int maxlen = 0, minc = INT_MAX, maxc = -1;
         if (s0 < 0 || s1 < s0 || s1 > A.nnz) {
@@ -267,152 +439,94 @@ __global__ void __launch_bounds__(AN_TILE)
         } else {
             s_long = 1;
         }
-        s_ops[t] = ops;
-        s_maxlen[t] = maxlen;
-        s_minc[t] = minc;
-        s_maxc[t] = maxc;
+        s.ops[t] = ops;
+        s.maxlen[t] = maxlen;
+        s.minc[t] = minc;
+        s.maxc[t] = maxc;
     }
     __syncthreads();
     if (s_long) {
-        // long rows: the CTA strides over the tile's entries, skipping short
-        // rows; a warp whose entries all fall in one row (a long row's
-        // stretch) combines them in registers and updates the row once,
-        // instead of 32 lanes contending for the same shared counters
-        const int p0 = max(s_rp[0], 0), p1 = min(s_rp[nr], A.nnz);
-        const int lane = t & 31;
-        // four entries a thread, their three dependent loads in flight
-        // together: a tile of hub rows is one CTA's (R-MAT 2^17: 0.78 ms of
-        // the analysis with one entry a thread)
-        for (int base0 = p0 + (t & ~31); base0 < p1; base0 += 4 * blockDim.x) {
-            int lo[4], len[4], first[4], last[4], k[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int64_t p = (int64_t)base0 + u * (int)blockDim.x + lane;
-                lo[u] = -1;
-                len[u] = 0;
-                first[u] = INT_MAX;
-                last[u] = -1;
-                k[u] = -1;
-                if (p < p1) {
-                    int l = 0, h = nr;  // largest i with s_rp[i] <= p
-                    while (h - l > 1) {
-                        const int mid = (l + h) >> 1;
-                        if (s_rp[mid] <= p) l = mid; else h = mid;
-                    }
-                    if (s_rp[l + 1] - s_rp[l] > AN_SHORT) {
-                        lo[u] = l;
-                        k[u] = A.ci[p];
-                    }
-                }
+        const int p0 = max(s.rp[0], 0), p1 = min(s.rp[nr], A.nnz);
+        const int64_t mean = (int64_t)A.nnz / gridDim.x;
+        if (big.done && p1 - p0 > AN_BIG && p1 - p0 > AN_BIG_MEANS * mean) {
+            if (t == 0) {
+                const int chunks = (p1 - p0 + AN_BIG_CHUNK - 1) / AN_BIG_CHUNK;
+                const unsigned long long at =
+                    atomicAdd(big.total, (1ull << 44) + (unsigned long long)chunks);
+                const int i = (int)(at >> 44);
+                big.first[i] = (int64_t)(at & ((1ull << 44) - 1));
+                big.tile[i] = blockIdx.x;
+                big.done[i] = 0;
             }
-            int bs[4], be[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                bs[u] = be[u] = 0;
-                if (lo[u] >= 0) row_range(B, k[u], &bs[u], &be[u], out.err);
+            if (t < nr) {
+                out.ops[r0 + t] = (int64_t)s.ops[t];
+                out.ub[r0 + t] = s.maxlen[t];
+                out.chunk_lo[r0 + t] = s.minc[t];
+                out.nchunks[r0 + t] = s.maxc[t];
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                int f = 0, g = -1;
-                if (be[u] > bs[u]) {
-                    f = B.ci[bs[u]];
-                    g = B.ci[be[u] - 1];
-                }
-                if (be[u] <= bs[u]) {
-                    lo[u] = -1;
-                } else if (f < 0 || g >= B.cols || g < f) {
-                    atomicOr(out.err, ERR_STRUCTURE);
-                    lo[u] = -1;
-                } else {
-                    len[u] = be[u] - bs[u];
-                    first[u] = f;
-                    last[u] = g;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const unsigned has = __ballot_sync(FULL, lo[u] >= 0);
-                if (!has) continue;
-                const int lead = __ffs(has) - 1;
-                const int lrow = __shfl_sync(FULL, lo[u], lead);
-                if (__all_sync(FULL, lo[u] < 0 || lo[u] == lrow)) {
-                    unsigned long long sum = (unsigned long long)len[u];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
-                    const int mxl = __reduce_max_sync(FULL, len[u]);
-                    const int mnc = __reduce_min_sync(FULL, first[u]);
-                    const int mxc = __reduce_max_sync(FULL, last[u]);
-                    if (lane == lead) {
-                        atomicAdd(&s_ops[lrow], sum);
-                        atomicMax(&s_maxlen[lrow], mxl);
-                        atomicMin(&s_minc[lrow], mnc);
-                        atomicMax(&s_maxc[lrow], mxc);
-                    }
-                } else if (lo[u] >= 0) {
-                    atomicAdd(&s_ops[lo[u]], (unsigned long long)len[u]);
-                    atomicMax(&s_maxlen[lo[u]], len[u]);
-                    atomicMin(&s_minc[lo[u]], first[u]);
-                    atomicMax(&s_maxc[lo[u]], last[u]);
-                }
-            }
+            return;
         }
+        an_long(A, B, s, nr, p0, p1, out.err);
         __syncthreads();
     }
-    // per row: bound, bin, heavy chunks, features; warp-aggregated counters
-    const bool live = t < nr;
-    const int row = r0 + t;
-    const int64_t ops = live ? (int64_t)s_ops[t] : 0;
-    const int32_t ub = (int32_t)min(ops, (int64_t)B.cols);
-    const int b = live ? bin_of(ops, ub, B.cols, P) : -1;
-    int nch = 0;
-    if (live) {
-        out.ops[row] = ops;
-        out.ub[row] = ub;
-        out.cnt[row] = 0;
-        if (out.slot_len) out.slot_len[row] = b < BIN_WARP0 ? ub : 0;
-        out.bin[row] = (uint8_t)b;
-        int clo = 0;
-        if (b == BIN_HEAVY) {
-            clo = s_minc[t] >> P.heavy_cw_log2;
-            nch = (s_maxc[t] >> P.heavy_cw_log2) - clo + 1;
+    an_finish(out, P, B.cols, s, blockIdx.x, gridDim.x, nr);
+}
+
+// The long rows of the tiles that k_analyze listed, AN_BIG_CHUNK entries a CTA
+// at a time; the CTA that ends a tile's last chunk finishes the tile.
+__global__ void __launch_bounds__(AN_TILE)
+    k_analyze_big(CsrView A, CsrView B, AnalyzeOut out, BinParams P, AnBig big, int tiles) {
+    __shared__ AnTile s;
+    __shared__ int s_last;
+    const unsigned long long total = *big.total;
+    const int n = (int)(total >> 44);
+    if (n == 0) return;
+    const int64_t chunks = (int64_t)(total & ((1ull << 44) - 1));
+    if (A.nnz < 0) A.nnz = A.rp[A.rows];
+    if (B.nnz < 0) B.nnz = B.rp[B.rows];
+    const int t = threadIdx.x;
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        int lo = 0, hi = n;  // the last listed tile that starts at c or before
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (big.first[mid] <= c) lo = mid; else hi = mid;
         }
-        out.chunk_lo[row] = clo;
-        out.nchunks[row] = nch;
-        if (out.feat) {
-            const int anz = s_rp[t + 1] - s_rp[t];
-            const int span = ops > 0 ? s_maxc[t] - s_minc[t] + 1 : 0;
-            out.feat[row] = make_float4((float)anz, (float)ops, (float)s_maxlen[t], (float)span);
+        const int tile = big.tile[lo], r0 = tile * AN_TILE, nr = min(AN_TILE, A.rows - r0);
+        __syncthreads();  // (the last chunk's readers of s)
+        for (int i = t; i <= nr; i += blockDim.x) s.rp[i] = A.rp[r0 + i];
+        s.ops[t] = 0;
+        s.maxlen[t] = 0;
+        s.minc[t] = INT_MAX;
+        s.maxc[t] = -1;
+        an_clear(s, t);
+        __syncthreads();
+        const int p0 = max(s.rp[0], 0), p1 = min(s.rp[nr], A.nnz);
+        const int mine = (int)(c - big.first[lo]);
+        const int own = (p1 - p0 + AN_BIG_CHUNK - 1) / AN_BIG_CHUNK;
+        const int q0 = p0 + mine * AN_BIG_CHUNK;
+        an_long(A, B, s, nr, q0, (int)min((int64_t)q0 + AN_BIG_CHUNK, (int64_t)p1), out.err);
+        __syncthreads();
+        if (t < nr && s.ops[t]) {
+            atomicAdd((unsigned long long*)&out.ops[r0 + t], s.ops[t]);
+            atomicMax(&out.ub[r0 + t], s.maxlen[t]);
+            atomicMin(&out.chunk_lo[r0 + t], s.minc[t]);
+            atomicMax(&out.nchunks[r0 + t], s.maxc[t]);
         }
-    }
-    warp_bin_add(b, NUM_BINS, (unsigned long long)ops, s_hist, s_bprod);
-    const unsigned long long wprod = warp_sum64((unsigned long long)ops);
-    const unsigned long long witems = warp_sum64((unsigned long long)nch);
-    if (__any_sync(FULL, nch > 0)) {  // heavy rows: their units and (chunk, unit) cells
-        const unsigned long long u =
-            nch > 0 ? (unsigned long long)(s_rp[t + 1] - s_rp[t] + HEAVY_UNIT - 1) / HEAVY_UNIT : 0ull;
-        const unsigned long long wu = warp_sum64(u), wc = warp_sum64(u * (unsigned long long)nch);
-        if (lane_id() == 0) {
-            atomicAdd(&s_units, wu);
-            atomicAdd(&s_cells, wc);
+        __threadfence();
+        __syncthreads();
+        if (t == 0) s_last = atomicAdd(&big.done[lo], 1) == own - 1;
+        __syncthreads();
+        if (s_last) {
+            __threadfence();
+            if (t < nr) {
+                s.ops[t] = (unsigned long long)__ldcg(&out.ops[r0 + t]);
+                s.maxlen[t] = __ldcg(&out.ub[r0 + t]);
+                s.minc[t] = __ldcg(&out.chunk_lo[r0 + t]);
+                s.maxc[t] = __ldcg(&out.nchunks[r0 + t]);
+            }
+            __syncthreads();
+            an_finish(out, P, B.cols, s, tile, tiles, nr);
         }
-    }
-    if (lane_id() == 0) {
-        if (wprod) atomicAdd(&s_prod, wprod);
-        if (witems) atomicAdd(&s_items, witems);
-    }
-    __syncthreads();
-    if (t < NUM_BINS) {
-        out.tile_hist[t * gridDim.x + blockIdx.x] = s_hist[t];
-        if (s_hist[t]) atomicAdd(&out.hist[t], s_hist[t]);
-        if (s_bprod[t]) atomicAdd((unsigned long long*)&out.bin_prod[t], s_bprod[t]);
-    }
-    if (t == 0) {
-        if (s_items) {
-            atomicAdd((unsigned long long*)&out.totals[0], s_items);
-            atomicAdd((unsigned long long*)&out.totals[2], s_units);
-            atomicAdd((unsigned long long*)&out.totals[3], s_cells);
-        }
-        atomicAdd((unsigned long long*)&out.totals[1], s_prod);
     }
 }
 
@@ -454,7 +568,7 @@ __global__ void __launch_bounds__(AN_TILE)
     for (int w = 0; w < warp; ++w) before += s_wc[w][b];
     bin_rows[s_off[b] + before + __popc(peers & ((1u << lane) - 1))] = row;
 }
-static_assert(NUM_BINS <= 32, "");
+static_assert(NUM_BINS <= 32 && NUM_BINS >= 4, "");
 
 // Per-row product counts in bin-list order (int32; rows beyond INT32_MAX
 // products flag *overflow), the input of the position-map offsets.
