@@ -62,8 +62,9 @@ RVSP_CUDA_API void rvsp_cuda_free(void *device_ptr);
  * RVSP_OWNS_HOST; the counterpart of free() at rv-sparse
  * src/core/matrix.c:99-104). Such arrays may also be released with free();
  * through this call arrays of 64 MiB and more are kept (at most 4, within a
- * sixteenth of host memory, 32 GiB at most) and handed out again to later
- * products, whose copy-back then writes pages already mapped.
+ * sixteenth of host memory, 32 GiB at most), and smaller ones of 256 KiB and
+ * more (at most 8, within 128 MiB), and handed out again to later products,
+ * whose copy-back then writes pages already mapped.
  * RVSP_HOST_CACHE=0 in the environment makes it a plain free(). NULL is
  * accepted.
  * Pageable host results of 64 MiB and more (and pageable operands of 16 MiB
@@ -101,6 +102,8 @@ RVSP_CUDA_API void *rvsp_cuda_plan_stream(rvsp_cuda_plan_t plan);
  *                     (1..4: load factor at most 2/3, 4/5, 8/9, 16/17)
  *   [2] warp_cap_max  largest warp hash table, a power of two in 64..4096;
  *                     rows needing more are split into column chunks, a warp each
+ *                     (rows under it with at most 2048 products, four to a
+ *                     possible column at most, are sorted instead of hashed)
  *   [3] heavy_cw_log2 log2 of the columns of one chunk (9..13)
  * Defaults: 32, 2, 2048, 11. Results do not depend on the parameters (the
  * pattern and the values are bit-identical under every valid setting); only
