@@ -313,14 +313,19 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+constexpr int COMPACT_LIST = 128;  // entries a chunk, on average, up to which 32 are one list
+
 // Copy the chunks of heavy rows finished in their slots (or the overflow
 // pool) into C, each chunk's entries from where the sweep put them to their
 // place in C (its row's start plus the counts of the row's earlier chunks).
 // One warp per 32 consecutive work items (grid-stride): lane l loads item l's
 // bookkeeping (all 32 items' loads in flight together), then the warp copies
-// the 32 chunks' entries as one list, 128 entries per step with each lane's
-// four loads issued before its stores; each lane finds its entry's chunk in
-// the scan of the chunks' counts. A chunk's source and destination offsets
+// the chunks one after the other, 128 entries per step with each lane's four
+// loads issued before its stores, or, where they have few entries, the 32
+// chunks' entries as one list, in which each lane finds its entry's chunk by
+// the scan of the chunks' counts (nine shuffles an entry: a row panel of R-MAT
+// 2^20, some 700 entries a stretch, took 4.14 ms as lists, 3.46 one after the
+// other). A chunk's source and destination offsets
 // are kept less the chunk's first index in the list, so an entry's two
 // addresses are one shuffle each (40 registers: 6 CTAs per SM). Items of a
 // row are consecutive, so the stores run contiguously through C.
@@ -355,6 +360,34 @@ __global__ void __launch_bounds__(256)
             if (lane >= o) incl += y;
         }
         const int total = __shfl_sync(FULL, incl, 31);
+        const unsigned some = __ballot_sync(FULL, k > 0);
+        if (total > COMPACT_LIST * __popc(some)) {
+            for (unsigned left = some; left; left &= left - 1) {
+                const int j = __ffs(left) - 1;
+                const int kj = __shfl_sync(FULL, k, j);
+                const int64_t sj = __shfl_sync(FULL, src, j);
+                const int64_t dj = __shfl_sync(FULL, dst, j);
+                for (int x0 = lane; x0 < kj; x0 += 128) {
+                    int32_t ci[4];
+                    float v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (x0 + 32 * u < kj) {
+                            ci[u] = tmp_ci[sj + x0 + 32 * u];
+                            v[u] = tmp_v[sj + x0 + 32 * u];
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (x0 + 32 * u < kj) {
+                            c_ci[dj + x0 + 32 * u] = ci[u];
+                            c_v[dj + x0 + 32 * u] = v[u];
+                        }
+                    }
+                }
+            }
+            continue;
+        }
         src -= incl - k;
         dst -= incl - k;
         for (int e0 = 0; e0 < total; e0 += 128) {
