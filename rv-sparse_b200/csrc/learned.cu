@@ -196,8 +196,9 @@ __global__ void k_need(int32_t rows, const uint8_t* __restrict__ lbin,
 }
 
 // Copy finished rows from their slots into C, one warp per row (the warp-bin
-// rows: tens to thousands of entries each), 128 entries per step with each
-// lane's four loads issued before its stores. Coalesced on both sides.
+// rows: tens to thousands of entries each), 256 entries per step with each
+// lane's eight loads issued before its stores (128 products of 256..65536 rows:
+// 2.05 ms, 2.28 with four). Coalesced on both sides.
 __global__ void __launch_bounds__(256)
     k_compact_rows(const int32_t* __restrict__ rows, int32_t n, const uint8_t* __restrict__ need,
                    const int32_t* __restrict__ cnt, const int64_t* __restrict__ slot_off,
@@ -212,11 +213,11 @@ __global__ void __launch_bounds__(256)
     const int k = cnt[row];
     const int64_t src = slot_off[row];
     const int dst = c_rp[row];
-    for (int x0 = 0; x0 < k; x0 += 128) {
-        int32_t ci[4];
-        float v[4];
+    for (int x0 = 0; x0 < k; x0 += 256) {
+        int32_t ci[8];
+        float v[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const int x = x0 + 32 * u + lane;
             if (x < k) {
                 ci[u] = tmp_ci[src + x];
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(256)
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const int x = x0 + 32 * u + lane;
             if (x < k) {
                 c_ci[dst + x] = ci[u];

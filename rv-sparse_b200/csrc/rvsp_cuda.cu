@@ -1450,14 +1450,15 @@ constexpr int64_t ONESHOT_FUSED_PRODUCTS = int64_t(1) << 25;
 // counted, into slots of their upper bound (8 bytes a product), and copied
 // into C once the row pointer is known: the copy moves 16 bytes an entry,
 // where counting first means sorting every product twice (tall-skinny 2M x
-// 100k: counts 2.1 ms, copy 1.1 ms, call 8.0 -> 7.0 ms). Below
+// 100k: counts 2.1 ms, copy 0.9 ms, call 8.0 -> 6.7 ms). Below
 // SLOT_MIN_PRODUCTS the scan of the slots and the copy cost what the counts do
 // (4096^2 x 16, 2^20 products: 113 us against 105); above SLOT_MAX_PRODUCTS (4
 // GiB of slots) the rows are counted.
 constexpr int64_t SLOT_MIN_PRODUCTS = int64_t(1) << 22;
 constexpr int64_t SLOT_MAX_PRODUCTS = int64_t(1) << 29;
 
-// Rows from their slots into C, 16 lanes a row; rows without a slot are left.
+// Rows from their slots into C, 16 lanes a row and eight entries a lane in
+// flight (that product: 0.92 ms, 1.11 with four); rows without a slot are left.
 static __global__ void __launch_bounds__(256)
     k_slots_to_c(int32_t rows, const int64_t* __restrict__ slot_off,
                  const int32_t* __restrict__ slot_ci, const float* __restrict__ slot_v,
@@ -1468,11 +1469,11 @@ static __global__ void __launch_bounds__(256)
     const int64_t src = slot_off[row];
     if (slot_off[row + 1] == src) return;
     const int dst = rp[row], n = rp[row + 1] - dst;
-    for (int x0 = lane; x0 < n; x0 += 64) {
-        int32_t c[4];
-        float y[4];
+    for (int x0 = lane; x0 < n; x0 += 128) {
+        int32_t c[8];
+        float y[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const int x = x0 + 16 * u;
             if (x < n) {
                 c[u] = slot_ci[src + x];
@@ -1480,7 +1481,7 @@ static __global__ void __launch_bounds__(256)
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const int x = x0 + 16 * u;
             if (x < n) {
                 ci[dst + x] = c[u];
