@@ -70,8 +70,11 @@ __global__ void k_row_starts(CsrView B, uint32_t* __restrict__ bits, int32_t* __
 // when it starts a row or its chunk differs from the entry before. COUNT
 // leaves each tile's number of runs, FILL writes {chunk, position} and, per 32
 // entries, the runs before them and the starts among them (words, for
-// k_row_runs). Columns out of range (a broken operand) flag ERR_STRUCTURE and
-// read as the nearest chunk.
+// k_row_runs). Entries outside every row (before the first row's start, past
+// the last one's end) are never a run. COUNT also sets *irregular where a row
+// is not strictly ascending or leaves B's columns: the lists hold each chunk
+// of a row once, as one range of distinct columns, so such a B takes the
+// lookups instead.
 constexpr int RUNS_TPB = 256;
 constexpr int RUNS_STEPS = 8;
 constexpr int RUNS_TILE = RUNS_TPB * RUNS_STEPS;
@@ -80,35 +83,40 @@ template <int MODE>
 __global__ void __launch_bounds__(RUNS_TPB)
     k_chunk_runs(CsrView B, int cw_log2, const uint32_t* __restrict__ row_bits,
                  int32_t* __restrict__ tile_cnt, const int64_t* __restrict__ tile_off,
-                 int2* __restrict__ runs, int2* __restrict__ words, int32_t* __restrict__ err) {
+                 int2* __restrict__ runs, int2* __restrict__ words,
+                 int32_t* __restrict__ irregular) {
     __shared__ int s_warp[RUNS_TPB / 32];
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * RUNS_TILE + warp * (32 * RUNS_STEPS);
-    const int top = (B.cols - 1) >> cw_log2;
-    int c[RUNS_STEPS];
+    const int first = max(B.rp[0], 0), end = min(B.rp[B.rows], B.nnz);
+    int c[RUNS_STEPS];  // columns
     unsigned m[RUNS_STEPS];
     int n = 0;
+    bool bad = false;
 #pragma unroll
     for (int s = 0; s < RUNS_STEPS; ++s) {
         const int64_t q = base + 32 * s + lane;
-        c[s] = 0;
-        if (q < B.nnz) {
-            const int col = B.ci[q];
-            if ((unsigned)col >= (unsigned)B.cols) atomicOr(err, ERR_STRUCTURE);
-            c[s] = min(max(col >> cw_log2, 0), top);
+        c[s] = q >= first && q < end ? B.ci[q] : 0;
+        if ((unsigned)c[s] >= (unsigned)B.cols) {
+            bad = true;
+            c[s] = 0;
         }
     }
-    const int edge = base > 0 && base <= B.nnz ? min(max(B.ci[base - 1] >> cw_log2, 0), top) : 0;
+    const int edge = base > first && base <= end ? B.ci[base - 1] : 0;
 #pragma unroll
     for (int s = 0; s < RUNS_STEPS; ++s) {
         const int64_t q = base + 32 * s + lane;
         int prev = __shfl_up_sync(FULL, c[s], 1);
         const int carry = s > 0 ? __shfl_sync(FULL, c[s > 0 ? s - 1 : 0], 31) : edge;
         if (lane == 0) prev = carry;
-        const bool start = q < B.nnz && ((row_bits[q >> 5] >> lane & 1u) || c[s] != prev);
+        const bool in = q >= first && q < end;
+        const bool row = in && (row_bits[q >> 5] >> lane & 1u);
+        const bool start = row || (in && (c[s] ^ prev) >> cw_log2 != 0);
+        bad |= in && !row && c[s] <= prev;
         m[s] = __ballot_sync(FULL, start);
         n += __popc(m[s]);
     }
+    if (MODE == COUNT && bad) atomicOr(irregular, 1);
     if (lane == 0) s_warp[warp] = n;
     __syncthreads();
     if (MODE == COUNT) {
@@ -127,7 +135,7 @@ __global__ void __launch_bounds__(RUNS_TPB)
         if (lane == 0 && q <= B.nnz) words[q >> 5] = make_int2(out, (int)m[s]);
         if (m[s] >> lane & 1u) {
             const int at = out + __popc(m[s] & ((1u << lane) - 1));
-            if (at < B.nnz) runs[at] = make_int2(c[s], (int)q);
+            if (at < B.nnz) runs[at] = make_int2(c[s] >> cw_log2, (int)q);
         }
         out += __popc(m[s]);
     }
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(ALIST_WARPS * 32)
                   const int32_t* __restrict__ chunk_lo, const int32_t* __restrict__ nchunks,
                   const int4* __restrict__ brow, const int2* __restrict__ runs, int cw_log2,
                   int32_t* __restrict__ cell_cnt, int32_t* __restrict__ cell_prod,
-                  int32_t* __restrict__ err, int stride) {
+                  int32_t* __restrict__ err, int32_t* __restrict__ irregular, int stride) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = lane_id();
     ListUnit L;
@@ -270,7 +278,7 @@ __global__ void __launch_bounds__(ALIST_WARPS * 32)
                     if ((unsigned)c < (unsigned)L.nch)
                         cur[c] += (1u << 24) + (uint32_t)min(max(t - s.y, 1), 1 << cw_log2);
                     else
-                        atomicOr(err, ERR_STRUCTURE);  // B row not sorted
+                        atomicOr(irregular, 1);  // B row not sorted
                 }
                 __syncwarp();
             }
@@ -336,17 +344,14 @@ __global__ void __launch_bounds__(ALIST_WARPS * 32)
                                               (uint32_t)(n - 1)));
                 ++at[b];
                 cur[b] = nxt[b];
-                if (at[b] + 1 < stop[b]) {
-                    nxt[b] = runs[at[b] + 1];
-                    // a list that would skip a run: B row not sorted
-                    if (nxt[b].x <= cur[b].x) atomicOr(err, ERR_STRUCTURE);
-                } else {
-                    nxt[b] = make_int2(INT_MAX, rend[b]);
-                }
+                nxt[b] = at[b] + 1 < stop[b] ? runs[at[b] + 1] : make_int2(INT_MAX, rend[b]);
             }
             o += __popc(m);
         }
     }
+#pragma unroll
+    for (int b = 0; b < NB; ++b)  // a run left over: an operand changed meanwhile
+        if (at[b] < stop[b]) atomicOr(err, ERR_STRUCTURE);
 }
 
 // The heavy rows' items, in list order, a warp per row; where each one's list
@@ -554,7 +559,9 @@ __device__ __forceinline__ void list_products(const CsrView& B, int2 sg, int len
 }
 
 // Segment i of a list (none past s1): its B position in sg.x, entries and A
-// value.
+// value. One that does not lie in the operands (an operand changed while its
+// lists were built) is flagged and stands in as B's first entry: the walks
+// take a list's segments to be its lanes' prefix, none of them empty.
 template <int MODE>
 __device__ __forceinline__ void list_segment(const CsrView& A, const CsrView& B,
                                              const HeavyLists& L, int64_t i, int64_t s1, int a0,
@@ -567,10 +574,10 @@ __device__ __forceinline__ void list_segment(const CsrView& A, const CsrView& B,
         *sg = L.seg[i];
         *len = (sg->y & ((1 << cw_log2) - 1)) + 1;
         const int64_t j = (int64_t)a0 + (int64_t)((uint32_t)sg->y >> cw_log2);
-        // (a broken operand can leave a list incomplete)
         if (sg->x < 0 || (int64_t)sg->x + *len > B.nnz || j >= A.nnz) {
             atomicOr(err, ERR_STRUCTURE);
-            *len = 0;
+            sg->x = 0;
+            *len = 1;
         } else if (MODE != COUNT) {
             *av = A.v[j];
         }

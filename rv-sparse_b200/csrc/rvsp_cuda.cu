@@ -690,10 +690,11 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
 }
 
 // The heavy rows' work items, and their segment lists (heavy_lists.cuh) unless
-// B has too many chunks for a unit's counters, an A row has too many entries
-// for a segment's word, or the lists would pass LIST_MAX_SEGS segments (8
-// bytes each) or not fit: lists_ok says whether they exist. One device->host
-// read of their size.
+// B has too many chunks for a unit's counters or is not canonical (rows not
+// strictly ascending: the lookups treat them as they always did), an A row has
+// too many entries for a segment's word, or the lists would pass LIST_MAX_SEGS
+// segments (8 bytes each) or not fit: lists_ok says whether they exist. One
+// device->host read of their size and of B's order.
 constexpr int64_t LIST_MAX_SEGS = int64_t(1) << 30;
 constexpr int64_t LIST_MAX_CELLS = int64_t(1) << 28;
 int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
@@ -759,7 +760,7 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
                                                           &misc->err);
             k_chunk_runs<COUNT><<<(unsigned)tiles, RUNS_TPB, 0, plan->stream>>>(
                 B, cl, plan->brow_bits.as<uint32_t>(), plan->brun_cnt.as<int32_t>(), nullptr,
-                nullptr, nullptr, &misc->err);
+                nullptr, nullptr, &misc->irregular);
             note_launch(plan, 2);
         }
         if ((st = scan_counts(plan, plan->brun_cnt.as<int32_t>(), tiles,
@@ -769,7 +770,7 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
             KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
             k_chunk_runs<FILL><<<(unsigned)tiles, RUNS_TPB, 0, plan->stream>>>(
                 B, cl, plan->brow_bits.as<uint32_t>(), nullptr, plan->brun_off.as<int64_t>(),
-                plan->bruns.as<int2>(), plan->brun_words.as<int2>(), &misc->err);
+                plan->bruns.as<int2>(), plan->brun_words.as<int2>(), nullptr);
             k_row_runs<<<kgrid, 256, 0, plan->stream>>>(B, plan->brun_words.as<int2>(),
                                                         plan->brows.as<int4>(), &misc->err);
             note_launch(plan, 2);
@@ -782,7 +783,7 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
                 plan->hcell0.as<int64_t>(), cells, plan->chunk_lo.as<int32_t>(),
                 plan->nchunks.as<int32_t>(), plan->brows.as<int4>(), plan->bruns.as<int2>(), cl,
                 plan->cell_cnt.as<int32_t>(), plan->cell_prod.as<int32_t>(), &misc->err,
-                (int)chunks);
+                &misc->irregular, (int)chunks);
             note_launch(plan, 1);
         }
         if ((st = scan_counts(plan, plan->cell_cnt.as<int32_t>(), cells,
@@ -790,14 +791,14 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
             return st;
         struct {
             int64_t total;
-            int32_t longest;
-        } got = {0, 0};
-        if ((e = cudaMemcpyAsync(&got, &misc->dir_total, 12, cudaMemcpyDeviceToHost,
+            int32_t longest, irregular;
+        } got = {0, 0, 0};
+        if ((e = cudaMemcpyAsync(&got, &misc->dir_total, sizeof(got), cudaMemcpyDeviceToHost,
                                  plan->stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(plan->stream)) != cudaSuccess)
             return fail(e, "segment lists");
         total = got.total;
-        lists = total <= LIST_MAX_SEGS && got.longest <= INT32_MAX >> cl &&
+        lists = !got.irregular && total <= LIST_MAX_SEGS && got.longest <= INT32_MAX >> cl &&
                 plan->seg.ensure((size_t)total * 8) == cudaSuccess;
         cudaGetLastError();
     }

@@ -50,7 +50,7 @@ struct Misc {
     int64_t ltile_total;
     int64_t dir_total;         // heavy-row B directory entries, or listed segments
     int32_t longest;           // entries of the longest heavy row of A
-    int32_t pad3;
+    int32_t irregular;         // a B row is not strictly ascending within B's columns
     int64_t nwork;             // heavy rows: entries of the work list
     int32_t heavy_queue;       // next heavy work item of the running launch
     int32_t row_queue;         // next row of the running warp-bin launch
