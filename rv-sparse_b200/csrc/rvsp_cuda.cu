@@ -957,12 +957,13 @@ int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     return st ? st : count_read(plan);
 }
 
-// The count kernels and scans, enqueued only (with slot_ci, tiny and sorted
-// rows are filled into their slots instead, plan->slot_off, which counts
-// them): C's row pointer lands in c_rp, or plan->c_rp when it is null, the heavy chunks' offsets in plan->item_scan, nnz(C) in
-// Misc::scan_total.
+// The count kernels and scans, enqueued only (with slot_ci, the rows of bins
+// slot_first up to the sorted ones are filled into their slots instead,
+// plan->slot_off, which counts them): C's row pointer lands in c_rp, or
+// plan->c_rp when it is null, the heavy chunks' offsets in plan->item_scan,
+// nnz(C) in Misc::scan_total.
 int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32_t* c_rp,
-                 int32_t* slot_ci, float* slot_v) {
+                 int32_t* slot_ci, float* slot_v, int slot_first) {
     cudaError_t e;
     const int64_t M = plan->a_rows;
     Misc* misc = plan->misc.as<Misc>();  // (the analysis zeroed cnt)
@@ -970,9 +971,13 @@ int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int32
     if (slot_ci) {
         RowOut f{plan->cnt.as<int32_t>(), nullptr, slot_ci, slot_v, &misc->err, false};
         f.ctl.slot_off = plan->slot_off.as<int64_t>();
+        f.bin_first = slot_first;
         f.bin_end = BIN_WARP0;
         run_rows(plan, FILL, A, B, f);
+        o.bin_end = slot_first;
+        run_rows(plan, COUNT, A, B, o);
         o.bin_first = BIN_WARP0;
+        o.bin_end = NUM_BINS;
     }
     run_rows(plan, COUNT, A, B, o);
     int st = scan_counts(plan, plan->cnt.as<int32_t>(), M, nullptr,
@@ -1451,12 +1456,22 @@ constexpr int64_t ONESHOT_FUSED_PRODUCTS = int64_t(1) << 25;
 // counted, into slots of their upper bound (8 bytes a product), and copied
 // into C once the row pointer is known: the copy moves 16 bytes an entry,
 // where counting first means sorting every product twice (tall-skinny 2M x
-// 100k: counts 2.1 ms, copy 0.9 ms, call 8.0 -> 6.7 ms). Below
-// SLOT_MIN_PRODUCTS the scan of the slots and the copy cost what the counts do
-// (4096^2 x 16, 2^20 products: 113 us against 105); above SLOT_MAX_PRODUCTS (4
-// GiB of slots) the rows are counted.
+// 100k: counts 2.1 ms, copy 0.9 ms, call 8.0 -> 6.7 ms). Where most rows are
+// tiny, those are counted: rows next to each other then leave for C as one
+// range, which slots give up (5-point stencils of 2048^2 and 500^2 points: 1.37
+// and 0.194 ms a call by slots, 0.90 and 0.155 counted; the 28 % of tiny rows
+// between others of the tall-skinny product: 6.64 ms by slots, 6.70 counted).
+// Below SLOT_MIN_PRODUCTS the scan of the slots and the copy cost what the
+// counts do (4096^2 x 16, 2^20 products: 113 us against 105); above
+// SLOT_MAX_PRODUCTS (4 GiB of slots) the rows are counted.
 constexpr int64_t SLOT_MIN_PRODUCTS = int64_t(1) << 22;
 constexpr int64_t SLOT_MAX_PRODUCTS = int64_t(1) << 29;
+
+static __global__ void k_no_tiny_slots(int32_t rows, const uint8_t* __restrict__ bin,
+                                       int32_t* __restrict__ slot_len) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < rows && bin[r] == BIN_TINY) slot_len[r] = 0;
+}
 
 // Rows from their slots into C, 16 lanes a row and eight entries a lane in
 // flight (that product: 0.92 ms, 1.11 with four); rows without a slot are left.
@@ -1515,7 +1530,8 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     const int64_t M = a_rows;
     Misc* misc = plan->misc.as<Misc>();
     int64_t slot_products = 0;
-    for (int b = BIN_TINY; b < BIN_WARP0; ++b) slot_products += plan->host_misc.bin_prod[b];
+    const int slot_first = 2 * (int64_t)plan->bin_count[BIN_TINY] > M ? BIN_SORT0 : BIN_TINY;
+    for (int b = slot_first; b < BIN_WARP0; ++b) slot_products += plan->host_misc.bin_prod[b];
     int32_t *rp = nullptr, *ci = nullptr, *slot_ci = nullptr;
     float *v = nullptr, *slot_v = nullptr;
     const auto release_slots = [&] {
@@ -1541,6 +1557,12 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         slots = false;
     }
     if (slots) {
+        if (slot_first > BIN_TINY && plan->bin_count[BIN_TINY] > 0) {
+            KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
+            k_no_tiny_slots<<<(unsigned)((M + 255) / 256), 256, 0, plan->stream>>>(
+                a_rows, plan->bin.as<uint8_t>(), plan->slot_len.as<int32_t>());
+            note_launch(plan, 1);
+        }
         if ((st = scan_counts(plan, plan->slot_len.as<int32_t>(), M, plan->slot_off.as<int64_t>(),
                               nullptr, &misc->scan_total2))) {
             release();
@@ -1555,7 +1577,7 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         release();
         return fail(e, "one-shot product");
     }
-    if ((st = count_launch(plan, A, B, rp, slots ? slot_ci : nullptr, slot_v)) ||
+    if ((st = count_launch(plan, A, B, rp, slots ? slot_ci : nullptr, slot_v, slot_first)) ||
         (!fused && (st = count_read(plan)))) {
         release();
         return st;
@@ -1567,7 +1589,10 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     if (e == cudaSuccess) {
         RowOut o{nullptr, rp, ci, v, &misc->err, false};
         if (slots) {
+            o.bin_end = slot_first;
+            run_rows(plan, FILL, A, B, o);
             o.bin_first = BIN_WARP0;
+            o.bin_end = NUM_BINS;
             KTime kt(plan->stream, plan->capturing, KF_COMPACT);
             k_slots_to_c<<<(unsigned)((M * 16 + 255) / 256), 256, 0, plan->stream>>>(
                 a_rows, plan->slot_off.as<int64_t>(), slot_ci, slot_v, rp, ci, v);

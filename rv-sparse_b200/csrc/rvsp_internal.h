@@ -233,7 +233,8 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
             int (*pre_sync)(rvsp_cuda_plan*) = nullptr, bool slots = false);
 int count_exact(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 int count_launch(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B,
-                 int32_t* c_rp = nullptr, int32_t* slot_ci = nullptr, float* slot_v = nullptr);
+                 int32_t* c_rp = nullptr, int32_t* slot_ci = nullptr, float* slot_v = nullptr,
+                 int slot_first = BIN_TINY);
 int count_read(rvsp_cuda_plan* plan);
 // One-shot exact product of device-resident operands into new device arrays
 // (rvsp_cuda_spgemm_f32's exact path when every operand array is on the
