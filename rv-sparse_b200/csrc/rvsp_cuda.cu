@@ -620,7 +620,10 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     ENS(plan->tile_hist, NUM_BINS * tiles * 4);
     ENS(plan->tile_off, (NUM_BINS * tiles + 1) * 4);
     if (features) ENS(plan->feat, M * 16);
-    if (slots) ENS(plan->slot_len, M * 4);
+    if (slots && plan->slot_len.ensure((size_t)M * 4) != cudaSuccess) {
+        cudaGetLastError();  // no slots then
+        slots = false;
+    }
     Misc* misc = plan->misc.as<Misc>();
     if ((e = cudaMemsetAsync(misc, 0, sizeof(Misc), plan->stream)) != cudaSuccess)
         return fail(e, "memset");
@@ -1546,7 +1549,8 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         if (ci) cudaFreeAsync(ci, plan->stream);
         if (v) cudaFreeAsync(v, plan->stream);
     };
-    bool slots = slot_products >= SLOT_MIN_PRODUCTS && slot_products <= SLOT_MAX_PRODUCTS;
+    bool slots = slot_products >= SLOT_MIN_PRODUCTS && slot_products <= SLOT_MAX_PRODUCTS &&
+                 plan->slot_len.p;
     if (slots && (plan->slot_off.ensure(((size_t)M + 1) * 8) != cudaSuccess ||
                   cudaMallocAsync((void**)&slot_ci, 4 * (size_t)slot_products, plan->stream) !=
                       cudaSuccess ||
@@ -1573,6 +1577,13 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
     int64_t cap = plan->products;
     // (the scan writes C's own row pointer, which the fill then reads)
     cudaError_t e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
+    if (e != cudaSuccess && slots) {
+        cudaGetLastError();
+        release_slots();
+        slots = false;
+        release_pool_memory(plan->stream);
+        e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
+    }
     if (e != cudaSuccess) {
         release();
         return fail(e, "one-shot product");
@@ -1583,9 +1594,32 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         return st;
     }
     if (!fused) cap = plan->c_nnz;
-    const size_t alloc = cap > 0 ? (size_t)cap : 1;
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&ci, alloc * 4, plan->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, alloc * 4, plan->stream);
+    const auto alloc_c = [&] {
+        const size_t bytes = 4 * (size_t)(cap > 0 ? cap : 1);
+        e = cudaMallocAsync((void**)&ci, bytes, plan->stream);
+        if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, bytes, plan->stream);
+        if (e != cudaSuccess) {
+            if (ci) cudaFreeAsync(ci, plan->stream);
+            ci = nullptr;
+            v = nullptr;
+            cudaGetLastError();
+        }
+        return e == cudaSuccess;
+    };
+    if (!alloc_c() && slots) {
+        // C beside the slots is too much: their memory goes back, and the
+        // rows are counted after all
+        release_slots();
+        slots = false;
+        release_pool_memory(plan->stream);
+        if ((e = cudaMemsetAsync(plan->cnt.p, 0, (size_t)M * 4, plan->stream)) != cudaSuccess)
+            st = fail(e, "memset");
+        if (st || (st = count_launch(plan, A, B, rp))) {
+            release();
+            return st;
+        }
+        alloc_c();
+    }
     if (e == cudaSuccess) {
         RowOut o{nullptr, rp, ci, v, &misc->err, false};
         if (slots) {

@@ -137,6 +137,7 @@ struct KTime {
 void init_kernel_attributes();
 BinParams default_params();  // the process-wide default of new and internal plans
 void keep_pool_memory();     // the device pool keeps freed blocks (one-shot entry points)
+void release_pool_memory(cudaStream_t s);  // ... and here gives the unused ones back
 
 }  // namespace rvsp
 

@@ -56,6 +56,17 @@ void keep_pool_memory() {
         cudaGetLastError();
     });
 }
+
+// Waits for `s` and returns what the pool keeps unused to the device, for an
+// allocation that its pieces did not fit.
+void release_pool_memory(cudaStream_t s) {
+    int dev = 0;
+    cudaMemPool_t pool;
+    if (cudaStreamSynchronize(s) == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+        cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
+}
 }  // namespace rvsp
 
 namespace {
