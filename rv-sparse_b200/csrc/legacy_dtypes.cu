@@ -297,9 +297,9 @@ struct Scratch {
         *out = static_cast<T*>(q);
         return e;
     }
-    void release() {
-        for (int i = 0; i < n; ++i) cudaFreeAsync(p[i], st);
-        n = 0;
+    void release(int from = 0) {
+        for (int i = from; i < n; ++i) cudaFreeAsync(p[i], st);
+        n = from;
     }
 };
 
@@ -383,62 +383,84 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
     int32_t *s_rp = nullptr, *s_ci = nullptr, *cnt, *o_rp;
     Out* s_v = nullptr;
     const unsigned wgrid = (unsigned)(((int64_t)a_rows * 32 + 255) / 256);
-    const bool slots = typed_rows_sort(plan) && plan->products <= TYPED_SLOT_PRODUCTS;
-    if (slots) {
-        const size_t pn = (size_t)(plan->products > 0 ? plan->products : 1);
-        if ((e = sc.get(&s_ci, 4 * pn)) || (e = sc.get(&s_v, sizeof(Out) * pn)) ||
-            (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
-            return bail(fail(e, "typed scratch"));
-        if ((st = run_rows_typed(plan, sizeof(In) == 8, A, B, d_av, d_bv, s_ci, s_v)))
-            return bail(st);
-        cnt = plan->cnt.as<int32_t>();
-    } else {
-        // structure: exact analysis and count, then a fill on zero-valued operands
-        if ((st = count_exact(plan, A, B))) return bail(st);
-        plan->analysed = true;
-        const int64_t nnz = plan->c_nnz;
-        float* zeros;
-        float* s_fv;
-        const size_t zn = (size_t)std::max(a_nnz, b_nnz) + 1, cn = (size_t)(nnz > 0 ? nnz : 1);
-        if ((e = sc.get(&zeros, 4 * zn)) || (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) ||
-            (e = sc.get(&s_ci, 4 * cn)) || (e = sc.get(&s_fv, 4 * cn)) ||
-            (e = sc.get(&s_v, sizeof(Out) * cn)) || (e = sc.get(&cnt, 4 * (size_t)a_rows)) ||
-            (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
-            return bail(fail(e, "typed scratch"));
-        cudaMemsetAsync(zeros, 0, 4 * zn, s);
-        if ((st = rvsp_cuda_numeric(plan, d_arp, d_aci, zeros, d_brp, d_bci, zeros, s_rp, s_ci,
-                                    s_fv, 1, nullptr)))
-            return bail(st);
-        // typed values on that structure
-        const int grid = (int)std::min<int64_t>(((int64_t)a_rows + TYPED_WARPS - 1) / TYPED_WARPS,
-                                                148 * 16);
-        k_typed_numeric<Ops><<<grid, TYPED_WARPS * 32, 0, s>>>(A, B, d_av, d_bv, s_rp, s_ci, s_v,
-                                                              &misc->err);
-        k_nonzero_count<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_v, cnt);
-        note_launch(plan, 2);
+    bool slots = typed_rows_sort(plan) && plan->products <= TYPED_SLOT_PRODUCTS;
+    // The slots hold every product: where they do not fit, alone or beside C,
+    // their memory goes back and the general way is taken, whose scratch grows
+    // with nnz(C).
+    const int operands = sc.n;
+    const auto give_up_slots = [&] {
+        cudaGetLastError();
+        if (!slots) return false;
+        sc.release(operands);
+        release_pool_memory(s);
+        slots = false;
+        return cudaMemsetAsync(plan->cnt.p, 0, 4 * (size_t)a_rows, s) == cudaSuccess;
+    };
+    int64_t total;
+    int32_t *rp, *ci;  // outputs where the inputs live
+    Out* v;
+    for (;;) {
+        if (slots) {
+            const size_t pn = (size_t)(plan->products > 0 ? plan->products : 1);
+            e = sc.get(&s_ci, 4 * pn);
+            if (e == cudaSuccess) e = sc.get(&s_v, sizeof(Out) * pn);
+            if (e == cudaSuccess) e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1));
+            st = e == cudaSuccess
+                     ? run_rows_typed(plan, sizeof(In) == 8, A, B, d_av, d_bv, s_ci, s_v)
+                     : fail(e, "typed scratch");
+            if (st == RVSP_ERROR_ALLOCATION_FAILED && give_up_slots()) continue;
+            if (st) return bail(st);
+            cnt = plan->cnt.as<int32_t>();
+        } else {
+            // structure: exact analysis and count, then a fill on zero-valued operands
+            if ((st = count_exact(plan, A, B))) return bail(st);
+            plan->analysed = true;
+            const int64_t nnz = plan->c_nnz;
+            float* zeros;
+            float* s_fv;
+            const size_t zn = (size_t)std::max(a_nnz, b_nnz) + 1, cn = (size_t)(nnz > 0 ? nnz : 1);
+            if ((e = sc.get(&zeros, 4 * zn)) || (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) ||
+                (e = sc.get(&s_ci, 4 * cn)) || (e = sc.get(&s_fv, 4 * cn)) ||
+                (e = sc.get(&s_v, sizeof(Out) * cn)) || (e = sc.get(&cnt, 4 * (size_t)a_rows)) ||
+                (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
+                return bail(fail(e, "typed scratch"));
+            cudaMemsetAsync(zeros, 0, 4 * zn, s);
+            if ((st = rvsp_cuda_numeric(plan, d_arp, d_aci, zeros, d_brp, d_bci, zeros, s_rp, s_ci,
+                                        s_fv, 1, nullptr)))
+                return bail(st);
+            // typed values on that structure
+            const int grid = (int)std::min<int64_t>(((int64_t)a_rows + TYPED_WARPS - 1) / TYPED_WARPS,
+                                                    148 * 16);
+            k_typed_numeric<Ops><<<grid, TYPED_WARPS * 32, 0, s>>>(A, B, d_av, d_bv, s_rp, s_ci, s_v,
+                                                                  &misc->err);
+            k_nonzero_count<Out><<<wgrid, 256, 0, s>>>(a_rows, s_rp, s_v, cnt);
+            note_launch(plan, 2);
+        }
+        if ((st = scan_counts(plan, cnt, a_rows, nullptr, o_rp, &misc->scan_total))) return bail(st);
+        total = 0;
+        int32_t err = 0;
+        if ((e = cudaMemcpyAsync(&total, &misc->scan_total, 8, cudaMemcpyDeviceToHost, s)) ||
+            (e = cudaMemcpyAsync(&err, &misc->err, 4, cudaMemcpyDeviceToHost, s)) ||
+            (e = cudaStreamSynchronize(s)))
+            return bail(fail(e, "typed numeric"));
+        if (err) {
+            g_err = "operand structure out of range (row_ptr or col_idx)";
+            return bail(RVSP_ERROR_INVALID_CSR);
+        }
+        rp = ci = nullptr;
+        v = nullptr;
+        const size_t on = (size_t)(total > 0 ? total : 1);
+        if ((e = cudaMallocAsync((void**)&rp, 4 * ((size_t)a_rows + 1), s)) ||
+            (e = cudaMallocAsync((void**)&ci, 4 * on, s)) ||
+            (e = cudaMallocAsync((void**)&v, sizeof(Out) * on, s))) {
+            if (rp) cudaFreeAsync(rp, s);
+            if (ci) cudaFreeAsync(ci, s);
+            if (give_up_slots()) continue;
+            return bail(fail(e, "C alloc"));
+        }
+        break;
     }
-    if ((st = scan_counts(plan, cnt, a_rows, nullptr, o_rp, &misc->scan_total))) return bail(st);
-    int64_t total = 0;
-    int32_t err = 0;
-    if ((e = cudaMemcpyAsync(&total, &misc->scan_total, 8, cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaMemcpyAsync(&err, &misc->err, 4, cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaStreamSynchronize(s)))
-        return bail(fail(e, "typed numeric"));
-    if (err) {
-        g_err = "operand structure out of range (row_ptr or col_idx)";
-        return bail(RVSP_ERROR_INVALID_CSR);
-    }
-    // outputs where the inputs live
-    int32_t *rp = nullptr, *ci = nullptr;
-    Out* v = nullptr;
     const size_t on = (size_t)(total > 0 ? total : 1);
-    if ((e = cudaMallocAsync((void**)&rp, 4 * ((size_t)a_rows + 1), s)) ||
-        (e = cudaMallocAsync((void**)&ci, 4 * on, s)) ||
-        (e = cudaMallocAsync((void**)&v, sizeof(Out) * on, s))) {
-        if (rp) cudaFreeAsync(rp, s);
-        if (ci) cudaFreeAsync(ci, s);
-        return bail(fail(e, "C alloc"));
-    }
     cudaMemcpyAsync(rp, o_rp, 4 * ((size_t)a_rows + 1), cudaMemcpyDeviceToDevice, s);
     if (slots)
         k_slots_to_rows<Out><<<(unsigned)(((int64_t)a_rows * 16 + 255) / 256), 256, 0, s>>>(

@@ -70,6 +70,9 @@ def _child(case, mb):
     fn, algo = "f32", rv.RVSP_CUDA_ALGO_EXACT
     if case == "oneshot":  # 410 MB of slots, 410 of C
         A, B = _strata(200000, 16, 65536, g), _strata(65536, 16, 65536, g)
+    if case == "f64":  # 1230 MB of slots, 440 of C
+        fn = "f64"
+        A, B = _strata(200000, 32, 65536, g), _strata(65536, 16, 192, g)
     small = _strata(512, 4, 512, g)
     if fn == "f64":
         A, B, small = ((*M[:4], M[4].double()) for M in (A, B, small))
@@ -87,7 +90,7 @@ def _child(case, mb):
     print("same", got[1].numel())
 
 
-@pytest.mark.parametrize("case,mb", [("oneshot", 640)])
+@pytest.mark.parametrize("case,mb", [("oneshot", 640), ("f64", 1200), ("f64", 1450)])
 def test_little_memory(gpu_lib, case, mb):
     import torch as T
 
