@@ -35,7 +35,11 @@ namespace rvsp {
 
 constexpr int LIST_MAX_CHUNKS = 2048;  // chunks of B: a unit's counters stay in shared memory
 constexpr int ALIST_WARPS = 4;
-constexpr int LIST_MAX_WARPS = 28;  // a CTA of k_heavy_list (72 registers a thread)
+// Warps of a CTA of k_heavy_list: FILL and REUSE 28 (72 registers a thread, one
+// CTA an SM), COUNT 24 (40 registers, two; R-MAT 2^17 and tall-skinny 2M x
+// 100k, calls: 10.46 and 6.65 ms at 32 registers with spills, 10.15 and 6.66
+// so, 10.27 and 6.72 at 56).
+constexpr int list_max_warps(int mode) { return mode == COUNT ? 24 : 28; }
 constexpr int COUNT_GROUP_SEGS = 256;  // segments of the chunks one warp counts together
 constexpr int LIST_LONG = 64;          // segments this long are walked on their own
 
@@ -327,6 +331,7 @@ __global__ void __launch_bounds__(ALIST_WARPS * 32)
         rend[b] = br.z;
         cur[b] = at[b] < stop[b] ? runs[at[b]] : make_int2(INT_MAX, br.z);
         nxt[b] = at[b] + 1 < stop[b] ? runs[at[b] + 1] : make_int2(INT_MAX, br.z);
+        if (at[b] < stop[b] && nxt[b].x <= cur[b].x) atomicOr(err, ERR_STRUCTURE);
     }
     int64_t o = cell_off[L.cell];
     for (int c = 0; c < L.nch; ++c) {
@@ -344,14 +349,17 @@ __global__ void __launch_bounds__(ALIST_WARPS * 32)
                                               (uint32_t)(n - 1)));
                 ++at[b];
                 cur[b] = nxt[b];
-                nxt[b] = at[b] + 1 < stop[b] ? runs[at[b] + 1] : make_int2(INT_MAX, rend[b]);
+                if (at[b] + 1 < stop[b]) {
+                    nxt[b] = runs[at[b] + 1];
+                    // a list that would skip a run: an operand changed meanwhile
+                    if (nxt[b].x <= cur[b].x) atomicOr(err, ERR_STRUCTURE);
+                } else {
+                    nxt[b] = make_int2(INT_MAX, rend[b]);
+                }
             }
             o += __popc(m);
         }
     }
-#pragma unroll
-    for (int b = 0; b < NB; ++b)  // a run left over: an operand changed meanwhile
-        if (at[b] < stop[b]) atomicOr(err, ERR_STRUCTURE);
 }
 
 // The heavy rows' items, in list order, a warp per row; where each one's list
@@ -820,13 +828,50 @@ __device__ __forceinline__ void sparse_stretch(
     __syncwarp();
 }
 
+// Entries drawn as draw_batched does, except at the list's end: a single index
+// past it (`limit`) does not end the warp, since the batch in flight may be the
+// CTA's last and would be left to the one warp that fetched it (16,000 items on
+// 592 CTAs of 16 warps, count: 6.3 ms, most of it with one warp a CTA at work,
+// against 1.0). The warp waits until the fetch, 1 us of its CTA's own warp, is
+// there; were it not after DRAW_POLLS the warp would leave, and the fetching
+// warp take the batch alone. Called by lane 0; returns the entry drawn, limit
+// or more at the end. What a draw past its batch does (draw_past; -1: draw
+// again) is kept out of the kernel's code: inlined it cost the loops 1 %.
+constexpr int DRAW_POLLS = 1 << 12;
+__device__ __noinline__ long long draw_past(unsigned long long* s_q, int32_t* queue, long long batch,
+                                            long long limit, long long c) {
+    if (c == batch) {
+        const int nb = atomicAdd(queue, (int)batch);
+        atomicExch(s_q, ((unsigned long long)(unsigned)nb << 32) | 1ull);
+        return nb;
+    }
+    const long long single = atomicAdd(queue, 1);
+    if (single < limit) return single;
+    for (int polls = 0; polls < DRAW_POLLS; ++polls) {
+        const unsigned long long v = *(volatile unsigned long long*)s_q;
+        if ((long long)(v & 0xffffffffull) <= batch) return (long long)(v >> 32) < limit ? -1 : limit;
+        __nanosleep(64);
+    }
+    return limit;
+}
+__device__ __forceinline__ long long draw_entry(unsigned long long* s_q, int32_t* queue,
+                                                long long batch, long long limit) {
+    long long w;
+    do {
+        const unsigned long long o = atomicAdd(s_q, 1ull);
+        const long long c = (long long)(o & 0xffffffffull);
+        w = c < batch ? (long long)(o >> 32) + c : draw_past(s_q, queue, batch, limit, c);
+    } while (w < 0);
+    return w;
+}
+
 // Heavy rows, items drawn in CTA batches by a grid that fills the GPU once, as
 // in k_heavy. COUNT: one warp per item, or per group of neighbouring items with
 // few segments. FILL and REUSE: the work list's entries; a warp takes its
 // chunks in stretches of at most SPARSE_PRODUCTS products (sparse_stretch), a
 // chunk beyond that through the dense accumulator.
 template <int MODE>
-__global__ void __launch_bounds__(LIST_MAX_WARPS * 32)
+__global__ void __launch_bounds__(list_max_warps(MODE) * 32, MODE == COUNT ? 2 : 0)
     k_heavy_list(CsrView A, CsrView B, const HeavyItem* __restrict__ items, int nitems,
                  HeavyLists L, int32_t* __restrict__ item_cnt, int32_t* __restrict__ row_cnt,
                  const int64_t* __restrict__ item_scan, const int32_t* __restrict__ c_rp,
@@ -843,15 +888,16 @@ __global__ void __launch_bounds__(LIST_MAX_WARPS * 32)
     for (int x = lane; x < bytes / 16; x += 32)
         reinterpret_cast<float4*>(mine)[x] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
-    const long long batch = 2 * (long long)(blockDim.x >> 5);
-    unsigned long long* s_q = reinterpret_cast<unsigned long long*>(
-        smem + (blockDim.x >> 5) * bytes);
-    if (threadIdx.x == 0) *s_q = (unsigned long long)batch;
     const int limit = MODE == COUNT ? nitems : (int)min(*L.nwork, (int64_t)nitems);
+    // (a launch of fewer entries than two a warp spreads them over all CTAs)
+    const int warps = blockDim.x >> 5;
+    const long long batch = min(max((limit + (long long)gridDim.x - 1) / gridDim.x, 1ll), 2ll * warps);
+    unsigned long long* s_q = reinterpret_cast<unsigned long long*>(smem + warps * bytes);
+    if (threadIdx.x == 0) *s_q = (unsigned long long)batch;
     __syncthreads();
     for (;;) {
         long long wq = 0;
-        if (lane == 0) wq = draw_batched(s_q, queue, batch);
+        if (lane == 0) wq = draw_entry(s_q, queue, batch, limit);
         wq = __shfl_sync(FULL, wq, 0);
         if (wq >= limit) break;
         const int2 wk = MODE == COUNT ? make_int2((int)wq, 1) : L.work[wq];

@@ -251,7 +251,7 @@ void init_kernel_attributes() {
             for (int m = 0; m < 6; ++m) {
                 int best_w = 1, best_n = 1, best = 0;
                 for (int W = 1; W <= HEAVY_MAX_WARPS; ++W) {
-                    if (m >= 3 && W > LIST_MAX_WARPS) break;
+                    if (m >= 3 && W > list_max_warps(m - 3)) break;
                     const size_t bytes = heavy_launch_smem(m, cl, W);
                     if (bytes > (size_t)HEAVY_SMEM_MAX) break;
                     int n = 0;
