@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -692,14 +693,54 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
     return RVSP_SUCCESS;
 }
 
-// The heavy rows' work items, and their segment lists (heavy_lists.cuh) unless
-// B has too many chunks for a unit's counters or is not canonical (rows not
-// strictly ascending: the lookups treat them as they always did), an A row has
-// too many entries for a segment's word, or the lists would pass LIST_MAX_SEGS
-// segments (8 bytes each) or not fit: lists_ok says whether they exist. One
-// device->host read of their size and of B's order.
 constexpr int64_t LIST_MAX_SEGS = int64_t(1) << 30;
 constexpr int64_t LIST_MAX_CELLS = int64_t(1) << 28;
+constexpr int64_t DIR_MAX_ENTRIES = int64_t(1) << 28;  // chunk directories of B's rows
+constexpr size_t SMASK_MAX_BYTES = 128u << 20;         // their chunk masks
+
+// Whether the segment lists take less time to build and walk than the lookups
+// that they replace, by estimates of the steps in which they differ (ps each,
+// B200). Z, K: entries and rows of B; E, V, H: the heavy rows' A entries,
+// (entry, chunk) pairs and products; hits: the pairs that find something, from
+// the mean visited B row as if its columns were uniform.
+//   lists    launches, 100 us; two sweeps of B's columns, 4.7 Z; counting, 77 E
+//            for 32 chunks of a B row; the fill walks the chunks one after the
+//            other, 0.4 us each, and writes the segments, 12.5 each, 5 where B's
+//            columns stay in L2; the walks gain 5 a product over the lookups'
+//   lookups  a sweep of B's long rows for directories, 4.5 Z, and one for chunk
+//            masks, 2 Z or 180 a row; a binary search per pair, 12.5 a step, 2.5
+//            where B's columns stay in L2, only for the hits with masks, none
+//            with directories, where a miss costs 5; launches of few items leave
+//            most of the GPU idle, 300 us
+// On forty shapes of uniform B (1..50,000 heavy rows of 30..20,000 entries times
+// 64k..16M rows of 4..256) it picks the faster side, of which the farthest apart:
+// one row of 600 entries x 4M rows of 64 in 4M columns, call: 0.77 ms by
+// lookups, 2.35 by lists; 2000 such rows: 245 and 11.6 ms; 50,000 rows of 512 x
+// rows of 4 equal columns: 2.55 and 4.7; 2000 rows of 600 x 1M rows of 64 in 256k
+// columns: 4.3 and 5.5. R-MAT 2^17: estimated 1 ms against 5.6 of gain.
+static bool lists_pay(const rvsp_cuda_plan* plan, int64_t chunks) {
+    const double Z = plan->b_nnz, K = plan->b_rows, E = plan->host_misc.totals[4],
+                 V = plan->host_misc.totals[5], H = plan->host_misc.bin_prod[BIN_HEAVY];
+    if (E <= 0 || V <= 0) return false;
+    const bool masks = chunks > 1 && K * ((chunks + 31) / 32) * 4 <= SMASK_MAX_BYTES;
+    const bool dir = Z >= DIR_MIN_LEN * K && K * (chunks + 1) <= DIR_MAX_ENTRIES;
+    const bool far = 4 * Z > (100 << 20);  // B's columns do not stay in L2
+    const double len = H / E, hits = V * (1.0 - exp(-H / V));
+    const double lists = 100e6 + 4.7 * Z + 77.0 * E * ceil(std::min(len, V / E) / 32.0) +
+                         0.4e6 * chunks + (far ? 12.5 : 5.0) * hits - 5.0 * H;
+    const double search = (far ? 12.5 : 2.5) * log2(std::max(len, 2.0));
+    const double pairs = dir ? 5.0 * (V - hits) : (masks ? hits : V) * search;
+    const double lookups = (masks ? std::max(2.0 * Z, 180.0 * K) : 0.0) + (dir ? 4.5 * Z : 0.0) +
+                           pairs + (plan->n_items < (1 << 15) ? 300e6 : 0.0);
+    return lists <= lookups;
+}
+
+// The heavy rows' work items, and their segment lists (heavy_lists.cuh) where
+// they pay, unless B has too many chunks for a unit's counters or is not
+// canonical (rows not strictly ascending: the lookups treat them as they always
+// did), an A row has too many entries for a segment's word, or the lists would
+// pass LIST_MAX_SEGS segments (8 bytes each) or not fit: lists_ok says whether
+// they exist. One device->host read of their size and of B's order.
 int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     const int nh = plan->bin_count[BIN_HEAVY];
     const int cl = plan->params.heavy_cw_log2;
@@ -722,6 +763,7 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
 #undef ENS
     const size_t bits_bytes = ((size_t)Z / 32 + 1) * 4;
     bool lists = chunks <= LIST_MAX_CHUNKS && units <= INT32_MAX && cells <= LIST_MAX_CELLS &&
+                 lists_pay(plan, chunks) &&
                  plan->brow_bits.ensure(bits_bytes) == cudaSuccess &&
                  plan->brun_cnt.ensure((size_t)tiles * 4) == cudaSuccess &&
                  plan->brun_off.ensure(((size_t)tiles + 1) * 8) == cudaSuccess &&
@@ -869,7 +911,7 @@ int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
                              plan->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(plan->stream)) != cudaSuccess)
         return fail(e, "directory size");
-    plan->dir_ok = total > 0 && total <= (int64_t(1) << 28) &&
+    plan->dir_ok = total > 0 && total <= DIR_MAX_ENTRIES &&
                    plan->bdir.ensure((size_t)total * 4) == cudaSuccess;
     cudaGetLastError();  // a refused directory allocation only costs the searches
     KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
@@ -887,7 +929,6 @@ int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
         const int64_t nchunks = ((int64_t)plan->b_cols + (1 << cl) - 1) >> cl;
         const int64_t words = (nchunks + 31) / 32;
         const size_t mbytes = (size_t)(K * words * 4);
-        constexpr size_t SMASK_MAX_BYTES = 128u << 20;
         plan->smask_words = 0;
         if (K > 0 && nchunks > 1 && mbytes <= SMASK_MAX_BYTES &&
             plan->bsmask.ensure(mbytes) == cudaSuccess &&

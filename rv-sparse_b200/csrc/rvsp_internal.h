@@ -29,7 +29,8 @@ struct DevBuf {
 struct Misc {
     int32_t hist[NUM_BINS];    // rows per bin
     int32_t cursor[NUM_BINS];  // bin scatter cursors
-    int64_t totals[4];         // heavy items, products, heavy units, heavy cells
+    int64_t totals[6];         // heavy items, products, and the heavy rows' units, cells,
+                               // A entries and (entry, chunk) pairs
     int32_t pad0;
     int32_t overflow;          // a 32-bit row pointer would overflow
     int64_t scan_total;        // nnz(C)

@@ -148,7 +148,8 @@ struct AnalyzeOut {
     float4* feat;        // [rows] learned-model features (optional)
     int32_t* hist;       // [NUM_BINS] rows per bin
     int32_t* tile_hist;  // [NUM_BINS][tiles] rows per bin per tile (stable binning)
-    int64_t* totals;     // [0] heavy items, [1] products, [2] heavy units, [3] heavy cells
+    int64_t* totals;     // [0] heavy items, [1] products, and of the heavy rows [2] units,
+                         // [3] cells, [4] A entries, [5] (entry, chunk) pairs
     int64_t* bin_prod;   // [NUM_BINS] products per bin
     int32_t* err;        // ERR_* bits
     int32_t* nnz_ab;     // [2] nnz of A and B as the kernel used them (read back with the bins)
@@ -199,7 +200,7 @@ struct AnTile {
     int32_t maxlen[AN_TILE], minc[AN_TILE], maxc[AN_TILE];
     int32_t hist[NUM_BINS];
     unsigned long long bprod[NUM_BINS];
-    unsigned long long items, prod, units, cells;
+    unsigned long long items, prod, units, cells, entries, pairs;
 };
 
 // Tiles left to k_analyze_big: their number << 44 | their chunks, and for each
@@ -224,6 +225,8 @@ __device__ __forceinline__ void an_clear(AnTile& s, int t) {
         s.prod = 0;
         s.units = 0;
         s.cells = 0;
+        s.entries = 0;
+        s.pairs = 0;
     }
 }
 
@@ -342,13 +345,16 @@ __device__ __forceinline__ void an_finish(const AnalyzeOut& out, const BinParams
     warp_bin_add(b, NUM_BINS, (unsigned long long)ops, s.hist, s.bprod);
     const unsigned long long wprod = warp_sum64((unsigned long long)ops);
     const unsigned long long witems = warp_sum64((unsigned long long)nch);
-    if (__any_sync(FULL, nch > 0)) {  // heavy rows: their units and (chunk, unit) cells
-        const unsigned long long u =
-            nch > 0 ? (unsigned long long)(s.rp[t + 1] - s.rp[t] + HEAVY_UNIT - 1) / HEAVY_UNIT : 0ull;
+    if (__any_sync(FULL, nch > 0)) {  // heavy rows: their units, (chunk, unit) cells, entries
+        const unsigned long long n = nch > 0 ? (unsigned long long)(s.rp[t + 1] - s.rp[t]) : 0ull;
+        const unsigned long long u = (n + HEAVY_UNIT - 1) / HEAVY_UNIT;
         const unsigned long long wu = warp_sum64(u), wc = warp_sum64(u * (unsigned long long)nch);
+        const unsigned long long we = warp_sum64(n), wp = warp_sum64(n * (unsigned long long)nch);
         if (lane_id() == 0) {
             atomicAdd(&s.units, wu);
             atomicAdd(&s.cells, wc);
+            atomicAdd(&s.entries, we);
+            atomicAdd(&s.pairs, wp);
         }
     }
     if (lane_id() == 0) {
@@ -366,6 +372,8 @@ __device__ __forceinline__ void an_finish(const AnalyzeOut& out, const BinParams
             atomicAdd((unsigned long long*)&out.totals[0], s.items);
             atomicAdd((unsigned long long*)&out.totals[2], s.units);
             atomicAdd((unsigned long long*)&out.totals[3], s.cells);
+            atomicAdd((unsigned long long*)&out.totals[4], s.entries);
+            atomicAdd((unsigned long long*)&out.totals[5], s.pairs);
         }
         atomicAdd((unsigned long long*)&out.totals[1], s.prod);
     }
