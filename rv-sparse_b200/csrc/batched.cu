@@ -275,6 +275,7 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
         }
         if (c_off_dev) cudaFreeAsync(c_off_dev, s0);
         cudaStreamSynchronize(s0);
+        for (rvsp_cuda_plan* p : plans) trim_lists(p, LIST_KEEP_BYTES / plans.size());
         return status;
     };
     cudaError_t e0 = plans[0]->misc.ensure(sizeof(Misc));
@@ -339,6 +340,14 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
     std::vector<CsrView> As(groups.size());
     CsrView Bv{pb.rp, pb.ci, pb.v, (int32_t)br, max_n, (int32_t)bz};
     int64_t total = 0;
+    // whether the first n groups' segment lists gave memory back
+    const auto yield = [&](size_t n) {
+        bool any = false;
+        int failed = RVSP_SUCCESS;
+        for (size_t g = 0; g < n && !failed; ++g)
+            any |= yield_lists(plans[g], As[g], Bv, &failed);
+        return any && !failed;
+    };
     for (size_t g = 0; g < groups.size(); ++g) {
         Group& G = groups[g];
         rvsp_cuda_plan* plan = plans[g];
@@ -363,12 +372,13 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
         if (ev) cudaEventDestroy(ev);
         if (e != cudaSuccess) return cleanup(fail(e, "batched streams"));
         As[g] = CsrView{pa.rp + G.row0, pa.ci, pa.v, G.rows, (int32_t)kshift, plan->a_nnz};
-        if (algo == RVSP_CUDA_ALGO_LEARNED) {
-            st = learned_symbolic(plan, As[g], Bv, true);
-        } else {
-            st = analyze(plan, As[g], Bv, false);
-            if (!st) st = count_exact(plan, As[g], Bv);
-        }
+        const auto symbolic = [&] {
+            if (algo == RVSP_CUDA_ALGO_LEARNED) return learned_symbolic(plan, As[g], Bv, true);
+            const int s = analyze(plan, As[g], Bv, false);
+            return s ? s : count_exact(plan, As[g], Bv);
+        };
+        st = symbolic();
+        if (st == RVSP_ERROR_ALLOCATION_FAILED && yield(g)) st = symbolic();
         if (st) return cleanup(st);
         plan->analysed = true;
         G.base = total;
@@ -376,10 +386,17 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
     }
     // one C for every product; every group fills its part
     const int64_t slots = ar + count;
-    cudaError_t e = cudaMallocAsync((void**)&rp, 4 * (size_t)slots, s0);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&ci, 4 * (size_t)std::max<int64_t>(total, 1), s0);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, 4 * (size_t)std::max<int64_t>(total, 1), s0);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&c_off_dev, 8 * ((size_t)count + 1), s0);
+    cudaError_t e = cudaSuccess;
+    const auto alloc_c = [&] {
+        const size_t bytes = 4 * (size_t)std::max<int64_t>(total, 1);
+        e = rp ? cudaSuccess : cudaMallocAsync((void**)&rp, 4 * (size_t)slots, s0);
+        if (e == cudaSuccess && !ci) e = cudaMallocAsync((void**)&ci, bytes, s0);
+        if (e == cudaSuccess && !v) e = cudaMallocAsync((void**)&v, bytes, s0);
+        if (e == cudaSuccess && !c_off_dev)
+            e = cudaMallocAsync((void**)&c_off_dev, 8 * ((size_t)count + 1), s0);
+        return e == cudaSuccess;
+    };
+    if (!alloc_c() && yield(groups.size())) alloc_c();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);  // C exists before other streams write it
     if (e != cudaSuccess) return cleanup(fail(e, "batched C"));
     for (size_t g = 0; g < groups.size(); ++g) {

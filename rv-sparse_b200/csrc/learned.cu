@@ -501,16 +501,26 @@ int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused) {
         (e = cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess)
         return fail(e, "mem info");
     if (fused) {
-        if (free_b != SIZE_MAX && (size_t)tmp_total * 8 > free_b / 2) {
+        const auto over = [&] {
+            return free_b != SIZE_MAX && (size_t)tmp_total * 8 > free_b / 2;
+        };
+        const auto buffers = [&] {
+            if ((e = plan->slot_off.ensure(((size_t)M + 1) * 8)) == cudaSuccess &&
+                (e = plan->tmp_ci.ensure((size_t)tmp_total * 4)) == cudaSuccess)
+                e = plan->tmp_v.ensure((size_t)tmp_total * 4);
+            return e == cudaSuccess;
+        };
+        // (the segment lists must not cost a product its slots)
+        if (over() && yield_lists(plan, A, B, &st) &&
+            (e = cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess)
+            return fail(e, "mem info");
+        if (st) return st;
+        if (over()) {
             g_err = "predicted capacity exceeds the memory budget";
             return RVSP_ERROR_ALLOCATION_FAILED;
         }
-        if ((e = plan->slot_off.ensure(((size_t)M + 1) * 8)) != cudaSuccess)
-            return fail(e, "slots");
-        if ((e = plan->tmp_ci.ensure((size_t)tmp_total * 4)) != cudaSuccess)
-            return fail(e, "slots");
-        if ((e = plan->tmp_v.ensure((size_t)tmp_total * 4)) != cudaSuccess)
-            return fail(e, "slots");
+        if (!buffers() && !(yield_lists(plan, A, B, &st) && buffers()))
+            return st ? st : fail(e, "slots");
     }
     if ((st = launch_bin_scatter(plan, plan->lbin.as<uint8_t>(), misc->lhist,
                                  plan->ltile_hist.as<int32_t>(), plan->ltile_off.as<int32_t>(),
@@ -668,9 +678,17 @@ int learned_spgemm(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, int32_t
     const size_t alloc = nnz > 0 ? (size_t)nnz : 1;
     int32_t *rp = nullptr, *ci = nullptr;
     float* v = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&rp, ((size_t)a_rows + 1) * 4, plan->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&ci, alloc * 4, plan->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, alloc * 4, plan->stream);
+    cudaError_t e = cudaSuccess;
+    const auto alloc_c = [&] {
+        if (!rp) e = cudaMallocAsync((void**)&rp, ((size_t)a_rows + 1) * 4, plan->stream);
+        if (e == cudaSuccess && !ci) e = cudaMallocAsync((void**)&ci, alloc * 4, plan->stream);
+        if (e == cudaSuccess) e = cudaMallocAsync((void**)&v, alloc * 4, plan->stream);
+        return e == cudaSuccess;
+    };
+    if (!alloc_c() && yield_lists(plan, A, B, &st)) {
+        e = cudaSuccess;
+        alloc_c();
+    }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(rp, plan->c_rp.p, ((size_t)a_rows + 1) * 4, cudaMemcpyDeviceToDevice,
                             plan->stream);

@@ -325,6 +325,7 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
         t_tplan->map_policy = 0;
     }
     rvsp_cuda_plan_t plan = t_tplan;
+    const ListTrim trim{plan};
     plan->params = default_params();
     keep_pool_memory();
     cudaStream_t s = plan->stream;
@@ -419,11 +420,20 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
             float* zeros;
             float* s_fv;
             const size_t zn = (size_t)std::max(a_nnz, b_nnz) + 1, cn = (size_t)(nnz > 0 ? nnz : 1);
-            if ((e = sc.get(&zeros, 4 * zn)) || (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) ||
-                (e = sc.get(&s_ci, 4 * cn)) || (e = sc.get(&s_fv, 4 * cn)) ||
-                (e = sc.get(&s_v, sizeof(Out) * cn)) || (e = sc.get(&cnt, 4 * (size_t)a_rows)) ||
-                (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))))
-                return bail(fail(e, "typed scratch"));
+            const auto scratch = [&] {
+                return (e = sc.get(&zeros, 4 * zn)) == cudaSuccess &&
+                       (e = sc.get(&s_rp, 4 * ((size_t)a_rows + 1))) == cudaSuccess &&
+                       (e = sc.get(&s_ci, 4 * cn)) == cudaSuccess &&
+                       (e = sc.get(&s_fv, 4 * cn)) == cudaSuccess &&
+                       (e = sc.get(&s_v, sizeof(Out) * cn)) == cudaSuccess &&
+                       (e = sc.get(&cnt, 4 * (size_t)a_rows)) == cudaSuccess &&
+                       (e = sc.get(&o_rp, 4 * ((size_t)a_rows + 1))) == cudaSuccess;
+            };
+            if (!scratch()) {
+                sc.release(operands);
+                if (!(yield_lists(plan, A, B, &st) && scratch()))
+                    return bail(st ? st : fail(e, "typed scratch"));
+            }
             cudaMemsetAsync(zeros, 0, 4 * zn, s);
             if ((st = rvsp_cuda_numeric(plan, d_arp, d_aci, zeros, d_brp, d_bci, zeros, s_rp, s_ci,
                                         s_fv, 1, nullptr)))
@@ -447,16 +457,22 @@ int typed_spgemm(int32_t a_rows, int32_t a_cols, int32_t b_cols, const int32_t* 
             g_err = "operand structure out of range (row_ptr or col_idx)";
             return bail(RVSP_ERROR_INVALID_CSR);
         }
-        rp = ci = nullptr;
-        v = nullptr;
         const size_t on = (size_t)(total > 0 ? total : 1);
-        if ((e = cudaMallocAsync((void**)&rp, 4 * ((size_t)a_rows + 1), s)) ||
-            (e = cudaMallocAsync((void**)&ci, 4 * on, s)) ||
-            (e = cudaMallocAsync((void**)&v, sizeof(Out) * on, s))) {
+        const auto alloc_c = [&] {
+            rp = ci = nullptr;
+            v = nullptr;
+            if ((e = cudaMallocAsync((void**)&rp, 4 * ((size_t)a_rows + 1), s)) == cudaSuccess &&
+                (e = cudaMallocAsync((void**)&ci, 4 * on, s)) == cudaSuccess &&
+                (e = cudaMallocAsync((void**)&v, sizeof(Out) * on, s)) == cudaSuccess)
+                return true;
             if (rp) cudaFreeAsync(rp, s);
             if (ci) cudaFreeAsync(ci, s);
+            return false;
+        };
+        if (!alloc_c()) {
             if (give_up_slots()) continue;
-            return bail(fail(e, "C alloc"));
+            release_lists(plan);  // (the rows are done)
+            if (!alloc_c()) return bail(fail(e, "C alloc"));
         }
         break;
     }

@@ -606,8 +606,13 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
             int (*pre_sync)(rvsp_cuda_plan*), bool slots) {
     const int64_t M = plan->a_rows;
     cudaError_t e;
-#define ENS(buf, bytes)                                        \
-    if ((e = (buf).ensure(bytes)) != cudaSuccess) return fail(e, "plan alloc " #buf)
+    plan->lists_ok = false;  // (the last product's)
+#define ENS(buf, bytes)                                                       \
+    if ((e = (buf).ensure(bytes)) != cudaSuccess && list_bytes(plan) > 0) {   \
+        release_lists(plan);                                                  \
+        e = (buf).ensure(bytes);                                              \
+    }                                                                         \
+    if (e != cudaSuccess) return fail(e, "plan alloc " #buf)
     ENS(plan->ops, M * 8);
     ENS(plan->ub, M * 4);
     ENS(plan->bin, M);
@@ -695,6 +700,7 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
 
 constexpr int64_t LIST_MAX_SEGS = int64_t(1) << 30;
 constexpr int64_t LIST_MAX_CELLS = int64_t(1) << 28;
+constexpr size_t LIST_HOLD_BYTES = (size_t)256 << 20;  // kept without a question
 constexpr int64_t DIR_MAX_ENTRIES = int64_t(1) << 28;  // chunk directories of B's rows
 constexpr size_t SMASK_MAX_BYTES = 128u << 20;         // their chunk masks
 
@@ -776,7 +782,10 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
                  plan->item_prod.ensure((size_t)plan->n_items * 4) == cudaSuccess &&
                  plan->cell_off.ensure(((size_t)cells + 1) * 8) == cudaSuccess &&
                  plan->item_seg.ensure(((size_t)plan->n_items + 1) * 8) == cudaSuccess;
-    cudaGetLastError();  // a refused allocation leaves the lookups
+    if (!lists) {
+        cudaGetLastError();  // a refused allocation leaves the lookups
+        if (list_bytes(plan) > LIST_HOLD_BYTES) release_lists(plan);
+    }
     {
         KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
         k_heavy_rows<<<(nh + 255) / 256, 256, 0, plan->stream>>>(
@@ -845,7 +854,10 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
         total = got.total;
         lists = !got.irregular && total <= LIST_MAX_SEGS && got.longest <= INT32_MAX >> cl &&
                 plan->seg.ensure((size_t)total * 8) == cudaSuccess;
-        cudaGetLastError();
+        if (!lists) {
+            cudaGetLastError();
+            if (list_bytes(plan) > LIST_HOLD_BYTES) release_lists(plan);
+        }
     }
     {
         KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
@@ -880,6 +892,55 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) 
     plan->lists_ok = lists;
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "heavy rows launch");
     return RVSP_SUCCESS;
+}
+
+size_t list_bytes(rvsp_cuda_plan* plan) {
+    DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
+    plan->list_bufs(b);
+    size_t n = 0;
+    for (DevBuf* x : b) n += x->cap;
+    return n;
+}
+
+void release_lists(rvsp_cuda_plan* plan) {
+    cudaGetLastError();
+    DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
+    plan->list_bufs(b);
+    for (DevBuf* x : b) x->release();
+    plan->lists_ok = false;
+}
+
+bool yield_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int* st) {
+    if (list_bytes(plan) == 0) return false;
+    const bool used = plan->lists_ok && plan->n_items > 0;
+    reset_graph(plan);  // (it holds the lists' addresses)
+    release_lists(plan);
+    if (used) *st = build_heavy_aux(plan, A, B);
+    return *st == RVSP_SUCCESS;
+}
+
+void trim_lists(rvsp_cuda_plan* plan, size_t keep) {
+    if (list_bytes(plan) > keep) release_lists(plan);
+}
+
+// What of the lists a plan whose C the caller is about to allocate keeps: not
+// what only building them reads, and nothing where C would not fit beside it.
+// (Both asked only of lists that matter to the device's memory: freeing and
+// querying are driver calls.)
+static int lists_beside_c(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
+    if (list_bytes(plan) <= LIST_HOLD_BYTES) return RVSP_SUCCESS;
+    cudaError_t e = cudaStreamSynchronize(plan->stream);
+    if (e != cudaSuccess) return fail(e, "symbolic");
+    DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
+    plan->list_bufs(b);
+    for (int i = 0; i < rvsp_cuda_plan::LIST_BUILD_BUFS; ++i) b[i]->release();
+    size_t free_b = 0, total_b = 0;
+    int st = RVSP_SUCCESS;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
+        cudaGetLastError();
+    else if (8 * (size_t)plan->c_nnz + 4 * ((size_t)plan->a_rows + 1) + (64u << 20) > free_b)
+        yield_lists(plan, A, B, &st);
+    return st;
 }
 
 // Per-B-row lookups of the heavy kernel (HeavyAux): metadata of every B row,
@@ -1349,6 +1410,7 @@ int rvsp_cuda_symbolic(rvsp_cuda_plan_t plan, int32_t a_rows, int32_t a_cols, in
         if ((st = analyze(plan, A, B, plan->features))) return st;
         if ((st = count_exact(plan, A, B))) return st;
     }
+    if ((st = lists_beside_c(plan, A, B))) return st;
     plan->analysed = true;
     *c_nnz_out = plan->c_nnz;
     *ws_bytes_out = 256;
@@ -1415,15 +1477,29 @@ int rvsp_cuda_numeric(rvsp_cuda_plan_t plan, const int32_t* a_rp, const int32_t*
     }
     CsrView A, B;
     int st = stage_operands(plan, a_rp, a_ci, a_v, b_rp, b_ci, b_v, true, &A, &B);
+    if (st == RVSP_ERROR_ALLOCATION_FAILED && plan->lists_ok) {
+        reset_graph(plan);
+        release_lists(plan);
+        st = stage_operands(plan, a_rp, a_ci, a_v, b_rp, b_ci, b_v, true, &A, &B);
+        if (!st && plan->n_items > 0) st = build_heavy_aux(plan, A, B);
+        if (st) plan->analysed = false;
+    }
     if (st) return st;
     int32_t* d_ci = c_ci;
     float* d_v = c_v;
+    const auto staging = [&](DevBuf& buf) {
+        if ((e = buf.ensure((size_t)nnz * 4)) != cudaSuccess && yield_lists(plan, A, B, &st))
+            e = buf.ensure((size_t)nnz * 4);
+        if (st) plan->analysed = false;
+        else if (e != cudaSuccess) st = fail(e, "C staging");
+        return st;
+    };
     if (!dev_ci) {
-        if ((e = plan->s_cci.ensure((size_t)nnz * 4)) != cudaSuccess) return fail(e, "C staging");
+        if (staging(plan->s_cci)) return st;
         d_ci = plan->s_cci.as<int32_t>();
     }
     if (!dev_v) {
-        if ((e = plan->s_cv.ensure((size_t)nnz * 4)) != cudaSuccess) return fail(e, "C staging");
+        if (staging(plan->s_cv)) return st;
         d_v = plan->s_cv.as<float>();
     }
     if (nnz > 0) {
@@ -1625,6 +1701,8 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         release_pool_memory(plan->stream);
         e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
     }
+    if (e != cudaSuccess && yield_lists(plan, A, B, &st))
+        e = cudaMallocAsync((void**)&rp, ((size_t)M + 1) * 4, plan->stream);
     if (e != cudaSuccess) {
         release();
         return fail(e, "one-shot product");
@@ -1647,7 +1725,12 @@ int oneshot_exact_device(rvsp_cuda_plan* plan, int32_t a_rows, int32_t a_cols, i
         }
         return e == cudaSuccess;
     };
-    if (!alloc_c() && slots) {
+    if (!alloc_c() && yield_lists(plan, A, B, &st)) alloc_c();
+    if (st) {
+        release();
+        return st;
+    }
+    if (e != cudaSuccess && slots) {
         // C beside the slots is too much: their memory goes back, and the
         // rows are counted after all
         release_slots();

@@ -178,6 +178,14 @@ struct rvsp_cuda_plan {
     rvsp::DevBuf brow_bits, brun_cnt, brun_off, brun_words, bruns, brows;
     rvsp::DevBuf cell_cnt, cell_prod, cell_off, item_seg, item_prod, work, seg;
     bool lists_ok = false;
+    // these buffers, and the ones of them that only building the lists reads
+    static constexpr int LIST_BUFS = 13, LIST_BUILD_BUFS = 9;
+    void list_bufs(rvsp::DevBuf* (&b)[LIST_BUFS]) {
+        rvsp::DevBuf* all[LIST_BUFS] = {&brow_bits, &brun_cnt, &brun_off, &brun_words, &bruns,
+                                        &brows, &cell_cnt, &cell_prod, &cell_off,
+                                        &item_seg, &item_prod, &work, &seg};
+        for (int i = 0; i < LIST_BUFS; ++i) b[i] = all[i];
+    }
     bool ameta_ok = false;
     bool dir_ok = false;
     int32_t smask_words = 0;    // words per B row of bsmask, 0: no masks
@@ -260,6 +268,19 @@ void note_launch(rvsp_cuda_plan* plan, int n);
 void reset_graph(rvsp_cuda_plan* plan);
 int build_heavy_aux(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
+// The segment lists' memory, for what else has to fit beside it: its size;
+// freed (plan->lists_ok false); freed for a plan whose rows are still to run,
+// which then take the lookups, false when there was nothing to free or the
+// lookups failed (*st); freed at the end of a call where it passes `keep`.
+size_t list_bytes(rvsp_cuda_plan* plan);
+void release_lists(rvsp_cuda_plan* plan);
+bool yield_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int* st);
+void trim_lists(rvsp_cuda_plan* plan, size_t keep);
+constexpr size_t LIST_KEEP_BYTES = (size_t)4 << 30;
+struct ListTrim {  // ... of a call on a thread's own plan
+    rvsp_cuda_plan* plan;
+    ~ListTrim() { trim_lists(plan, LIST_KEEP_BYTES); }
+};
 // Stable partition of the plan's rows by bin from the tiles' histograms and
 // their totals (hist); tile_off is scratch for their scan.
 int launch_bin_scatter(rvsp_cuda_plan* plan, const uint8_t* bin, const int32_t* hist,

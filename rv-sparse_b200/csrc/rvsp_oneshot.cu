@@ -125,6 +125,7 @@ extern "C" int rvsp_cuda_spgemm_f32(int algo, int32_t a_rows, int32_t a_cols, in
         if ((st = rvsp_cuda_plan_create(&plan, algo))) return st;
         plan->map_policy = 0;  // a one-shot product is never reused
     }
+    const ListTrim trim{plan};
     int32_t a_nnz = -1, b_nnz = -1;
     trace_point("one-shot: enter");
     const bool dev = is_dev(a_rp);
