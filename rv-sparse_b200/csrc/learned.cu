@@ -57,20 +57,31 @@ struct LearnedBinsOut {
     int32_t* tile_hist;  // [NUM_BINS][tiles]
     int32_t* hist;       // [NUM_BINS]
     int64_t* slot_total;
+    int64_t* slot_spare;  // what k_tight_slots would save
 };
+
+// Slot of a sorted row (no table: the prediction c sizes only the slot): the
+// prediction where it at least halves the bound, or, for tight slots, where it
+// is of a smaller table class, as for table rows.
+__device__ __forceinline__ bool predicted_slot(int c, int ub, bool tight, const BinParams& P) {
+    return tight ? table_bin(c, P) < table_bin(ub, P) : c < ub / 2;
+}
 
 __global__ void __launch_bounds__(AN_TILE)
     k_learned_bins(int32_t rows, const uint8_t* __restrict__ bin, const int64_t* __restrict__ ops,
                    const int32_t* __restrict__ ub, const int32_t* __restrict__ cap_pred,
                    LearnedBinsOut out, BinParams P) {
     __shared__ int32_t s_hist[NUM_BINS];
-    __shared__ unsigned long long s_slots;
+    __shared__ unsigned long long s_slots, s_spare;
     const int t = threadIdx.x;
     if (t < NUM_BINS) s_hist[t] = 0;
-    if (t == 0) s_slots = 0;
+    if (t == 0) {
+        s_slots = 0;
+        s_spare = 0;
+    }
     __syncthreads();
     const int row = blockIdx.x * AN_TILE + t;
-    int lb = -1, cap = 0;
+    int lb = -1, cap = 0, spare = 0;
     if (row < rows) {
         const int b = bin[row];
         int predicted = 0;
@@ -80,15 +91,14 @@ __global__ void __launch_bounds__(AN_TILE)
             lb = BIN_TINY;
             cap = (int)ops[row];
         } else if (b < BIN_WARP0) {
-            // sorted rows need no table: the prediction sizes only the slot,
-            // and only where it at least halves the bound's (which cannot
-            // overflow)
             lb = b;
-            cap = ub[row];
+            cap = ub[row];  // (cannot overflow)
             const int c = max(cap_pred[row], 1);
-            if (c < cap / 2) {
+            if (predicted_slot(c, cap, false, P)) {
                 cap = c;
                 predicted = 1;
+            } else if (predicted_slot(c, cap, true, P)) {
+                spare = cap - c;
             }
         } else {
             // the prediction is used only where it buys a smaller table than
@@ -131,12 +141,30 @@ __global__ void __launch_bounds__(AN_TILE)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sl += __shfl_xor_sync(FULL, sl, o);
     if ((t & 31) == 0 && sl) atomicAdd(&s_slots, sl);
+    if (__any_sync(FULL, spare > 0)) {
+        spare = __reduce_add_sync(FULL, spare);  // (rows of at most 2048 products)
+        if ((t & 31) == 0) atomicAdd(&s_spare, (unsigned long long)spare);
+    }
     __syncthreads();
     if (t < NUM_BINS) {
         out.tile_hist[t * gridDim.x + blockIdx.x] = s_hist[t];
         if (s_hist[t]) atomicAdd(&out.hist[t], s_hist[t]);
     }
     if (t == 0 && s_slots) atomicAdd((unsigned long long*)out.slot_total, s_slots);
+    if (t == 0 && s_spare) atomicAdd((unsigned long long*)out.slot_spare, s_spare);
+}
+
+// Sorted rows' slots made tight, for products whose slots would not fit.
+__global__ void k_tight_slots(int32_t rows, const uint8_t* __restrict__ bin,
+                              const int32_t* __restrict__ ub,
+                              const int32_t* __restrict__ cap_pred, int32_t* __restrict__ lcap,
+                              uint8_t* __restrict__ predicted, BinParams P) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= rows || bin[row] < BIN_SORT0 || bin[row] >= BIN_WARP0 || predicted[row]) return;
+    const int c = max(cap_pred[row], 1);
+    if (!predicted_slot(c, ub[row], true, P)) return;
+    lcap[row] = c;
+    predicted[row] = 1;
 }
 
 // Rows the sweep could not finish: too large for a table, or sized by the
@@ -457,12 +485,36 @@ static int learned_pre_sync(rvsp_cuda_plan* plan) {
         LearnedBinsOut lo{plan->lbin.as<uint8_t>(), plan->lcap.as<int32_t>(),
                           plan->pflag.as<uint8_t>(),
                           plan->heavy_slots ? plan->hmask.as<uint8_t>() : nullptr,
-                          plan->ltile_hist.as<int32_t>(), misc->lhist, &misc->slot_total};
+                          plan->ltile_hist.as<int32_t>(), misc->lhist, &misc->slot_total,
+                          &misc->slot_spare};
         k_learned_bins<<<(unsigned)tiles, AN_TILE, 0, plan->stream>>>(
             (int32_t)M, plan->bin.as<uint8_t>(), plan->ops.as<int64_t>(), plan->ub.as<int32_t>(),
             plan->pred_cap.as<int32_t>(), lo, plan->params);
     }
     note_launch(plan, 2);
+    return RVSP_SUCCESS;
+}
+
+// The slot buffers of plan->slot_total entries and, for heavy rows' chunks that
+// outgrow their predicted slot, an overflow pool of a quarter of the slots
+// after them in the same buffers. Buffers that must grow past 1 GiB must fit in
+// half the free memory (queried only then: the query waits behind any other
+// client of the driver, e.g. a clock monitor, with the GPU idle).
+static int slot_buffers(rvsp_cuda_plan* plan) {
+    plan->pool_cap = plan->n_items > 0 ? plan->slot_total / 4 : 0;
+    const int64_t tmp_total = plan->slot_total + plan->pool_cap;
+    cudaError_t e;
+    if ((size_t)tmp_total * 4 > plan->tmp_ci.cap && (size_t)plan->slot_total * 10 > (1ull << 30)) {
+        size_t free_b = 0, total_b = 0;
+        if ((e = cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess) return fail(e, "mem info");
+        if ((size_t)tmp_total * 8 > free_b / 2) {
+            g_err = "predicted capacity exceeds the memory budget";
+            return RVSP_ERROR_ALLOCATION_FAILED;
+        }
+    }
+    if ((e = plan->tmp_ci.ensure((size_t)tmp_total * 4)) != cudaSuccess ||
+        (e = plan->tmp_v.ensure((size_t)tmp_total * 4)) != cudaSuccess)
+        return fail(e, "slots");
     return RVSP_SUCCESS;
 }
 
@@ -488,39 +540,33 @@ int learned_symbolic(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool fused) {
     }
     plan->slot_total = plan->host_misc.slot_total;
     cudaError_t e;
-    // heavy rows' chunks that outgrow their predicted slot share an overflow
-    // pool of a quarter of the slots, after them in the same buffers
-    plan->pool_cap = fused && plan->n_items > 0 ? plan->slot_total / 4 : 0;
-    const int64_t tmp_total = plan->slot_total + plan->pool_cap;
-    size_t free_b = SIZE_MAX, total_b = 0;
-    // slot buffers that must grow past 1 GiB must fit in half the free
-    // memory (queried only then: the query waits behind any other client of
-    // the driver, e.g. a clock monitor, with the GPU idle)
-    if (fused && (size_t)tmp_total * 4 > plan->tmp_ci.cap &&
-        (size_t)plan->slot_total * 10 > (1ull << 30) &&
-        (e = cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess)
-        return fail(e, "mem info");
     if (fused) {
-        const auto over = [&] {
-            return free_b != SIZE_MAX && (size_t)tmp_total * 8 > free_b / 2;
-        };
-        const auto buffers = [&] {
-            if ((e = plan->slot_off.ensure(((size_t)M + 1) * 8)) == cudaSuccess &&
-                (e = plan->tmp_ci.ensure((size_t)tmp_total * 4)) == cudaSuccess)
-                e = plan->tmp_v.ensure((size_t)tmp_total * 4);
-            return e == cudaSuccess;
-        };
-        // (the segment lists must not cost a product its slots)
-        if (over() && yield_lists(plan, A, B, &st) &&
-            (e = cudaMemGetInfo(&free_b, &total_b)) != cudaSuccess)
-            return fail(e, "mem info");
-        if (st) return st;
-        if (over()) {
-            g_err = "predicted capacity exceeds the memory budget";
-            return RVSP_ERROR_ALLOCATION_FAILED;
-        }
-        if (!buffers() && !(yield_lists(plan, A, B, &st) && buffers()))
+        if ((e = plan->slot_off.ensure(((size_t)M + 1) * 8)) != cudaSuccess &&
+            !(yield_lists(plan, A, B, &st) &&
+              (e = plan->slot_off.ensure(((size_t)M + 1) * 8)) == cudaSuccess))
             return st ? st : fail(e, "slots");
+        // What may stand in the way of the slots: first the segment lists,
+        // then the sorted rows' loose slots.
+        for (int relief = 0;; ++relief) {
+            st = slot_buffers(plan);
+            if (st != RVSP_ERROR_ALLOCATION_FAILED || relief == 2) break;
+            if (relief == 0) {
+                st = RVSP_SUCCESS;
+                yield_lists(plan, A, B, &st);
+                if (st) return st;
+            } else if (plan->host_misc.slot_spare > 0) {
+                KTime kt(plan->stream, plan->capturing, KF_LEARNED);
+                k_tight_slots<<<(unsigned)((M + 255) / 256), 256, 0, plan->stream>>>(
+                    (int32_t)M, plan->bin.as<uint8_t>(), plan->ub.as<int32_t>(),
+                    plan->pred_cap.as<int32_t>(), plan->lcap.as<int32_t>(),
+                    plan->pflag.as<uint8_t>(), plan->params);
+                note_launch(plan, 1);
+                plan->slot_total -= plan->host_misc.slot_spare;
+            }
+        }
+        if (st) return st;
+    } else {
+        plan->pool_cap = 0;
     }
     if ((st = launch_bin_scatter(plan, plan->lbin.as<uint8_t>(), misc->lhist,
                                  plan->ltile_hist.as<int32_t>(), plan->ltile_off.as<int32_t>(),

@@ -47,6 +47,7 @@ struct Misc {
     int32_t n_need;            // learned path: rows sent to the exact path
     int32_t n_need_heavy;      //   of which heavy rows
     int64_t slot_total;        // learned path: sum of predicted capacities
+    int64_t slot_spare;        // ... and how much less tight slots would be
     int64_t lstats[8];         // learned path statistics (see rvsp_cuda_plan_learned_stats)
     int64_t ltile_total;
     int64_t dir_total;         // heavy-row B directory entries, or listed segments

@@ -117,6 +117,12 @@ def _child(case, mb):
     if case == "f64":  # 1230 MB of slots, 440 of C
         fn = "f64"
         A, B = _strata(200000, 32, 65536, g), _strata(65536, 16, 192, g)
+    if case == "slots_learned":  # 1.1 GB of loose slots, 0.8 of tight ones, 0.5 of C
+        A, B = _strata(150000, 30, 235, g), _strata(160000, 30, 265, g)
+        A[3].add_(T.arange(150000, device="cuda", dtype=T.int32).repeat_interleave(30))
+        B[3].add_(T.arange(160000, device="cuda", dtype=T.int32).repeat_interleave(30))
+        A, B = (150000, 160000) + A[2:], (160000, 161000) + B[2:]
+        algo = rv.RVSP_CUDA_ALGO_LEARNED
     if case.startswith("heavy"):  # 600 MB of segment lists and what builds them, 550 of C
         A, B = _strata(3000, 600, 204800, g), _strata(204800, 40, 1 << 18, g)
         algo = rv.RVSP_CUDA_ALGO_LEARNED if case == "heavy_learned" else algo
@@ -140,7 +146,7 @@ def _child(case, mb):
 
 @pytest.mark.parametrize("case,mb", [
     ("oneshot", 640), ("f64", 1200), ("f64", 1450), ("heavy_exact", 850), ("heavy_learned", 1600),
-    ("heavy_descriptor", 900), ("heavy_f64", 2250)])
+    ("slots_learned", 1700), ("heavy_descriptor", 900), ("heavy_f64", 2250)])
 def test_little_memory(gpu_lib, case, mb):
     _run(case, mb)
 
