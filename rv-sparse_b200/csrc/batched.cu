@@ -133,35 +133,57 @@ void release(cudaStream_t st, Packed& p) {
     p = Packed{};
 }
 
-// Intermediate products of each packed product: block i sums the B-row
-// lengths its A entries [a_off[i], a_off[i + 1]) reference (B rows are the
-// stacked B's: A's columns were shifted when packing). PRODUCT_PARTS CTAs a
-// product: one CTA each left the largest products running alone (128 products
-// of 256..65536 rows: 5.1 ms of a 20 ms call). ops starts at zero.
-constexpr int PRODUCT_PARTS = 64;
+// Intermediate products of each packed product: the sums of the B-row lengths
+// that its A entries [a_off[i], a_off[i + 1]) reference (B rows are the stacked
+// B's: A's columns were shifted when packing). A warp takes PRODUCT_STEPS steps
+// of 32 entries, of whichever products they are: a CTA a product left the
+// largest running alone (128 products of 256..65536 rows: 5.1 ms of a 20 ms
+// call), 64 CTAs a product are mostly empty for small ones (100,000 products of
+// 64 rows: 4.4 ms, 0.25 with one CTA each, 0.19 so). ops starts at zero.
+constexpr int PRODUCT_STEPS = 16;
 __global__ void __launch_bounds__(256)
-    k_product_ops(const int64_t* __restrict__ a_off, const int32_t* __restrict__ aci,
+    k_product_ops(const int64_t* __restrict__ a_off, int count, const int32_t* __restrict__ aci,
                   const int32_t* __restrict__ brp, int32_t b_rows, int64_t* __restrict__ ops,
                   int32_t* __restrict__ err) {
-    __shared__ unsigned long long s_sum;
-    if (threadIdx.x == 0) s_sum = 0;
-    __syncthreads();
-    const int i = blockIdx.x;
-    unsigned long long sum = 0;
-    for (int64_t j = a_off[i] + (int64_t)blockIdx.y * blockDim.x + threadIdx.x; j < a_off[i + 1];
-         j += (int64_t)gridDim.y * blockDim.x) {
-        const int k = aci[j];
-        if ((unsigned)k >= (unsigned)b_rows) {
-            atomicOr(err, ERR_STRUCTURE);
+    const int lane = threadIdx.x & 31;
+    const int64_t first = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * PRODUCT_STEPS);
+    const int64_t end = min(first + 32 * PRODUCT_STEPS, a_off[count]);
+    if (first >= end) return;
+    // the product of entry j, at or after product i
+    const auto product = [&](int64_t j, int i) {
+        if (j < a_off[i + 1]) return i;
+        int lo = i + 1, hi = count;  // a_off[lo] <= j < a_off[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (a_off[mid] <= j) lo = mid; else hi = mid;
+        }
+        return lo;
+    };
+    const auto add = [&](int i, unsigned long long x) {
+        if (x) atomicAdd((unsigned long long*)&ops[i], x);
+    };
+    int cur = product(first, 0);
+    unsigned long long sum = 0;  // this lane's share of product cur
+    for (int64_t base = first; base < end; base += 32) {
+        const int64_t j = base + lane;
+        unsigned long long len = 0;
+        if (j < end) {
+            const int k = aci[j];
+            if ((unsigned)k >= (unsigned)b_rows) atomicOr(err, ERR_STRUCTURE);
+            else len = (unsigned long long)max(brp[k + 1] - brp[k], 0);
+        }
+        if (min(base + 32, end) <= a_off[cur + 1]) {
+            sum += len;
             continue;
         }
-        const int len = brp[k + 1] - brp[k];
-        if (len > 0) sum += (unsigned long long)len;
+        add(cur, sum);  // a step of several products
+        sum = 0;
+        const int mine = product(min(j, end - 1), cur);
+        add(mine, len);
+        cur = __shfl_sync(FULL, mine, 31);
     }
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&s_sum, sum);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_sum) atomicAdd((unsigned long long*)&ops[i], s_sum);
+    if (lane == 0) add(cur, sum);
 }
 
 // Every product's own row pointer from its group's: slot s of the group
@@ -297,9 +319,12 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
                                 cudaMemcpyHostToDevice, s0);
         if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, 8 * (size_t)count, s0);
         if (e == cudaSuccess) {
-            k_product_ops<<<dim3((unsigned)count, PRODUCT_PARTS), 256, 0, s0>>>(d + count, pa.ci, pb.rp, (int32_t)br, d,
-                                                  &misc->err);
-            note_launch(nullptr, 1);
+            if (az > 0) {
+                const int64_t warps = (az + 32 * PRODUCT_STEPS - 1) / (32 * PRODUCT_STEPS);
+                k_product_ops<<<(unsigned)((warps + 7) / 8), 256, 0, s0>>>(
+                    d + count, count, pa.ci, pb.rp, (int32_t)br, d, &misc->err);
+                note_launch(nullptr, 1);
+            }
             e = cudaGetLastError();
         }
         int32_t err = 0;
