@@ -343,6 +343,38 @@ __global__ void __launch_bounds__(CS_TPB)
     if (threadIdx.x == 0) tile_runs[blockIdx.x] = s_sum;
 }
 
+// Rows between two entries that one lane writes the row pointer of; more are
+// its warp's (1000 entries in 2^28 rows, call: 143 ms by the lanes, 17 so; 16.8 M
+// entries in the first 64 of 2^20 rows: 4.9 and 1.25).
+constexpr int ROWS_ALONE = 32;
+
+// The row pointer of the warp's runs that start ROWS_ALONE rows and more after
+// the last one (bit s of heads: entry base + 32 s + lane starts a run; out: the
+// warp's first). Out of the kernel's way, as few warps have any.
+template <class K>
+__device__ __noinline__ void far_rows(int64_t base, const K* __restrict__ keys, unsigned heads,
+                                      int64_t out, int cb, int32_t* __restrict__ rp) {
+    const int lane = c_lane();
+    for (int s = 0; s < RUN_ITEMS; ++s) {
+        const int64_t i = base + 32 * s + lane;
+        const bool head = heads >> s & 1u;
+        const unsigned hm = __ballot_sync(CS_FULL, head);
+        int32_t row = 0, first = 0;
+        if (head) {
+            row = (int32_t)(keys[i] >> cb);
+            if (i > 0) first = (int32_t)(keys[i - 1] >> cb) + 1;
+        }
+        const int32_t o = (int32_t)(out + __popc(hm & ((1u << lane) - 1)));
+        for (unsigned m = __ballot_sync(CS_FULL, head && row - first >= ROWS_ALONE); m; m &= m - 1) {
+            const int j = __ffs(m) - 1;
+            const int32_t l = __shfl_sync(CS_FULL, row, j), x = __shfl_sync(CS_FULL, o, j);
+            for (int64_t r = (int64_t)__shfl_sync(CS_FULL, first, j) + lane; r <= l; r += 32)
+                rp[r] = x;
+        }
+        out += __popc(hm);
+    }
+}
+
 // One output entry per run: its column, and its values summed in COO order
 // from the first one (no added zero: a lone -0.0 stays). A run that starts a
 // new row writes the row pointer of every row since the last run's; the last
@@ -381,6 +413,8 @@ __global__ void __launch_bounds__(CS_TPB)
     __syncthreads();
     int64_t out = tile_off[blockIdx.x];
     for (int w = 0; w < warp; ++w) out += s_warp[w];
+    const int64_t out0 = out;
+    bool far = false;
 #pragma unroll
     for (int s = 0; s < RUN_ITEMS; ++s) {
         const int64_t i = base + 32 * s + lane;
@@ -400,13 +434,18 @@ __global__ void __launch_bounds__(CS_TPB)
             const int32_t row = (int32_t)(key[s] >> cb);
             out_ci[o] = (int32_t)(key[s] & (((K)1 << cb) - 1));
             out_v[o] = acc;
-            for (int32_t r = i == 0 ? 0 : (int32_t)(prev >> cb) + 1; r <= row; ++r)
-                rp[r] = (int32_t)o;
+            const int32_t first = i == 0 ? 0 : (int32_t)(prev >> cb) + 1;
+            if (row - first < ROWS_ALONE)
+                for (int32_t r = first; r <= row; ++r) rp[r] = (int32_t)o;
+            else
+                far = true;
         }
-        if (i == n - 1)
-            for (int32_t r = (int32_t)(key[s] >> cb) + 1; r <= rows; ++r) rp[r] = out_n;
         out += __popc(hm);
     }
+    if (__any_sync(CS_FULL, far)) far_rows(base, keys, heads, out0, cb, rp);
+    if (blockIdx.x == gridDim.x - 1)  // the rows after the last entry's
+        for (int64_t r = (int64_t)(keys[n - 1] >> cb) + 1 + threadIdx.x; r <= rows; r += CS_TPB)
+            rp[r] = out_n;
 }
 
 int bits_for(int64_t x) {  // bits to hold 0 .. x - 1
