@@ -107,13 +107,23 @@ struct CachedArray {
     void* p;
     size_t bytes;  // malloc_usable_size
 };
+// (fixed room: keeping an array allocates nothing that could throw out of a
+// free, and nothing is destroyed under a thread that still frees at exit)
 struct ArrayCache {
-    size_t max_arrays;
+    static constexpr int ROOM = 8;
+    int max_arrays;
     std::mutex mu;
-    std::vector<CachedArray> arrays;  // oldest first
+    CachedArray arrays[ROOM + 1] = {};  // oldest first
+    int n = 0;
     size_t held = 0;
+    CachedArray take(int i) {
+        const CachedArray a = arrays[i];
+        for (--n; i < n; ++i) arrays[i] = arrays[i + 1];
+        held -= a.bytes;
+        return a;
+    }
 };
-ArrayCache g_cache_large{4}, g_cache_small{8};
+ArrayCache g_cache_large{4}, g_cache_small{ArrayCache::ROOM};
 
 bool cache_on() {
     static const bool on = [] {
@@ -166,16 +176,11 @@ void* host_alloc(size_t bytes) {
         // the smallest cached array that holds bytes and wastes at most half
         std::lock_guard<std::mutex> hold(c->mu);
         int best = -1;
-        for (int i = 0; i < (int)c->arrays.size(); ++i)
+        for (int i = 0; i < c->n; ++i)
             if (c->arrays[i].bytes >= bytes && c->arrays[i].bytes / 2 <= bytes &&
                 (best < 0 || c->arrays[i].bytes < c->arrays[best].bytes))
                 best = i;
-        if (best >= 0) {
-            void* p = c->arrays[best].p;
-            c->held -= c->arrays[best].bytes;
-            c->arrays.erase(c->arrays.begin() + best);
-            return p;
-        }
+        if (best >= 0) return c->take(best).p;
     }
     if (bytes < STAGED_MIN) return malloc(bytes ? bytes : 1);
     void* p = nullptr;
@@ -190,18 +195,15 @@ void host_free(void* p) {
     ArrayCache* c = cache_of(bytes);
     const size_t cap = c == &g_cache_small ? 2 * STAGED_MIN : cache_cap();
     if (c && bytes <= cap) {
-        std::vector<void*> evict;
+        void* evict[ArrayCache::ROOM + 1];
+        int m = 0;
         {
             std::lock_guard<std::mutex> hold(c->mu);
-            c->arrays.push_back({p, bytes});
+            c->arrays[c->n++] = {p, bytes};
             c->held += bytes;
-            while (c->arrays.size() > c->max_arrays || c->held > cap) {
-                evict.push_back(c->arrays.front().p);
-                c->held -= c->arrays.front().bytes;
-                c->arrays.erase(c->arrays.begin());
-            }
+            while (c->n > c->max_arrays || c->held > cap) evict[m++] = c->take(0).p;
         }
-        for (void* q : evict) free(q);
+        while (m > 0) free(evict[--m]);
         return;
     }
     free(p);
