@@ -638,7 +638,8 @@ int analyze(rvsp_cuda_plan* plan, CsrView& A, CsrView& B, bool features,
                    plan->bin.as<uint8_t>(),
                    plan->chunk_lo.as<int32_t>(), plan->nchunks.as<int32_t>(),
                    features ? plan->feat.as<float4>() : nullptr, misc->hist,
-                   plan->tile_hist.as<int32_t>(), misc->totals, misc->bin_prod, &misc->err,
+                   plan->tile_hist.as<int32_t>(), misc->totals, &misc->longest_b,
+                   misc->bin_prod, &misc->err,
                    misc->nnz_ab};
     {
         KTime kt(plan->stream, plan->capturing, KF_ANALYSIS);
@@ -714,7 +715,8 @@ constexpr size_t SMASK_MAX_BYTES = 128u << 20;         // their chunk masks
 //            other, 0.4 us each, and writes the segments, 12.5 each, 5 where B's
 //            columns stay in L2; the walks gain 5 a product over the lookups'
 //   lookups  a sweep of B's long rows for directories, 4.5 Z, and one for chunk
-//            masks, 2 Z or 180 a row; a binary search per pair, 12.5 a step, 2.5
+//            masks, 2 Z or 180 a row, both by a warp a row, 12,800 an entry of
+//            the longest; a binary search per pair, 12.5 a step, 2.5
 //            where B's columns stay in L2, only for the hits with masks, none
 //            with directories, where a miss costs 5; launches of few items leave
 //            most of the GPU idle, 300 us
@@ -737,7 +739,8 @@ static bool lists_pay(const rvsp_cuda_plan* plan, int64_t chunks) {
     const double search = (far ? 12.5 : 2.5) * log2(std::max(len, 2.0));
     const double pairs = dir ? 5.0 * (V - hits) : (masks ? hits : V) * search;
     const double lookups = (masks ? std::max(2.0 * Z, 180.0 * K) : 0.0) + (dir ? 4.5 * Z : 0.0) +
-                           pairs + (plan->n_items < (1 << 15) ? 300e6 : 0.0);
+                           12.8e3 * plan->host_misc.longest_b + pairs +
+                           (plan->n_items < (1 << 15) ? 300e6 : 0.0);
     return lists <= lookups;
 }
 

@@ -31,7 +31,7 @@ struct Misc {
     int32_t cursor[NUM_BINS];  // bin scatter cursors
     int64_t totals[6];         // heavy items, products, and the heavy rows' units, cells,
                                // A entries and (entry, chunk) pairs
-    int32_t pad0;
+    int32_t longest_b;         // entries of the longest B row that a heavy row uses
     int32_t overflow;          // a 32-bit row pointer would overflow
     int64_t scan_total;        // nnz(C)
     int64_t scan_total2;       // heavy item total / learned capacity total

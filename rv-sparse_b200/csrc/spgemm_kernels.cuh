@@ -150,6 +150,7 @@ struct AnalyzeOut {
     int32_t* tile_hist;  // [NUM_BINS][tiles] rows per bin per tile (stable binning)
     int64_t* totals;     // [0] heavy items, [1] products, and of the heavy rows [2] units,
                          // [3] cells, [4] A entries, [5] (entry, chunk) pairs
+    int32_t* longest_b;  // entries of the longest B row that a heavy row uses
     int64_t* bin_prod;   // [NUM_BINS] products per bin
     int32_t* err;        // ERR_* bits
     int32_t* nnz_ab;     // [2] nnz of A and B as the kernel used them (read back with the bins)
@@ -350,7 +351,9 @@ __device__ __forceinline__ void an_finish(const AnalyzeOut& out, const BinParams
         const unsigned long long u = (n + HEAVY_UNIT - 1) / HEAVY_UNIT;
         const unsigned long long wu = warp_sum64(u), wc = warp_sum64(u * (unsigned long long)nch);
         const unsigned long long we = warp_sum64(n), wp = warp_sum64(n * (unsigned long long)nch);
+        const int longest = __reduce_max_sync(FULL, nch > 0 ? s.maxlen[t] : 0);
         if (lane_id() == 0) {
+            atomicMax(out.longest_b, longest);
             atomicAdd(&s.units, wu);
             atomicAdd(&s.cells, wc);
             atomicAdd(&s.entries, we);
