@@ -194,6 +194,13 @@ RVSP_CUDA_API int rvsp_cuda_op_counts(rvsp_cuda_plan_t plan, int64_t *op_counts_
  * with transparent huge pages advised). op_counts_out is optional (a_rows
  * entries, host or device). algo is RVSP_CUDA_ALGO_EXACT or
  * RVSP_CUDA_ALGO_LEARNED.
+ * Scratch memory, beside some 100 bytes a row: exact products of 2^22..2^29
+ * products of rows of at most 2048 hold 8 bytes a product while C is made;
+ * rows of more hold their segment lists (8 bytes a segment, 8 GiB at most, and
+ * 8 bytes an entry of B while they are built); learned products their slots.
+ * Where these do not fit beside C they are given up for the slower ways
+ * without them. Buffers are kept for the thread's next call, lists of up to
+ * 4 GiB among them.
  */
 RVSP_CUDA_API int rvsp_cuda_spgemm_f32(int algo, int32_t a_rows, int32_t a_cols, int32_t b_cols,
                          const int32_t *a_row_ptr, const int32_t *a_col_idx,
@@ -422,7 +429,10 @@ RVSP_CUDA_API int64_t rvsp_cuda_launch_count(void);
  * recorded pairs and writes each family's total milliseconds (and launch
  * count, when launches_out is non-NULL); n must be at least
  * RVSP_CUDA_KERNEL_FAMILIES. rvsp_cuda_kernel_family(i) names family i
- * (NULL out of range).
+ * (NULL out of range). A family is a class of rows and what is done to it,
+ * whichever kernel does it: "k_tiny" rows of at most 32 products (k_tiny_sort
+ * among them), "k_warp" the others whose products or columns fit a table
+ * (k_sort among them), "k_heavy" the rest (k_heavy_list among them).
  */
 #define RVSP_CUDA_KERNEL_FAMILIES 14
 RVSP_CUDA_API int rvsp_cuda_kernel_timing(int on);

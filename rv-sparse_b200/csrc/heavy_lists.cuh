@@ -20,13 +20,14 @@
 //   k_heavy_list  the products: a warp per item or group of items
 //
 // Measured (B200; device time, the lookup kernel k_heavy first): R-MAT 2^17,
-// COUNT 5.4 -> 3.0 ms, FILL 11.3 -> 5.8 ms; one 2^31-product row panel of R-MAT
+// COUNT 5.4 -> 2.8 ms, FILL 11.3 -> 5.8 ms; one 2^31-product row panel of R-MAT
 // 2^20, learned FILL 42.9 -> 17.5 ms; reuse of R-MAT 2^16, 4.5 -> 2.2 ms; the
 // lists themselves and the items take 0.8 ms of the first and 4.0 ms of the
 // second (the lookups' tables took 0.3 and 1.5). FILL is bound by the latency
 // of short work on 28 resident warps an SM and by the size of its code: every
 // path that is added costs all others (a third step in flight 12 %, a second
-// way to combine equal columns 3 %). COUNT is bound by issue (83 %).
+// way to combine equal columns 3 %). COUNT is bound by issue. Where the lists
+// would take longer than the lookups, k_heavy runs instead (lists_pay).
 #pragma once
 
 #include "spgemm_kernels.cuh"

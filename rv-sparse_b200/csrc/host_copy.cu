@@ -23,9 +23,10 @@
 // more holds at most 4 arrays and a sixteenth of the host memory (32 GiB at
 // most), the one of smaller arrays 8 arrays and 128 MiB; each frees its
 // oldest first, and RVSP_HOST_CACHE=0 turns both off. They keep allocations
-// only: every product computes and copies its C in full. (Products of 4096 and
-// 20000 rows, 8 and 40 MB of C in host memory: 3.9 and 20.3 ms a call without
-// the smaller arrays' cache, 0.76 and 2.8 with it.)
+// only: every product computes and copies its C in full. (Product of 4096 rows,
+// 8 MB of C in host memory: 0.77 ms a call; 0.8 to 2.6 without the smaller
+// arrays' cache, 4.1 in a process whose C library gives every freed array back
+// to the kernel.)
 #include <malloc.h>
 #include <sched.h>
 #include <stdlib.h>

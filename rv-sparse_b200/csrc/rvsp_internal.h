@@ -28,7 +28,6 @@ struct DevBuf {
 // Small device-side block of counters and flags of one plan.
 struct Misc {
     int32_t hist[NUM_BINS];    // rows per bin
-    int32_t cursor[NUM_BINS];  // bin scatter cursors
     int64_t totals[6];         // heavy items, products, and the heavy rows' units, cells,
                                // A entries and (entry, chunk) pairs
     int32_t longest_b;         // entries of the longest B row that a heavy row uses

@@ -160,7 +160,9 @@ __host__ __device__ inline bool sort_cols_fit(int32_t b_cols, int cap) {
 
 // A row goes to a sort bin when its products and B's columns fit and it could
 // hold at least one distinct column in SORT_UB_RATIO products: sorting costs
-// by the product, a table of few columns by the column.
+// by the product, a table of few columns by the column. (At four products a
+// column the sort is still ahead, 100,000 rows, calls by table and by sort: 100
+// columns 0.83 and 0.54 ms, 200 1.55 and 1.22, 400 3.29 and 2.59.)
 constexpr int SORT_UB_RATIO = 4;
 
 __host__ __device__ inline int bin_of(int64_t ops, int32_t ub, int32_t b_cols,
