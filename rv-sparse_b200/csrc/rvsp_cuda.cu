@@ -926,23 +926,33 @@ void trim_lists(rvsp_cuda_plan* plan, size_t keep) {
     if (list_bytes(plan) > keep) release_lists(plan);
 }
 
-// What of the lists a plan whose C the caller is about to allocate keeps: not
-// what only building them reads, and nothing where C would not fit beside it.
-// (Both asked only of lists that matter to the device's memory: freeing and
-// querying are driver calls.)
+// What of the lists a plan whose C the caller is about to allocate keeps: where
+// C would not fit beside them, or they pass what a thread's own plan would keep,
+// what only building them reads goes, and then, for C, the rest. (Asked only of
+// lists that matter to the device's memory, when they or C grew since the last
+// question: the query is a driver call of some 100 us, and freed buffers are
+// mapped anew by the next analysis, 1.5 ms a GB.)
 static int lists_beside_c(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     if (list_bytes(plan) <= LIST_HOLD_BYTES) return RVSP_SUCCESS;
-    cudaError_t e = cudaStreamSynchronize(plan->stream);
-    if (e != cudaSuccess) return fail(e, "symbolic");
-    DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
-    plan->list_bufs(b);
-    for (int i = 0; i < rvsp_cuda_plan::LIST_BUILD_BUFS; ++i) b[i]->release();
-    size_t free_b = 0, total_b = 0;
-    int st = RVSP_SUCCESS;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
+    const size_t need = 8 * (size_t)plan->c_nnz + 4 * ((size_t)plan->a_rows + 1) + (64u << 20);
+    if (list_bytes(plan) <= plan->asked_lists && need <= plan->asked_c) return RVSP_SUCCESS;
+    const auto fits = [need] {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) return need <= free_b;
         cudaGetLastError();
-    else if (8 * (size_t)plan->c_nnz + 4 * ((size_t)plan->a_rows + 1) + (64u << 20) > free_b)
-        yield_lists(plan, A, B, &st);
+        return true;
+    };
+    int st = RVSP_SUCCESS;
+    if (list_bytes(plan) > LIST_KEEP_BYTES || !fits()) {
+        cudaError_t e = cudaStreamSynchronize(plan->stream);
+        if (e != cudaSuccess) return fail(e, "symbolic");
+        DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
+        plan->list_bufs(b);
+        for (int i = 0; i < rvsp_cuda_plan::LIST_BUILD_BUFS; ++i) b[i]->release();
+        if (!fits()) yield_lists(plan, A, B, &st);
+    }
+    plan->asked_lists = list_bytes(plan);
+    plan->asked_c = need;
     return st;
 }
 

@@ -178,6 +178,7 @@ struct rvsp_cuda_plan {
     rvsp::DevBuf brow_bits, brun_cnt, brun_off, brun_words, bruns, brows;
     rvsp::DevBuf cell_cnt, cell_prod, cell_off, item_seg, item_prod, work, seg;
     bool lists_ok = false;
+    size_t asked_lists = 0, asked_c = 0;  // the last question of lists_beside_c
     // these buffers, and the ones of them that only building the lists reads
     static constexpr int LIST_BUFS = 13, LIST_BUILD_BUFS = 9;
     void list_bufs(rvsp::DevBuf* (&b)[LIST_BUFS]) {
