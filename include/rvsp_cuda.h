@@ -199,8 +199,8 @@ RVSP_CUDA_API int rvsp_cuda_op_counts(rvsp_cuda_plan_t plan, int64_t *op_counts_
  * rows of more hold their segment lists (8 bytes a segment, 8 GiB at most, and
  * 8 bytes an entry of B while they are built); learned products their slots.
  * Where these do not fit beside C they are given up for the slower ways
- * without them. Buffers are kept for the thread's next call, lists of up to
- * 4 GiB among them.
+ * without them. Buffers are kept for the thread's next call; lists of 64 MiB and
+ * more return to the device's pool, like C when it is released.
  */
 RVSP_CUDA_API int rvsp_cuda_spgemm_f32(int algo, int32_t a_rows, int32_t a_cols, int32_t b_cols,
                          const int32_t *a_row_ptr, const int32_t *a_col_idx,

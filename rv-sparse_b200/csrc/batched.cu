@@ -297,7 +297,7 @@ extern "C" int rvsp_cuda_spgemm_batched_f32(
         }
         if (c_off_dev) cudaFreeAsync(c_off_dev, s0);
         cudaStreamSynchronize(s0);
-        for (rvsp_cuda_plan* p : plans) trim_lists(p, LIST_KEEP_BYTES / plans.size());
+        for (rvsp_cuda_plan* p : plans) trim_lists(p);
         return status;
     };
     cudaError_t e0 = plans[0]->misc.ensure(sizeof(Misc));

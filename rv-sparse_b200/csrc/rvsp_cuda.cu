@@ -149,17 +149,18 @@ KTime::~KTime() {
 
 cudaError_t DevBuf::ensure(size_t bytes) {
     if (bytes <= cap && p) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
+    release();
     const size_t want = bytes < 256 ? 256 : bytes;
-    cudaError_t e = cudaMalloc(&p, want);
+    pooled = stream && want >= POOL_MIN;
+    cudaError_t e = pooled ? cudaMallocAsync(&p, want, stream) : cudaMalloc(&p, want);
     if (e == cudaSuccess) cap = want;
+    else p = nullptr;
     return e;
 }
 
 void DevBuf::release() {
-    if (p) cudaFree(p);
+    if (p && pooled) cudaFreeAsync(p, stream);
+    else if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
 }
@@ -910,6 +911,7 @@ void release_lists(rvsp_cuda_plan* plan) {
     DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
     plan->list_bufs(b);
     for (DevBuf* x : b) x->release();
+    release_pool_memory(plan->stream);
     plan->lists_ok = false;
 }
 
@@ -922,16 +924,24 @@ bool yield_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int* 
     return *st == RVSP_SUCCESS;
 }
 
-void trim_lists(rvsp_cuda_plan* plan, size_t keep) {
-    if (list_bytes(plan) > keep) release_lists(plan);
+void trim_lists(rvsp_cuda_plan* plan) {
+    DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
+    plan->list_bufs(b);
+    bool any = false;
+    for (DevBuf* x : b)
+        if (x->p && x->pooled) {
+            x->release();
+            any = true;
+        }
+    // (only what is known to be free is given to other allocations)
+    if (any) cudaStreamSynchronize(plan->stream);
+    plan->lists_ok = false;
 }
 
 // What of the lists a plan whose C the caller is about to allocate keeps: where
-// C would not fit beside them, or they pass what a thread's own plan would keep,
-// what only building them reads goes, and then, for C, the rest. (Asked only of
-// lists that matter to the device's memory, when they or C grew since the last
-// question: the query is a driver call of some 100 us, and freed buffers are
-// mapped anew by the next analysis, 1.5 ms a GB.)
+// C would not fit beside them, what only building them reads goes, and then the
+// rest. (Asked only of lists that matter to the device's memory, when they or C
+// grew since the last question: the query is a driver call of some 100 us.)
 static int lists_beside_c(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B) {
     if (list_bytes(plan) <= LIST_HOLD_BYTES) return RVSP_SUCCESS;
     const size_t need = 8 * (size_t)plan->c_nnz + 4 * ((size_t)plan->a_rows + 1) + (64u << 20);
@@ -943,15 +953,15 @@ static int lists_beside_c(rvsp_cuda_plan* plan, const CsrView& A, const CsrView&
         return true;
     };
     int st = RVSP_SUCCESS;
-    if (list_bytes(plan) > LIST_KEEP_BYTES || !fits()) {
-        cudaError_t e = cudaStreamSynchronize(plan->stream);
-        if (e != cudaSuccess) return fail(e, "symbolic");
+    const size_t held = list_bytes(plan);
+    if (!fits()) {
         DevBuf* b[rvsp_cuda_plan::LIST_BUFS];
         plan->list_bufs(b);
         for (int i = 0; i < rvsp_cuda_plan::LIST_BUILD_BUFS; ++i) b[i]->release();
+        release_pool_memory(plan->stream);  // (what the pool keeps counts as taken)
         if (!fits()) yield_lists(plan, A, B, &st);
     }
-    plan->asked_lists = list_bytes(plan);
+    plan->asked_lists = held;
     plan->asked_c = need;
     return st;
 }
@@ -1291,6 +1301,9 @@ int rvsp_cuda_plan_create(rvsp_cuda_plan_t* out, int algo) {
         delete p;
         return fail(e, "stream create");
     }
+    DevBuf* lists[rvsp_cuda_plan::LIST_BUFS];
+    p->list_bufs(lists);
+    for (DevBuf* b : lists) b->stream = p->stream;
     *out = p;
     return RVSP_SUCCESS;
 }

@@ -13,10 +13,16 @@
 
 namespace rvsp {
 
-// Grow-only device buffer.
+// Grow-only device buffer. One that is given a stream takes POOL_MIN bytes and
+// more from the device's stream-ordered pool, where a release and the next
+// allocation cost microseconds and what nobody uses goes to other allocations
+// of the process that need it.
 struct DevBuf {
+    static constexpr size_t POOL_MIN = (size_t)64 << 20;
     void* p = nullptr;
     size_t cap = 0;
+    cudaStream_t stream = nullptr;
+    bool pooled = false;
     cudaError_t ensure(size_t bytes);
     void release();
     template <class T>
@@ -272,15 +278,14 @@ int build_heavy_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B);
 // The segment lists' memory, for what else has to fit beside it: its size;
 // freed (plan->lists_ok false); freed for a plan whose rows are still to run,
 // which then take the lookups, false when there was nothing to free or the
-// lookups failed (*st); freed at the end of a call where it passes `keep`.
+// lookups failed (*st); its pool memory freed at the end of a call.
 size_t list_bytes(rvsp_cuda_plan* plan);
 void release_lists(rvsp_cuda_plan* plan);
 bool yield_lists(rvsp_cuda_plan* plan, const CsrView& A, const CsrView& B, int* st);
-void trim_lists(rvsp_cuda_plan* plan, size_t keep);
-constexpr size_t LIST_KEEP_BYTES = (size_t)4 << 30;
+void trim_lists(rvsp_cuda_plan* plan);
 struct ListTrim {  // ... of a call on a thread's own plan
     rvsp_cuda_plan* plan;
-    ~ListTrim() { trim_lists(plan, LIST_KEEP_BYTES); }
+    ~ListTrim() { trim_lists(plan); }
 };
 // Stable partition of the plan's rows by bin from the tiles' histograms and
 // their totals (hist); tile_off is scratch for their scan.
